@@ -50,6 +50,7 @@ struct ps4_ctx {
     double last_ms = 0.0;
     uint64_t last_launches = 0;
     unsigned tile_log2 = 13;             // current tile size (may shrink on E_TILE)
+    unsigned run_tile_log2 = 13;         // the tile size of the launches in flight (smaller for narrow calls)
     PendingSearch pend;
     uint64_t *d_raw = nullptr;           // per tile-kernel CTA: SUPER_K tile lists of RAW_PER_TILE
     uint64_t raw_words = 0;
@@ -60,6 +61,8 @@ struct ps4_ctx {
     bool fused_fallback = false;         // this call re-runs on the fused kernel (engine list overflow)
     bool persist_fallback = false;       // this call re-runs on the two-kernel pipeline (a persistent-kernel
                                          //   wait gave up, or a tile outgrew the 2^13-S tile lists)
+    bool wide_tiles = false;             // this call re-runs without the smaller tiles of narrow calls (one of
+                                         //   them outgrew its lists)
     uint32_t *d_seq = nullptr;           // the persistent kernel's ring: slot states (ring_cap u32); its
     uint64_t seq_cap = 0;                //   4-sets use d_jobs with ring_cap entries
     uint64_t ring_cap = 1ull << 26;
@@ -247,6 +250,14 @@ const char *fatal_text(unsigned code) {
     }
 }
 
+unsigned narrow_tile_log2(unsigned TL, uint64_t tiles, int num_sms) {
+    while (TL > 12 && tiles < (uint64_t)gen_grid(num_sms, TL)) {
+        TL--;
+        tiles *= 2;
+    }
+    return TL;
+}
+
 // 4-sets per S grow slowly with S (0.13 below 1e10, 0.29 near 2e12); a batch of the
 // two-kernel pipeline is sized so that this bound, with margin, fills at most 90 % of the queue.
 double jobs_per_S_bound(uint64_t S_hi) {
@@ -360,13 +371,19 @@ static int enqueue_items(ps4_ctx *c) {
     int kernel = c->fused_fallback ? (int)PS4_KERNEL_FUSED : (int)c->cfg.kernel;
     if (kernel == PS4_KERNEL_PERSIST && c->persist_fallback) kernel = PS4_KERNEL_BATCHED;
     const bool persist = kernel == PS4_KERNEL_PERSIST;
-    const unsigned TL = persist ? 13u : c->tile_log2;      // the persistent kernel's tiles are 2^13 S
+    unsigned TL = persist ? 13u : c->tile_log2;            // the persistent kernel's tiles are 2^13 S
+    if (kernel == PS4_KERNEL_BATCHED && !c->wide_tiles) {
+        uint64_t tiles = 0;
+        for (const Item &it : p.items) tiles += (it.hi - it.lo + (1ull << TL) - 1) >> TL;
+        TL = narrow_tile_log2(TL, tiles, c->num_sms);
+    }
     if (kernel == PS4_KERNEL_BATCHED) {          // queue: the call's expected 4-sets, 2^20 .. jobs_cap_max
         double need = 0;
         for (uint32_t i = 0; i < n_items; i++)
             need += jobs_per_S_bound(p.items[i].hi) * (double)(p.items[i].hi - p.items[i].lo);
         while (c->jobs_cap < c->jobs_cap_max && (double)c->jobs_cap * 0.9 < need) c->jobs_cap <<= 1;
     }
+    c->run_tile_log2 = TL;
     std::vector<Item> segs;                      // all batches' segments, batch after batch
     std::vector<size_t> batch_start;             // segs index where each batch begins
     std::vector<uint64_t> batch_tiles;
@@ -416,9 +433,16 @@ static int enqueue_items(ps4_ctx *c) {
     }
     if (kernel == PS4_KERNEL_BATCHED && c->d_jobs_words < 6 * c->jobs_cap)
         if (grow(c, c->d_jobs, c->d_jobs_words, 6 * c->jobs_cap)) return PS4_ERR_CUDA;
-    if (kernel == PS4_KERNEL_BATCHED &&
-        c->raw_words < (uint64_t)c->num_sms * c->gen_ctas * SUPER_K * RAW_PER_TILE)
-        if (grow(c, c->d_raw, c->raw_words, (uint64_t)c->num_sms * 2 * SUPER_K * RAW_PER_TILE)) return PS4_ERR_CUDA;
+    // gen_ctas counts 512 threads per SM: one or two 512-thread CTAs on 2^14-S tiles, twice as
+    // many 256-thread ones on smaller tiles; a narrow call needs no more CTAs (nor lists for them)
+    // than it has tiles
+    const int g_full = c->num_sms * (int)c->gen_ctas * (gen_threads(14) / gen_threads(TL));
+    uint64_t most_tiles = 1;
+    for (uint64_t t : batch_tiles) most_tiles = std::max(most_tiles, t);
+    const int g_gen = (int)std::min<uint64_t>((uint64_t)g_full, (most_tiles + GEN_CLUSTER - 1) / GEN_CLUSTER * GEN_CLUSTER);
+    const uint64_t raw_need = (uint64_t)g_gen * SUPER_K * raw_cap_for(TL);
+    if (kernel == PS4_KERNEL_BATCHED && c->raw_words < raw_need)
+        if (grow(c, c->d_raw, c->raw_words, raw_need)) return PS4_ERR_CUDA;
     const int g_persist = c->num_sms * persist_ctas_per_sm();
     const uint32_t raw_cap_persist = RAW_PER_TILE / 2;           // 2^13-S tiles: half the representations
     if (persist) {
@@ -464,9 +488,7 @@ static int enqueue_items(ps4_ctx *c) {
         a.raw_cap = raw_cap_persist;
     }
     const bool ext = !(c->cfg.flags & PS4_F_NOEXT);
-    // gen_ctas counts 512 threads per SM: one or two 512-thread CTAs on 2^14-S tiles, twice as
-    // many 256-thread ones on smaller tiles
-    const int g_gen = c->num_sms * (int)c->gen_ctas * (gen_threads(14) / gen_threads(TL)), g_ext = c->num_sms * (int)c->ext_ctas;
+    const int g_ext = c->num_sms * (int)c->ext_ctas;
 
     // A call of several batches runs as one CUDA graph holding its whole launch sequence; the
     // graph is kept and replayed while the next call is the same (items, sizes, buffers).
@@ -515,11 +537,11 @@ static int enqueue_items(ps4_ctx *c) {
                 a.items = c->d_items + s0;
                 a.n_items = (uint32_t)(s1 - s0);
                 a.n_tiles = batch_tiles[b];
-                const int g = (int)std::min<uint64_t>((uint64_t)g_gen, std::max<uint64_t>(a.n_tiles, 1));
+                a.s_top = segs[s1 - 1].hi;                   // a batch's segments ascend by their end
                 // n_jobs, tile_next, ext_next: the per-batch tail of the status block
                 e = cudaMemsetAsync(&c->d_status->n_jobs, 0, 2 * sizeof(unsigned long long), c->stream);
                 if (timed && e == cudaSuccess) e = cudaEventRecord(c->kev[4 * b], c->stream);
-                if (e == cudaSuccess) e = (cudaError_t)launch_gen(a, g, c->stream);
+                if (e == cudaSuccess) e = (cudaError_t)launch_gen(a, g_gen, c->stream);
                 if (timed && e == cudaSuccess) e = cudaEventRecord(c->kev[4 * b + 1], c->stream);
                 c->last_launches++;
                 if (e == cudaSuccess && ext) {
@@ -576,6 +598,7 @@ static int begin_items(ps4_ctx *c, const uint64_t *lo, const uint64_t *hi, uint3
     p.items.assign(n_items, Item{});
     c->fused_fallback = false;
     c->persist_fallback = false;
+    c->wide_tiles = false;
     c->last_launches = 0;
     c->last_ms = 0.0;
     c->h2d_bytes = c->d2h_bytes = 0;
@@ -655,6 +678,10 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
             !c->fused_fallback) {
             c->fused_fallback = true;            // more extensions in one engine round than its list holds: fused kernel
             continue;
+        }
+        if (code == E_TILE && !c->wide_tiles) {  // a no-op unless the call was narrow; then as it would be without
+            c->wide_tiles = true;
+            if (c->run_tile_log2 < c->tile_log2) continue;
         }
         if (code == E_TILE || code == E_EXTLIST) {
             if (c->tile_log2 > 12) { c->tile_log2--; continue; }

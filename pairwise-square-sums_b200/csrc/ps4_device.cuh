@@ -385,6 +385,20 @@ __device__ __forceinline__ uint32_t isqrt_lt2p46(uint64_t x) {
     return r;
 }
 
+// p = ceil(sqrt(m)) for 0 < m < 2^44, and over = p^2 - m.  The estimate's relative error is below
+// 2^-23 (sqrt.approx) + 2^-25 (half the conversion's), so for a root below 2^22 it is off by less than
+// 0.7 and its floor by at most one either way: one exact correction step, without branches.
+__device__ __forceinline__ uint32_t ceil_sqrt_lt2p44(uint64_t m, uint32_t &over) {
+    float f;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"((float)m));
+    uint32_t r = (uint32_t)f;
+    int32_t d = (int32_t)(m - (uint64_t)r * r);            // |d| < 2^24: the difference's low word
+    if (d < 0) { r--; d += 2 * (int32_t)r + 1; }           // floor(root) or one below it from here on
+    if (d > 2 * (int32_t)r) { d -= 2 * (int32_t)r + 1; r++; }
+    over = d > 0 ? 2 * r + 1 - (uint32_t)d : 0u;
+    return d > 0 ? r + 1 : r;
+}
+
 // P1 / P3: scan every representation S = p^2 + q^2, 1 <= p <= q, S in [S0, S0+n).
 // q-major: q runs over [ceil(sqrt(S0/2)), isqrt(S1-2)] (strided over the threads), p from
 // ceil(sqrt(S0-q^2)) by a float estimate with exact integer correction (S < 2^44).
@@ -421,43 +435,77 @@ __device__ __forceinline__ uint32_t scan_reps(uint64_t S0, uint32_t n, uint32_t 
     return found;
 }
 
-// The scan of scan_reps over a group of up to SUPER_K adjacent tiles [SS0, SS1) of one
-// segment, done once: every representation goes to its tile's list (offset in the tile | p << 14 |
-// q << 36; p <= q < 2^22, offset < 2^14), in the slice of the warp that found it (one shared
-// atomic per representation).  Slice counts above `slice` mean the list overflowed; that tile
-// then scans for itself.  NT threads, NT/32 warp slices per tile.
-template <int NT = BS>
-__device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned TLv, uint64_t *lists,
-                                           uint32_t list_cap, uint32_t *raw_n, uint32_t slice) {
+constexpr uint32_t SCAN_RUN = 24;      // a q with more p than this is walked by a whole warp
+
+// The scan of scan_reps over a group of adjacent tiles [SS0, SS1) of one segment, done once by
+// `parts` CTAs together (this one takes every parts-th q, from `part`): every representation goes
+// to its tile's list (offset in the tile | p << 14 | q << 36; p <= q < 2^22, offset < 2^14), each CTA
+// into its own part of the list, `cap` entries long, counted in cnt[tile] (one shared-memory atomic
+// per representation).  A count above cap means the part overflowed; that tile then scans for itself.
+template <int NT>
+__device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned TLv, uint64_t *lists, uint32_t cap,
+                                           uint32_t *cnt, uint32_t part, uint32_t parts) {
     uint32_t qmin = (uint32_t)ceil_sqrt64((SS0 + 1) >> 1);
     if (qmin < 1) qmin = 1;
     const uint32_t qmax = SS1 >= 2 ? (uint32_t)isqrt64(SS1 - 2) : 0;
-    const int wid = threadIdx.x >> 5;
-    const uint32_t wmask = (1u << TLv) - 1u;
-    for (uint32_t q = qmin + threadIdx.x; q <= qmax; q += NT) {
+    const uint32_t width = (uint32_t)(SS1 - SS0), wmask = (1u << TLv) - 1u;
+    // long runs need 2 * SCAN_RUN * p < width, so p < pc and q^2 >= SS0 - pc^2: below qc there are none
+    const uint64_t pc = width / (2 * SCAN_RUN);
+    const uint32_t qc = pc * pc < SS0 ? (uint32_t)isqrt64(SS0 - pc * pc) : 0u;
+    const int lane = threadIdx.x & 31;
+    lists += (size_t)part * cap;
+    auto put = [&](uint32_t q, uint32_t p, uint32_t i) {                 // S = SS0 + i
+        const uint32_t j = i >> TLv;
+        const uint32_t pos = atomicAdd(&cnt[j], 1u);
+        if (pos < cap)
+            lists[(size_t)(j * parts) * cap + pos] = (uint64_t)(i & wmask) | ((uint64_t)p << 14) | ((uint64_t)q << 36);
+    };
+    for (uint32_t qw = qmin + part + parts * (threadIdx.x - lane); qw <= qmax; qw += parts * NT) {   // warp-uniform
+        const uint32_t q = qw + parts * lane;
         const uint64_t q2 = (uint64_t)q * q;
-        uint32_t p = 1;
+        uint32_t p = 1, i = 0;                             // i = p^2 + q^2 - SS0, below width where it counts
+        bool live = q <= qmax;
         if (SS0 > q2 + 1) {
-            const uint64_t m = SS0 - q2;
-            const uint32_t r = isqrt_lt2p46(m);
-            p = r + ((uint64_t)r * r < m ? 1u : 0u);
+            p = ceil_sqrt_lt2p44(SS0 - q2, i);
+        } else {
+            live = live && q2 + 1 - SS0 < width;
+            i = (uint32_t)(q2 + 1 - SS0);
         }
-        for (uint64_t s = (uint64_t)p * p + q2; p <= q && s < SS1; s += 2 * p + 1, p++) {
-            const uint32_t i = (uint32_t)(s - SS0), j = i >> TLv;
-            const uint32_t pos = atomicAdd(&raw_n[j * (NT / 32) + wid], 1u);
-            if (pos < slice)
-                lists[(size_t)j * list_cap + (size_t)wid * slice + pos] =
-                    (uint64_t)(i & wmask) | ((uint64_t)p << 14) | ((uint64_t)q << 36);
+        live = live && p <= q && i < width;
+        // a q with a long run of p (the top of the q range: p small against the width) is walked
+        // by the whole warp, the others by their lanes
+        if (qw + 31 * parts >= qc) {                       // warp-uniform
+            unsigned coop = __ballot_sync(0xffffffffu, live && i + SCAN_RUN * (2 * p + SCAN_RUN) < width);
+            if (coop >> lane & 1u) live = false;
+            while (coop) {
+                const int o = __ffs((int)coop) - 1;
+                coop &= coop - 1;
+                const uint32_t cq = __shfl_sync(0xffffffffu, q, o), p0 = __shfl_sync(0xffffffffu, p, o);
+                const uint32_t i0 = __shfl_sync(0xffffffffu, i, o);
+                // p^2 - p0^2 = (p - p0)(p + p0); p < p0 + 32 + width / (2 p0), within 32 bits by width < 2^21
+                for (uint32_t k = lane;; k += 32) {
+                    const uint64_t ck = (uint64_t)k * (k + 2 * p0) + i0;
+                    if (p0 + k > cq || ck >= width) break;
+                    put(cq, p0 + k, (uint32_t)ck);
+                }
+            }
+        }
+        for (; live; live = p <= q && i < width) {
+            put(q, p, i);
+            i += 2 * p + 1;
+            p++;
         }
     }
 }
 
 // P1-P4 for one tile.  Returns false if the tile was abandoned (error raised).  With `list` (the
-// tile's representations from scan_group, list_n[w] entries in warp slice w of `slice`) P1 and
-// P3 read the list; without, they scan.
+// tile's representations from scan_group, list_n[w] entries in part w of `parts`, `cap` apart; other
+// CTAs of the cluster may have written them: read through L2) P1 and P3 read the list; without,
+// they scan.
 template <int TL, int NT = BS>
 __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0, uint32_t n,
-                          const uint64_t *list = nullptr, const uint32_t *list_n = nullptr, uint32_t slice = 0) {
+                          const uint64_t *list = nullptr, const uint32_t *list_n = nullptr, uint32_t parts = 0,
+                          uint32_t cap = 0) {
     using L = TileLayout<TL>;
     uint32_t *cnt32 = (uint32_t *)(smem + L::OFF_CNT);
     uint16_t *is_off = (uint16_t *)(smem + L::OFF_IS_OFF);
@@ -473,10 +521,10 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
     // P1: count, from the list or by scanning
     uint32_t found = 0;
     if (list) {
-        for (int w = 0; w < NT / 32; w++) {
+        for (uint32_t w = 0; w < parts; w++) {
             const uint32_t cw = list_n[w];
             for (uint32_t o = tid; o < cw; o += NT) {
-                const uint32_t i = (uint32_t)list[(size_t)w * slice + o] & 0x3FFFu;
+                const uint32_t i = (uint32_t)__ldcg(list + (size_t)w * cap + o) & 0x3FFFu;
                 atomicAdd(&cnt32[i >> 1], 1u << ((i & 1) * 16));
                 found++;
             }
@@ -563,10 +611,10 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
     __syncthreads();
     // P3: fill, from the list or by scanning again
     if (list) {
-        for (int w = 0; w < NT / 32; w++) {
+        for (uint32_t w = 0; w < parts; w++) {
             const uint32_t cw = list_n[w];
             for (uint32_t o = tid; o < cw; o += NT) {
-                const uint64_t e = list[(size_t)w * slice + o];
+                const uint64_t e = __ldcg(list + (size_t)w * cap + o);
                 const uint32_t i = (uint32_t)e & 0x3FFFu, wd = i >> 1, sh = (i & 1) * 16;
                 const uint32_t cur = (((volatile uint32_t *)cnt32)[wd] >> sh) & 0xFFFFu;
                 if (cur == 0xFFFFu) continue;          // S not selected

@@ -18,10 +18,16 @@
 //
 // Every counter and every reported line is identical to the reference's.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "ps4_device.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace ps4 {
 
@@ -229,143 +235,196 @@ __device__ __forceinline__ uint32_t lane_pairs(const SearchArgs &a, uint32_t gw,
     return n;
 }
 
-// One claimed group of tiles, the last-but-c0 SUPER_K tiles of the launch (tiles are taken from
-// the last one down, costliest first): per segment of the group one scan for all its tiles (when
-// `lists` is given), then per tile P1-P4, the count pass, one reservation for the tile's
-// 4-sets, the write pass.  NT threads.  RING: the 4-sets go to the persistent kernel's ring and
-// each lane publishes its contiguous run after a fence.  Returns the number of tiles.
+// The segment of tile ti: the last one whose first tile is not after it.
+__device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
+    uint32_t lo = 0, hi = a.n_items;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (a.items[mid].tile_base <= ti) lo = mid; else hi = mid;
+    }
+    return a.items[lo];
+}
+
+// One tile [S0, S0+n) of query item `item`: P1-P4 (from its list's parts, or by scanning when list
+// is null), the count pass, one reservation for the tile's 4-sets, the write
+// pass.  NT threads.  RING: the 4-sets go to the persistent kernel's ring and each lane publishes
+// its contiguous run after a fence.
 template <int TL, int NT, bool RING>
-__device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t c0,
-                                  uint64_t *lists, uint32_t *raw_n, uint32_t slice, unsigned long long &s_base,
-                                  int &s_store) {
+__device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0, uint32_t n,
+                                             uint32_t item, const uint64_t *list, const uint32_t *list_n,
+                                             uint32_t parts, uint32_t cap, unsigned long long &s_base, int &s_store) {
     using L = TileLayout<TL>;
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x;
     const bool noext = (a.flags & PS4_F_NOEXT) != 0;
     const bool need_write_pass = !noext || (a.flags & (PS4_F_DUMP4 | PS4_F_VERIFY));
+    tile_reset(ts);
+    __syncthreads();
+    if (!tile_reps<TL, NT>(a, ts, smem, S0, n, list, list_n, parts, cap)) { __syncthreads(); return; }
+    const uint16_t *is_off = (const uint16_t *)(smem + L::OFF_IS_OFF);
+    const uint16_t *is_k = (const uint16_t *)(smem + L::OFF_IS_K);
+    const uint16_t *is_start = (const uint16_t *)(smem + L::OFF_IS_START);
+    const uint32_t *is_pbase = (const uint32_t *)(smem + L::OFF_IS_PBASE);
+    const uint32_t *rep_p = (const uint32_t *)(smem + L::OFF_REP_P);
+    const uint32_t *rep_q = (const uint32_t *)(smem + L::OFF_REP_Q);
+    const uint32_t nI = ts.n_is, nPairs = ts.n_pairs;
+    // count pass, one reservation for the tile, write pass in the same order
+    // each warp a contiguous block of pairs (whole multiples of 32)
+    const int lane = tid & 31, wid = tid >> 5;
+    const uint32_t blk = ((nPairs + NW * 32 - 1) / (NW * 32)) * 32;
+    const uint32_t gw = (uint32_t)wid * blk, ge = min(nPairs, gw + blk);
+    uint32_t mine = lane_pairs<false>(a, gw, ge, lane, nI, is_off, is_k, is_start, is_pbase, rep_p, rep_q, S0, item, 0,
+                                      false);
+    uint32_t off, d1, d2, tot[3];
+    block_scan3<NT>(mine, 0u, 0u, off, d1, d2, tot, ts.wsum);
+    if (tid == 0) {
+        ts.cnt[K_SETS4] += tot[0];
+        s_base = 0;
+        s_store = 0;
+        if (!noext && tot[0]) {
+            if (RING) {
+                // room: the ring holds the reserved-but-unfinished 4-sets plus this tile's
+                WaitClock wc;
+                bool ok = true;
+                while (ld_vol(&a.status->q_tail) + tot[0] - ld_vol(&a.status->q_freed) > a.jobs_cap) {
+                    if (ld_vol(&a.status->err) != 0ull || wc.expired(a, 3)) { ok = false; break; }
+                    __nanosleep(256);
+                }
+                if (ok) {
+                    s_base = atomicAdd(&a.status->q_tail, (ull)tot[0]);
+                    s_store = 1;
+                }
+            } else {
+                s_base = atomicAdd(&a.status->n_jobs, (ull)tot[0]);
+                if (s_base + tot[0] <= a.jobs_cap) s_store = 1;
+                else raise_capacity(a.status, E_QUEUE, 5, s_base + tot[0], a.jobs_cap, S0);
+            }
+        }
+    }
+    __syncthreads();
+    if (need_write_pass) {
+        const bool store = s_store != 0;
+        lane_pairs<true, RING>(a, gw, ge, lane, nI, is_off, is_k, is_start, is_pbase, rep_p, rep_q, S0, item,
+                               s_base + off, store);
+        if (RING && store && mine) {               // publish this lane's run [s_base+off, +mine)
+            __threadfence();
+            for (uint32_t i = 0; i < mine; i++) {
+                const uint64_t pos = s_base + off + i;
+                *(volatile uint32_t *)&a.seq[pos & a.ring_mask] = (uint32_t)(pos + 1);
+            }
+        }
+    }
+    __syncthreads();
+    if (RING && tid == 0 && s_store && tot[0]) atomicAdd(&a.status->q_pub, (ull)tot[0]);
+    tile_flush_counters(a, ts, item);
+    __syncthreads();
+}
+
+// The persistent kernel's claim of SUPER_K tiles, the last-but-c0 ones of the launch (tiles are
+// taken from the last one down, costliest first): per segment among them one scan for all its
+// tiles, then tile by tile.  Returns the number of tiles.
+template <int TL, int NT>
+__device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t c0,
+                                  uint64_t *lists, uint32_t *raw_n, unsigned long long &s_base, int &s_store) {
+    using L = TileLayout<TL>;
     const uint64_t cn = min((uint64_t)SUPER_K, a.n_tiles - c0);
     uint64_t ti = a.n_tiles - c0 - cn;
     const uint64_t ti_end = a.n_tiles - c0;
     while (ti < ti_end) {
-        // a group: the claimed tiles of one segment, one scan for all of them
-        uint32_t lo = 0, hi = a.n_items;
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (a.items[mid].tile_base <= ti) lo = mid; else hi = mid;
-        }
-        const Item it = a.items[lo];
+        const Item it = segment_of(a, ti);
         const uint64_t seg_tiles = (it.hi - it.lo + (1ull << TL) - 1) >> TL;
         const uint64_t g_end = min(ti_end, it.tile_base + seg_tiles);
         const uint32_t ng = (uint32_t)(g_end - ti);
         const uint64_t SA = it.lo + ((ti - it.tile_base) << TL);
         const uint64_t SB = min(it.hi, SA + ((uint64_t)ng << TL));
-        const uint32_t item = it.id;
-        const bool grouped = lists != nullptr;
-        if (grouped) {
-            if (tid < SUPER_K * NW) raw_n[tid] = 0;
-            __syncthreads();
-            scan_group<NT>(SA, SB, TL, lists, a.raw_cap, raw_n, slice);
-            __syncthreads();
-        }
+        if (threadIdx.x < SUPER_K) raw_n[threadIdx.x] = 0;
+        __syncthreads();
+        scan_group<NT>(SA, SB, TL, lists, a.raw_cap, raw_n, 0, 1);
+        __syncthreads();
         for (uint32_t j = 0; j < ng; j++) {
-            tile_reset(ts);
-            __syncthreads();
             const uint64_t S0 = SA + ((uint64_t)j << TL);
-            const uint32_t n = (uint32_t)min((uint64_t)L::W, SB - S0);
-            bool use_list = grouped;
-            for (int w = 0; w < NW; w++) use_list = use_list && raw_n[j * NW + w] <= slice;
-            if (!tile_reps<TL, NT>(a, ts, smem, S0, n, use_list ? lists + (size_t)j * a.raw_cap : nullptr,
-                                   &raw_n[j * NW], slice)) { __syncthreads(); continue; }
-            const uint16_t *is_off = (const uint16_t *)(smem + L::OFF_IS_OFF);
-            const uint16_t *is_k = (const uint16_t *)(smem + L::OFF_IS_K);
-            const uint16_t *is_start = (const uint16_t *)(smem + L::OFF_IS_START);
-            const uint32_t *is_pbase = (const uint32_t *)(smem + L::OFF_IS_PBASE);
-            const uint32_t *rep_p = (const uint32_t *)(smem + L::OFF_REP_P);
-            const uint32_t *rep_q = (const uint32_t *)(smem + L::OFF_REP_Q);
-            const uint32_t nI = ts.n_is, nPairs = ts.n_pairs;
-            // count pass, one reservation for the tile, write pass in the same order
-            // each warp a contiguous block of pairs (whole multiples of 32)
-            const int lane = tid & 31, wid = tid >> 5;
-            const uint32_t blk = ((nPairs + NW * 32 - 1) / (NW * 32)) * 32;
-            const uint32_t gw = (uint32_t)wid * blk, ge = min(nPairs, gw + blk);
-            uint32_t mine = lane_pairs<false>(a, gw, ge, lane, nI, is_off, is_k, is_start, is_pbase, rep_p, rep_q, S0,
-                                              item, 0, false);
-            uint32_t off, d1, d2, tot[3];
-            block_scan3<NT>(mine, 0u, 0u, off, d1, d2, tot, ts.wsum);
-            if (tid == 0) {
-                ts.cnt[K_SETS4] += tot[0];
-                s_base = 0;
-                s_store = 0;
-                if (!noext && tot[0]) {
-                    if (RING) {
-                        // room: the ring holds the reserved-but-unfinished 4-sets plus this tile's
-                        WaitClock wc;
-                        bool ok = true;
-                        while (ld_vol(&a.status->q_tail) + tot[0] - ld_vol(&a.status->q_freed) > a.jobs_cap) {
-                            if (ld_vol(&a.status->err) != 0ull || wc.expired(a, 3)) { ok = false; break; }
-                            __nanosleep(256);
-                        }
-                        if (ok) {
-                            s_base = atomicAdd(&a.status->q_tail, (ull)tot[0]);
-                            s_store = 1;
-                        }
-                    } else {
-                        s_base = atomicAdd(&a.status->n_jobs, (ull)tot[0]);
-                        if (s_base + tot[0] <= a.jobs_cap) s_store = 1;
-                        else raise_capacity(a.status, E_QUEUE, 5, s_base + tot[0], a.jobs_cap, S0);
-                    }
-                }
-            }
-            __syncthreads();
-            if (need_write_pass) {
-                const bool store = s_store != 0;
-                lane_pairs<true, RING>(a, gw, ge, lane, nI, is_off, is_k, is_start, is_pbase, rep_p, rep_q, S0, item,
-                                       s_base + off, store);
-                if (RING && store && mine) {       // publish this lane's run [s_base+off, +mine)
-                    __threadfence();
-                    for (uint32_t i = 0; i < mine; i++) {
-                        const uint64_t pos = s_base + off + i;
-                        *(volatile uint32_t *)&a.seq[pos & a.ring_mask] = (uint32_t)(pos + 1);
-                    }
-                }
-            }
-            __syncthreads();
-            if (RING && tid == 0 && s_store && tot[0]) atomicAdd(&a.status->q_pub, (ull)tot[0]);
-            tile_flush_counters(a, ts, item);
-            __syncthreads();
+            produce_tile<TL, NT, true>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
+                                       raw_n[j] <= a.raw_cap ? lists + (size_t)j * a.raw_cap : nullptr, &raw_n[j], 1,
+                                       a.raw_cap, s_base, s_store);
         }
         ti = g_end;
     }
     return (uint32_t)cn;
 }
 
+// The tile kernel: clusters of CTAs claim `a.group` tiles at a time (from the last one down,
+// costliest first).  Per segment among them the cluster's CTAs share one scan -- each takes every
+// nc-th q and appends what it finds to its part of the tiles' lists -- and then take the tiles one
+// by one from a common counter.  A scan costs ~0.29 sqrt(S) steps however few S it covers, and a
+// narrow call has too few tiles for one CTA each on a scan of its own, so both ends gain from sharing it.
 template <int TL, int NT>
 __global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const SearchArgs a) {
     using L = TileLayout<TL>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileShared ts;
-    __shared__ unsigned long long s_base;
+    __shared__ unsigned long long s_base, s_claim;
     __shared__ int s_store;
-    __shared__ unsigned long long s_claim;
+    __shared__ uint32_t s_tile, s_fit;
+    // entries that this CTA's scan appended to each tile's list, and the next tile to take (CTA 0's
+    // is used).  Two sets, one for each parity of the group: a set is cleared while the other one's
+    // group is scanned, between the two cluster barriers that no CTA passes before all have
+    // finished the group that used it last.
+    __shared__ uint32_t raw_n[2][GEN_CLUSTER * SUPER_K];
+    __shared__ uint32_t s_take[2];
+    __shared__ uint32_t s_n[GEN_CLUSTER];                                // the parts' entries of the tile at hand
     const int tid = threadIdx.x;
-    uint64_t *lists = a.raw ? a.raw + (size_t)blockIdx.x * SUPER_K * a.raw_cap : nullptr;
-    // per tile of a group and warp: representations appended to the tile's list; in the tile
-    // layout's extension-list area, which this kernel does not use otherwise
-    uint32_t *raw_n = (uint32_t *)(smem + L::OFF_ELIST);
-    const uint32_t slice = a.raw ? a.raw_cap / (NT / 32) : 0;
-    for (;;) {
-        // claim SUPER_K tiles; tiles are taken from the last one down (costliest first)
-        if (tid == 0) {
-            s_claim = atomicAdd(&a.status->tile_next, SUPER_K);
-            ts.skip = *(volatile ull *)&a.status->err != 0ull;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), nc = cluster.num_blocks();
+    const uint32_t cap = a.raw_cap / nc;
+    uint64_t *lists = a.raw + (size_t)(blockIdx.x / nc) * nc * SUPER_K * a.raw_cap;
+    for (uint32_t i = tid; i < GEN_CLUSTER * SUPER_K; i += NT) raw_n[0][i] = 0;
+    if (tid == 0) s_take[0] = 0;
+    uint64_t ti = 0, ti_end = 0;
+    for (uint32_t par = 0;; par ^= 1) {                                  // every CTA of the cluster alike
+        if (ti == ti_end) {
+            if (rank == 0 && tid == 0)
+                s_claim = *(volatile ull *)&a.status->err != 0ull ? a.n_tiles
+                                                                  : (ull)atomicAdd(&a.status->tile_next, a.group);
+            cluster.sync();
+            const uint64_t c0 = *cluster.map_shared_rank(&s_claim, 0);
+            if (c0 >= a.n_tiles) break;
+            ti_end = a.n_tiles - c0;
+            ti = ti_end - min((uint64_t)a.group, ti_end);
+        } else {
+            cluster.sync();
         }
-        __syncthreads();
-        const uint64_t c0 = s_claim;
-        const bool stop = c0 >= a.n_tiles || ts.skip;
-        __syncthreads();                                                 // s_claim read by all
-        if (stop) break;                                                 // block-uniform
-        produce_group<TL, NT, false>(a, ts, smem, c0, lists, raw_n, slice, s_base, s_store);
+        for (uint32_t i = tid; i < GEN_CLUSTER * SUPER_K; i += NT) raw_n[par ^ 1][i] = 0;
+        if (tid == 0) s_take[par ^ 1] = 0;
+        const Item it = segment_of(a, ti);
+        const uint64_t seg_tiles = (it.hi - it.lo + (1ull << TL) - 1) >> TL;
+        const uint64_t g_end = min(ti_end, it.tile_base + seg_tiles);
+        const uint32_t ng = (uint32_t)(g_end - ti);
+        const uint64_t SA = it.lo + ((ti - it.tile_base) << TL);
+        const uint64_t SB = min(it.hi, SA + ((uint64_t)ng << TL));
+        scan_group<NT>(SA, SB, TL, lists, cap, raw_n[par], rank, nc);
+        cluster.sync();
+        for (;;) {
+            if (tid == 0) {
+                s_tile = atomicAdd(cluster.map_shared_rank(&s_take[par], 0), 1u);
+                s_fit = 1;
+            }
+            __syncthreads();
+            const uint32_t j = s_tile;
+            if (j >= ng) break;                                          // block-uniform
+            if (tid < nc) {
+                const uint32_t c = *cluster.map_shared_rank(&raw_n[par][j], tid);
+                s_n[tid] = c;
+                if (c > cap) s_fit = 0;
+            }
+            __syncthreads();
+            const uint64_t S0 = SA + ((uint64_t)j << TL);
+            produce_tile<TL, NT, false>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
+                                        s_fit ? lists + (size_t)j * nc * cap : nullptr, s_n, nc, cap, s_base, s_store);
+        }
+        __syncthreads();                                                 // s_tile read by all
+        ti = g_end;
     }
+    cluster.sync();                          // no CTA leaves while another may read its shared memory
 }
 
 // ================================================================== extend_jobs
@@ -1018,7 +1077,7 @@ constexpr int PWARPS = PBS / 32;
 // the tile state of the producing role sits in the dynamic area too, after the tile layout and
 // the group's list counters, so that the kernel's static shared memory stays a few words and three
 // CTAs (each with the 1 KB the hardware reserves per block) fit in the SM's 228 KB
-constexpr size_t P_TS_OFF = (TileLayout<PTL>::OFF_ELIST + SUPER_K * PWARPS * sizeof(uint32_t) + 15) & ~(size_t)15;
+constexpr size_t P_TS_OFF = (TileLayout<PTL>::OFF_ELIST + SUPER_K * sizeof(uint32_t) + 15) & ~(size_t)15;
 static_assert(P_TS_OFF + sizeof(TileShared) <= PWARPS * sizeof(WarpArea),
               "the tile layout and tile state fit in the engine's warp areas");
 static_assert(PWARPS * sizeof(WarpArea) + 1024 + 128 <= 228 * 1024 / 3, "three persistent CTAs per SM");
@@ -1031,9 +1090,8 @@ __global__ void __launch_bounds__(PBS, 3) search_persist(const SearchArgs a) {
     __shared__ unsigned int s_claim;
     __shared__ int s_store, s_role, s_busy;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    uint64_t *lists = a.raw ? a.raw + (size_t)blockIdx.x * SUPER_K * a.raw_cap : nullptr;
+    uint64_t *lists = a.raw + (size_t)blockIdx.x * SUPER_K * a.raw_cap;
     uint32_t *raw_n = (uint32_t *)(smem + L::OFF_ELIST);
-    const uint32_t slice = a.raw ? a.raw_cap / PWARPS : 0;
     if (tid == 0) s_idle0 = 0;
     for (;;) {
         if (tid == 0) {
@@ -1064,7 +1122,7 @@ __global__ void __launch_bounds__(PBS, 3) search_persist(const SearchArgs a) {
         const int role = s_role;
         if (role == 0) break;                                // block-uniform
         if (role == 1) {
-            const uint32_t cn = produce_group<PTL, PBS, true>(a, ts, smem, s_claim, lists, raw_n, slice, s_base, s_store);
+            const uint32_t cn = produce_group<PTL, PBS>(a, ts, smem, s_claim, lists, raw_n, s_base, s_store);
             if (tid == 0) {
                 __threadfence();
                 atomicAdd(&a.status->q_produced, (ull)cn);
@@ -1105,25 +1163,59 @@ __global__ void ring_init(uint32_t *seq, uint64_t n) {
 
 // ================================================================== launchers
 
+// the tile layout up to its extension-list area, which the tile kernel does not use
+template <int TL>
+static int setup_gen(size_t &smem) {
+    smem = TileLayout<TL>::OFF_ELIST;
+    return (int)cudaFuncSetAttribute(gen_jobs<TL, gen_threads(TL)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem);
+}
+
+// the tile kernel's full residency for 2^TL-S tiles
 int gen_grid(int num_sms, unsigned TL) { return num_sms * (BS / gen_threads(TL)) * 2; }
 int ext_grid(int num_sms) { return num_sms * 3; }
 
 template <int TL>
-static int launch_gen_tl(const SearchArgs &a, int grid, cudaStream_t s) {
-    // the tile layout up to its extension-list area, then the group's list counters there
-    constexpr int NT = gen_threads(TL);
-    const size_t smem = TileLayout<TL>::OFF_ELIST + SUPER_K * (NT / 32) * sizeof(uint32_t);
-    cudaFuncSetAttribute(gen_jobs<TL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gen_jobs<TL, NT><<<grid, NT, smem, s>>>(a);
-    return (int)cudaGetLastError();
+static int launch_gen_tl(const SearchArgs &a, int grid, uint32_t cluster, cudaStream_t s) {
+    size_t smem;
+    if (const int e = setup_gen<TL>(smem)) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(gen_threads(TL));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, gen_jobs<TL, gen_threads(TL)>, a);
 }
 
-int launch_gen(const SearchArgs &a, int grid, void *stream) {
+// Launch shape of the tile kernel.  A group's scan visits 0.29 sqrt(S) q, as much work as s tiles
+// (68,000 q cost what a tile of 2^13 S does: 2.7 ps against 183 ns of the whole device at S = 1e12).
+//  * Cluster: 8 CTAs where scans weigh, i.e. for high S and for calls with few tiles, else 2 (a
+//    cluster of 8 costs 8 % in barriers and in CTAs that fit no GPC; of 2, nothing).  Measured, tile
+//    kernel with 8 / 2 / 1 CTAs: [1,1e10) 155.6 / 141.1 / 140.4 ms; 2e8 S at 1e12 4.95 / 6.27 / 8.32; 3e7 S
+//    at 1.2e13 2.81 / 5.71 / 9.75; 2e4 S at 4e11 0.079 / 0.140 / 0.220; 2e6 S at 1e9 0.103 / 0.109 / 0.129.
+//  * Tiles per claim: n tiles in groups of G on K clusters take n + s n / G of work and about G K / 2 of
+//    idling at the end, least at G = sqrt(2 n s / K).
+// `grid`: the CTAs that the lists of a.raw are sized for; whole clusters of them are launched, no more
+// than there are tiles to take.
+int launch_gen(SearchArgs a, int grid, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
+    const double n = (double)std::max<uint64_t>(a.n_tiles, 1);
+    const double scan = 0.29 * std::sqrt((double)a.s_top) / (68e3 * std::ldexp(1.0, (int)a.log2_tile - 13));
+    const uint32_t cl = n < 23e3 * scan || grid < 16 ? GEN_CLUSTER : 2;
+    const uint64_t fit = std::max<uint64_t>((uint64_t)grid / cl, 1), want = ((uint64_t)n + cl - 1) / cl;
+    const uint64_t K = std::min(fit, want), ctas = K * cl;
+    const double G = std::min(std::sqrt(2 * n * scan / (double)K), std::ceil(n / (double)K));
+    a.group = (uint32_t)std::min<double>(std::max<double>(G, cl), cl * SUPER_K);
     switch (a.log2_tile) {
-        case 12: return launch_gen_tl<12>(a, grid, s);
-        case 13: return launch_gen_tl<13>(a, grid, s);
-        default: return launch_gen_tl<14>(a, grid, s);
+        case 12: return launch_gen_tl<12>(a, (int)ctas, cl, s);
+        case 13: return launch_gen_tl<13>(a, (int)ctas, cl, s);
+        default: return launch_gen_tl<14>(a, (int)ctas, cl, s);
     }
 }
 

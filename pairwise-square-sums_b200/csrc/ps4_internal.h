@@ -82,8 +82,10 @@ struct SearchArgs {
     uint32_t flags;            // PS4_F_*
     uint32_t *jobs;            // 4-set job queue between gen_jobs and extend_jobs: jobs_cap 24-byte records
     uint64_t jobs_cap;
-    uint64_t *raw;             // optional (gen_jobs): per CTA, SUPER_K lists of one tile's representations,
-    uint32_t raw_cap;          //   raw_cap entries each, in one equal slice per warp
+    uint64_t *raw;             // tile and persistent kernel: per CTA, SUPER_K lists of one tile's
+    uint32_t raw_cap;          //   representations, raw_cap entries each (a cluster pools its CTAs' lists)
+    uint64_t s_top;            // the launch's largest S, for the tile kernel's launch shape
+    uint32_t group;            // tile kernel: tiles a cluster claims at once (set by launch_gen)
     // persistent kernel: jobs is a ring of jobs_cap (a power of two) slots; seq[slot] tells its state
     // for position pos = slot + lap * jobs_cap: pos = free for pos, pos + 1 = 4-set of pos written
     uint32_t *seq;
@@ -96,17 +98,16 @@ struct SearchArgs {
 // the persistent kernel's threads per CTA, and the time any of its waits may take before it gives up
 constexpr int PBS = 256;
 constexpr unsigned long long WAIT_NS = 2000000000ull;
-// representations a 2^14-S tile's list holds: (pi/8) * 2^14 = 6434 expected, 8192 with margin;
+// representations a 2^14-S tile's list holds: (pi/8) * 2^14 = 6434 expected, 10240 with margin;
 // a 2^TL-S tile's list holds raw_cap_for(TL), in proportion
-constexpr uint32_t RAW_PER_TILE = 8192;
+constexpr uint32_t RAW_PER_TILE = 10240;
 constexpr uint32_t raw_cap_for(unsigned TL) { return RAW_PER_TILE >> (14 - TL); }
-// tiles a tile-kernel CTA claims at once and scans as one range: the scan of a tile costs
-// ~0.29 sqrt(S) steps whatever its width, so one scan of SUPER_K adjacent tiles, recorded into
-// their lists, divides that cost by SUPER_K (lists: 592 CTAs x 16 x 32 KB = 310 MB; 16 tiles of
-// 2^13 S instead of 8: tile kernel -8 % at S = 5e11, per 5e8-S step).  With these tiles the group
-// scan pays at every S: per [1,1e10) step of the tile kernel 195.4 ms with groups from S = 5e9 up,
-// 161.0 from 1e9, 159.7 everywhere.
+// tile lists per CTA of the tile and the persistent kernel (592 CTAs x 16 x 40 KB = 388 MB): a
+// cluster of the tile kernel scans up to GEN_CLUSTER * SUPER_K adjacent tiles as one range, a
+// CTA of the persistent kernel SUPER_K
 constexpr uint32_t SUPER_K = 16;
+// CTAs of a tile-kernel cluster (the portable maximum)
+constexpr uint32_t GEN_CLUSTER = 8;
 // threads of a tile-kernel CTA: 512 on 2^14-S tiles (two CTAs per SM), 256 on smaller ones (four
 // per SM).  At 2^13 S and four CTAs a barrier waits for 8 warps, not 16, and while one CTA waits
 // at it the other three issue: per [1,1e10) step of the tile kernel 219.2 -> 195.2 ms.
@@ -136,6 +137,9 @@ enum { TRI_OK = 0, TRI_INVALID = 1, TRI_RANGE = 2 };
 void stats_add(ps4_stats *s, const unsigned long long *k);      // fold one counter block into stats (+=)
 const char *fatal_text(unsigned code);                            // the reference's FATAL message text
 double jobs_per_S_bound(uint64_t S_hi);                           // 4-set job queue entries per S, bound
+// Tile size of a call with `tiles` tiles of 2^TL S: smaller ones (down to 2^12) while the tile
+// kernel's CTAs outnumber the tiles, since a narrow call lasts as long as one CTA's tiles.
+unsigned narrow_tile_log2(unsigned TL, uint64_t tiles, int num_sms);
 void canonical_order(std::vector<ps4_hit> &hits, std::vector<ps4_ext> &exts, std::vector<ps4_six> &sixes);
 void canonical_order_into(const ps4_hit *hits, uint64_t nh, const ps4_ext *exts, ps4_six *sixes, uint64_t ns,
                           ps4_hit *out_hits, ps4_ext *out_exts);
@@ -157,7 +161,7 @@ int ctx_fail(ps4_ctx *c, int code, const char *msg);
 int launch_tables(uint64_t *spfq, uint16_t *ndiv, uint64_t tab_n, void *stream);
 int launch_fac3(uint4 *fac3, uint64_t tab_n, void *stream);
 // two-kernel pipeline (ps4_extend.cu): 4-set generation into the job queue, then extension
-int launch_gen(const SearchArgs &a, int grid, void *stream);
+int launch_gen(SearchArgs a, int grid, void *stream);
 int launch_ext(const SearchArgs &a, int grid, void *stream);
 // the persistent kernel (ps4_extend.cu): tiles of 2^13 S, ring of a.jobs_cap slots
 int launch_persist(const SearchArgs &a, int grid, void *stream);

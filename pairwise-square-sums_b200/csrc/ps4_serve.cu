@@ -284,6 +284,7 @@ struct ps4_server {
     std::vector<int> free_slots;
     std::deque<uint32_t> unreported;
     unsigned tile_log2 = 13;
+    bool wide_tiles = false;                 // no smaller tiles for narrow steps (one of them outgrew its lists)
     uint32_t batch_div = 1;
     bool fused_next = false;
     uint64_t seq = 0;
@@ -519,10 +520,16 @@ void plan_step(ps4_server *s, StepBuf &b) {
 
 int launch_step(ps4_server *s, StepBuf &b) {
     const uint32_t n_items = (uint32_t)b.chunks.size(), n_tri = (uint32_t)b.tris.size();
+    uint64_t tiles = 0, s_top = 0;
+    if (!b.fused && !s->wide_tiles) {
+        for (const Chunk &c : b.chunks) tiles += (c.hi - c.lo + (1ull << b.tile_log2) - 1) >> b.tile_log2;
+        b.tile_log2 = narrow_tile_log2(b.tile_log2, tiles, s->v.num_sms);
+        tiles = 0;
+    }
     const unsigned TL = b.tile_log2;
-    uint64_t tiles = 0;
     for (uint32_t i = 0; i < n_items; i++) {
         const Chunk &c = b.chunks[i];
+        s_top = std::max(s_top, c.hi);
         Item it;
         it.lo = c.lo; it.hi = c.hi; it.tile_base = tiles; it.id = i; it.pad = 0;
         tiles += (c.hi - c.lo + (1ull << TL) - 1) >> TL;
@@ -593,8 +600,8 @@ int launch_step(ps4_server *s, StepBuf &b) {
         a.jobs = s->d_jobs; a.jobs_cap = s->jobs_cap;
         if (!b.fused) {
             a.raw = s->d_raw; a.raw_cap = raw_cap_for(TL);
-            const int g = (int)std::min<uint64_t>((uint64_t)gen_grid(s->v.num_sms, TL), std::max<uint64_t>(tiles, 1));
-            SRV_CUDA(s, (cudaError_t)launch_gen(a, g, st));
+            a.s_top = s_top;
+            SRV_CUDA(s, (cudaError_t)launch_gen(a, gen_grid(s->v.num_sms, TL), st));
             if (!(s->v.flags & PS4_F_NOEXT)) SRV_CUDA(s, (cudaError_t)launch_ext(a, ext_grid(s->v.num_sms), st));
         } else {
             const uint32_t stage_cap = stage_cap_for(TL, s->v.cap_reps);
@@ -649,7 +656,9 @@ int check_step(ps4_server *s, StepBuf &b) {
         s->fused_next = true;
         rerun = true;
     } else if (code == E_TILE || code == E_EXTLIST) {
-        if (s->tile_log2 > 12) {
+        if (code == E_TILE && b.tile_log2 < s->tile_log2) {
+            s->wide_tiles = true;
+        } else if (s->tile_log2 > 12) {
             s->tile_log2--;
             s->fused_next = b.fused;
         } else {

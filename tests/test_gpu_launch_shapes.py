@@ -1,0 +1,43 @@
+"""The launch shapes of the two-kernel pipeline: narrow calls (smaller tiles, clusters of eight
+tile CTAs sharing one scan, few 4-sets per engine warp) and the sizes where the shape changes.
+
+Bar: bit-exact against the oracle for narrow calls, and against the same range cut in two (other
+tiles, other groups) where a call fills the device.
+"""
+from __future__ import annotations
+
+import pytest
+
+from conftest import COUNTERS, assert_stats_equal
+from oracle import orc
+from ps4b200 import Search
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def wide():
+    with Search(1 << 44) as s:
+        yield s
+
+
+@pytest.mark.parametrize("lo", [1, 10 ** 6 + 7, 10 ** 9, 4 * 10 ** 11 + 1, 12 * 10 ** 12 + 5])
+@pytest.mark.parametrize("width", [1, 4095, 4097, 8 * 4096 + 1, 70001])
+def test_narrow_calls_vs_oracle(wide, lo, width):
+    r = wide.range(lo, lo + width)
+    rc, ost, olines, err = orc.search(lo, lo + width)
+    assert rc == 0, err
+    assert sorted(r.lines) == sorted(olines)
+    assert_stats_equal(r.stats, ost)
+
+
+# 592 tile CTAs: one tile of 2^13 S each and a little less or more; several groups per cluster
+@pytest.mark.parametrize("lo", [1, 10 ** 9, 10 ** 12])
+@pytest.mark.parametrize("width", [592 * 8192 - 1, 592 * 8192 + 1, 592 * 3 * 8192 + 4097])
+def test_shape_changes_vs_split_calls(wide, lo, width):
+    one = wide.range(lo, lo + width)
+    cut = lo + width // 3 + 1
+    a, b = wide.range(lo, cut), wide.range(cut, lo + width)
+    assert one.lines == a.lines + b.lines
+    for k in COUNTERS:
+        assert one.stats[k] == a.stats[k] + b.stats[k], k
