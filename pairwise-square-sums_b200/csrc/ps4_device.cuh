@@ -498,11 +498,159 @@ __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned 
     }
 }
 
+// The parity index of a list of k representations, sorted by p: ev[i], 0 <= i <= k, the number of even
+// p among the first i; pp[0..k) the positions of the even p, then those of the odd ones, each
+// ascending.  The j-th z of [z0, z1) whose p has a given parity is then one lookup.  Both lie in the
+// counters' area, which is free after P3; list s starts at ev[is_start[s] + s] and pp[is_start[s]].
+template <int TL>
+struct TileIndex {
+    using L = TileLayout<TL>;
+    static constexpr size_t OFF_EV = L::OFF_CNT, OFF_PP = OFF_EV + 2 * (size_t)(L::REP_CAP + L::IS_CAP);
+    static_assert(OFF_PP + 2 * (size_t)L::REP_CAP <= L::OFF_CNT + 2 * (size_t)L::W, "the index fits the counters' area");
+};
+
+// A list of more than 32 by one warp: ranks into `tmp`, one lane moves the elements (at most k swaps).
+static __device__ __noinline__ void sort_long(uint32_t *p, uint32_t *q, uint16_t *tmp, uint32_t k, int lane) {
+    for (uint32_t i = lane; i < k; i += 32) {
+        const uint32_t x = p[i];
+        uint32_t r = 0;
+        for (uint32_t j = 0; j < k; j++) r += p[j] < x;
+        tmp[i] = (uint16_t)r;
+    }
+    __syncwarp();
+    if (lane == 0)
+        for (uint32_t i = 0; i < k; i++)
+            while (tmp[i] != i) {
+                const uint32_t r = tmp[i], xp = p[r], xq = q[r];
+                p[r] = p[i]; q[r] = q[i]; p[i] = xp; q[i] = xq;
+                tmp[i] = tmp[r]; tmp[r] = (uint16_t)r;
+            }
+    __syncwarp();
+}
+
+// P4: every list ascending in p (distinct within a list), with its parity index where INDEX.  Three
+// quarters of the lists have at most four entries: one thread sorts such a list in registers.  Up to
+// eight entries, eight lanes rank one each (four lists of the warp at a time), longer lists take
+// the whole warp.  (One thread per list by insertion kept a warp waiting for its longest list:
+// 14 % of the tile kernel, 40,000 cycles for one tile at S = 4e11.)
+template <int TL, int NT, bool INDEX>
+__device__ __forceinline__ void sort_lists(unsigned char *smem, uint32_t n_is) {
+    using L = TileLayout<TL>;
+    const unsigned FULL = 0xffffffffu;
+    const uint16_t *is_k = (const uint16_t *)(smem + L::OFF_IS_K);
+    const uint16_t *is_start = (const uint16_t *)(smem + L::OFF_IS_START);
+    uint32_t *rep_p = (uint32_t *)(smem + L::OFF_REP_P);
+    uint32_t *rep_q = (uint32_t *)(smem + L::OFF_REP_Q);
+    uint16_t *ev_all = (uint16_t *)(smem + TileIndex<TL>::OFF_EV);
+    uint16_t *pp_all = (uint16_t *)(smem + TileIndex<TL>::OFF_PP);
+    const int lane = threadIdx.x & 31;
+    for (uint32_t base = threadIdx.x - lane; base < n_is; base += NT) {          // warp-uniform
+        const uint32_t s = base + lane;
+        const uint32_t k = s < n_is ? is_k[s] : 0, st = s < n_is ? is_start[s] : 0;
+        if (k == 3 || k == 4) {
+            uint32_t p[4], q[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                p[i] = i < (int)k ? rep_p[st + i] : 0xFFFFFFFFu;
+                q[i] = i < (int)k ? rep_q[st + i] : 0;
+            }
+            auto cx = [&](int i, int j) {
+                const bool sw = p[j] < p[i];
+                const uint32_t a = sw ? p[j] : p[i], b = sw ? p[i] : p[j], c = sw ? q[j] : q[i], d = sw ? q[i] : q[j];
+                p[i] = a; p[j] = b; q[i] = c; q[j] = d;
+            };
+            cx(0, 1); cx(2, 3); cx(0, 2); cx(1, 3); cx(1, 2);
+            uint32_t e = 0, ne = 0;
+            if (INDEX) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) ne += i < (int)k && !(p[i] & 1);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (i < (int)k) {
+                    rep_p[st + i] = p[i];
+                    rep_q[st + i] = q[i];
+                    if (INDEX) {
+                        ev_all[st + s + i] = (uint16_t)e;
+                        pp_all[st + (p[i] & 1 ? ne + i - e : e)] = (uint16_t)i;
+                        e += !(p[i] & 1);
+                    }
+                }
+            if (INDEX) ev_all[st + s + k] = (uint16_t)ne;
+        }
+        // five to eight entries: the next four such lists, one per eight lanes
+        for (unsigned m8 = __ballot_sync(FULL, k > 4 && k <= 8); m8;) {
+            int src = -1;
+#pragma unroll
+            for (int g = 0; g < 4; g++)
+                if (m8) {
+                    if (lane >> 3 == g) src = __ffs((int)m8) - 1;
+                    m8 &= m8 - 1;
+                }
+            const uint32_t gk0 = __shfl_sync(FULL, k, src & 31), gst = __shfl_sync(FULL, st, src & 31);
+            const uint32_t gk = src < 0 ? 0 : gk0, gs = base + src, i = lane & 7;
+            const bool mine = i < gk;
+            const uint32_t p = mine ? rep_p[gst + i] : 0xFFFFFFFFu, q = mine ? rep_q[gst + i] : 0;
+            uint32_t r = 0, e = 0, ne = 0;
+#pragma unroll
+            for (int x = 0; x < 8; x++) {
+                const uint32_t px = __shfl_sync(FULL, p, (lane & 24) | x);
+                const bool below = px < p, even = !(px & 1);                     // 0xFFFFFFFF: neither
+                r += below;
+                e += below && even;
+                ne += even;
+            }
+            __syncwarp();
+            if (mine) {
+                rep_p[gst + r] = p;
+                rep_q[gst + r] = q;
+                if (INDEX) {
+                    ev_all[gst + gs + r] = (uint16_t)e;
+                    pp_all[gst + (p & 1 ? ne + r - e : e)] = (uint16_t)r;
+                    if (i == 0) ev_all[gst + gs + gk] = (uint16_t)ne;
+                }
+            }
+        }
+        for (unsigned mb = __ballot_sync(FULL, k > 8); mb; mb &= mb - 1) {       // longer: one at a time
+            const int src = __ffs((int)mb) - 1;
+            const uint32_t gk = __shfl_sync(FULL, k, src), gst = __shfl_sync(FULL, st, src), gs = base + src;
+            if (gk <= 32) {
+                const bool mine = (uint32_t)lane < gk;
+                const uint32_t p = mine ? rep_p[gst + lane] : 0xFFFFFFFFu, q = mine ? rep_q[gst + lane] : 0;
+                uint32_t r = 0;
+                for (uint32_t x = 0; x < gk; x++) r += __shfl_sync(FULL, p, x) < p;
+                __syncwarp();
+                if (mine) { rep_p[gst + r] = p; rep_q[gst + r] = q; }
+            } else {
+                sort_long(rep_p + gst, rep_q + gst, pp_all + gst, gk, lane);
+            }
+            __syncwarp();
+            if (INDEX) {
+                uint32_t ne = 0, e = 0;
+                for (uint32_t x = 0; x < gk; x += 32)
+                    ne += __popc(__ballot_sync(FULL, x + lane < gk && !(rep_p[gst + x + lane] & 1)));
+                for (uint32_t x = 0; x < gk; x += 32) {
+                    const uint32_t z = x + lane;
+                    const bool even = z < gk && !(rep_p[gst + z] & 1);
+                    const unsigned m = __ballot_sync(FULL, even);
+                    const uint32_t ez = e + __popc(m & ((1u << lane) - 1u));
+                    if (z < gk) {
+                        ev_all[gst + gs + z] = (uint16_t)ez;
+                        pp_all[gst + (even ? ez : ne + z - ez)] = (uint16_t)z;
+                    }
+                    e += __popc(m);
+                }
+                if (lane == 0) ev_all[gst + gs + gk] = (uint16_t)ne;
+            }
+        }
+    }
+}
+
 // P1-P4 for one tile.  Returns false if the tile was abandoned (error raised).  With `list` (the
 // tile's representations from scan_group, list_n[w] entries in part w of `parts`, `cap` apart; other
 // CTAs of the cluster may have written them: read through L2) P1 and P3 read the list; without,
-// they scan.
-template <int TL, int NT = BS>
+// they scan.  INDEX: P4 also leaves each list's parity index (sort_lists).
+template <int TL, int NT = BS, bool INDEX = false>
 __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0, uint32_t n,
                           const uint64_t *list = nullptr, const uint32_t *list_n = nullptr, uint32_t parts = 0,
                           uint32_t cap = 0) {
@@ -557,7 +705,7 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
             if (i >= n) continue;
             kmax = max(kmax, k);
             if (k >= 3 && ((S0 + i) & 3) != 2) {
-                nI++; nR += k; nP += k * (k - 1) / 2;
+                nI++; nR += k; nP += (k - 1) * (k - 2) / 2;      // pairs (x,y) with a z above y
                 trip += (ull)k * (k - 1) * (k - 2) / 6;
                 if (k > a.cap_reps) over = true;
             }
@@ -601,7 +749,7 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
                     is_off[bI] = (uint16_t)ii; is_k[bI] = (uint16_t)k; is_start[bI] = (uint16_t)bR;
                     is_pbase[bI] = bP;
                     val = bR;
-                    bI++; bR += k; bP += k * (k - 1) / 2;
+                    bI++; bR += k; bP += (k - 1) * (k - 2) / 2;
                 }
             }
             word |= val << (h * 16);
@@ -628,15 +776,7 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
     }
     __syncthreads();
     // P4: each list ascending in p
-    for (uint32_t s = tid; s < ts.n_is; s += NT) {
-        const uint32_t st = is_start[s], k = is_k[s];
-        for (uint32_t x = st + 1; x < st + k; x++) {
-            const uint32_t kp = rep_p[x], kq = rep_q[x];
-            uint32_t y = x;
-            while (y > st && rep_p[y - 1] > kp) { rep_p[y] = rep_p[y - 1]; rep_q[y] = rep_q[y - 1]; y--; }
-            rep_p[y] = kp; rep_q[y] = kq;
-        }
-    }
+    sort_lists<TL, NT, INDEX>(smem, ts.n_is);
     __syncthreads();
     return true;
 }
@@ -784,13 +924,17 @@ __device__ __forceinline__ void block_add_ext_counters(TileShared &ts, ull c, ul
     }
 }
 
-// decode pair index j -> (x < y) with j = y(y-1)/2 + x
+// decode pair index j -> (x < y) with j = y(y-1)/2 + x.  j < 2^25 (lists of a tile are shorter than
+// 8192), so the estimate's floor is off by one at most.
 __device__ __forceinline__ void decode_pair(uint32_t j, uint32_t &x, uint32_t &y) {
-    uint32_t yy = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)j)) * 0.5f);
-    while (yy * (yy - 1) / 2 > j) yy--;
-    while ((yy + 1) * yy / 2 <= j) yy++;
+    float f;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"(1.0f + 8.0f * (float)j));
+    uint32_t yy = (uint32_t)((1.0f + f) * 0.5f);
+    uint32_t t = (yy * (yy - 1)) >> 1;
+    if (t > j) { yy--; t -= yy; }
+    if (t + yy <= j) { t += yy; yy++; }
     y = yy;
-    x = j - yy * (yy - 1) / 2;
+    x = j - t;
 }
 
 }  // namespace ps4

@@ -1,9 +1,9 @@
 // ps4_extend.cu -- the batched search as two persistent kernels per batch of S:
 //
 //   gen_jobs<TL,NT>  tiles of 2^TL S in shared memory (P1-P4 of ps4_device.cuh), then every
-//                 4-set of the tile (P5: closed-form z ranges per representation pair) is
-//                 written to a global job queue: a count pass, one block scan, one atomic
-//                 reservation per tile, a write pass.                         (s4.c:280-341)
+//                 4-set of the tile (P5: two searches per representation pair give the z intervals)
+//                 is written to a global job queue, each warp into stretches it reserves.
+//                                                                             (s4.c:280-341)
 //   extend_jobs   the extension engine.  Each lane of a warp holds one queued 4-set; it picks
 //                 the difference to extend by and factors it.  In rounds, the warp places the
 //                 factored odd-divisor lists of as many of its 4-sets as fit in its shared
@@ -162,78 +162,138 @@ __device__ __forceinline__ uint64_t ring_claim(const SearchArgs &a, uint32_t n, 
 
 // ================================================================== gen_jobs
 
-// The 4-sets of representation pair gidx of the tile (P5), pair given as list s and (x, y).
-// Counts them; with WRITE also builds, checks, dumps and (when `store`) queues them at out, ...
-template <bool WRITE, bool RING = false>
-__device__ __forceinline__ uint32_t pair_quads(const SearchArgs &a, uint32_t st, uint32_t k, uint64_t S,
-                                               uint32_t x, uint32_t y, const uint32_t *rep_p,
-                                               const uint32_t *rep_q, uint32_t item, uint64_t out, bool store) {
-    const uint32_t px = rep_p[st + x], py = rep_p[st + y];
-    const uint64_t Px = (uint64_t)px * px, Py = (uint64_t)py * py;
-    const uint32_t pxy = (px + py) & 1;
-    const uint32_t Sodd = (uint32_t)(S & 1);
-    uint32_t n = 0;
-    for (int cls = 0; cls < 2; cls++) {
-        // class 0: z upward while P_z < P_x + P_y;  class 1: z downward while P_z > S - P_x - P_y
-        const uint32_t want = cls == 0 ? 0u : Sodd;
-        for (uint32_t z = cls == 0 ? y + 1 : k - 1; z > y && z < k; z = cls == 0 ? z + 1 : z - 1) {
-            const uint32_t pz = rep_p[st + z];
-            const uint64_t Pz = (uint64_t)pz * pz;
-            if (cls == 0 ? Pz >= Px + Py : Pz <= S - Px - Py) break;
-            if (((pxy + pz) & 1) != want) continue;
-            const uint32_t qz = rep_q[st + z];
-            if (cls == 1 && qz == pz) continue;
-            if (WRITE) {
-                uint32_t r[6];
-                r[0] = rep_q[st + x]; r[1] = rep_q[st + y]; r[4] = py; r[5] = px;
-                r[2] = cls == 0 ? qz : pz;
-                r[3] = cls == 0 ? pz : qz;
-                if (a.flags & PS4_F_VERIFY) {
-                    uint64_t v[4], Sq;
-                    quad_values(r, v, Sq);
-                    if (!quad_roots_ok(v, r)) record_verify_failure(a, S, v);
-                }
-                if (a.flags & PS4_F_DUMP4) dump_quad(a, r);
-                if (store) {
-                    if (!RING) {
-                        put_job(a.jobs, out + n, r, item);
-                    } else if (ring_wait_free(a, out + n)) {
-                        put_job(a.jobs, (out + n) & a.ring_mask, r, item);
-                    }
-                }
-            }
-            n++;
-        }
+// P5: the 4-sets of a representation pair x < y are its z > y with, in class 0, P_z < P_x + P_y (P =
+// p^2) and p_z of p_x + p_y's parity, and, in class 1, P_z > S - P_x - P_y, p_z of that parity or, for
+// odd S, the other, and q_z != p_z (which only the last z can violate).  Both are intervals of the
+// sorted list, found by two binary searches, and the list's parity index turns them into a count and
+// the j-th z of each.  (A loop over z per pair, once to count and once to write, took 42 % of the
+// tile kernel: 82,000 of a tile's 190,000 cycles at S = 4e11.  Per [1,1e10) step of the tile kernel
+// 141.4 -> 99.5 ms with this and the lane-wise sort of P4; 2e8 S at 1e12 4.76 -> 3.36, 3e7 at 1.2e13 1.63 -> 1.10.)
+struct TileView {
+    const uint16_t *off, *k, *start;
+    const uint32_t *pbase, *rep_p, *rep_q;
+    const uint16_t *ev, *pp;
+    uint32_t n_is;
+};
+struct PairSets {
+    uint32_t sx;                       // list start | x << 16
+    uint32_t ya;                       // y | 4-sets of class 0 << 16
+    uint32_t ab;                       // first z of class 0 | of class 1 << 16, as places in the parity index
+};
+
+// The pairs g of a warp, one per lane (32 consecutive ones; ge ends the warp's block): each lane's
+// number of 4-sets and where they are.  lo0: a selected S not after the first pair's, warp-uniform;
+// moved on to the last one's.
+__device__ __forceinline__ uint32_t pair_sets(const TileView &v, uint64_t S0, uint32_t g, uint32_t ge, int lane,
+                                              uint32_t &lo0, PairSets &ps) {
+    // every selected S has a pair at least, so 32 consecutive pairs lie in 32 consecutive ones
+    const uint32_t pb = lo0 + lane < v.n_is ? v.pbase[lo0 + lane] : 0xFFFFFFFFu;
+    uint32_t o = 0;
+#pragma unroll
+    for (uint32_t step = 16; step; step >>= 1)
+        if (__shfl_sync(0xffffffffu, pb, o + step) <= g) o += step;
+    const uint32_t base = __shfl_sync(0xffffffffu, pb, o);
+    const uint32_t lo = lo0 + o;
+    lo0 = __shfl_sync(0xffffffffu, lo, 31);
+    if (g >= ge) return 0;
+    const uint32_t st = v.start[lo], k = v.k[lo];
+    const uint64_t S = S0 + v.off[lo];
+    uint32_t x, y;
+    decode_pair(g - base, x, y);
+    const uint32_t *p = v.rep_p + st;
+    const uint16_t *ev = v.ev + st + lo;
+    const uint32_t px = p[x], py = p[y];
+    const uint64_t T = (uint64_t)px * px + (uint64_t)py * py, U = S - T;
+    uint32_t za = y + 1, zb = y + 1, n = k - 1 - y;        // first z with P_z >= T / with P_z > U
+    while (n > 1) {
+        const uint32_t h = n >> 1, pa = p[za + h - 1], pb2 = p[zb + h - 1];
+        if ((uint64_t)pa * pa < T) za += h;
+        if ((uint64_t)pb2 * pb2 <= U) zb += h;
+        n -= h;
     }
-    return n;
+    {
+        const uint32_t pa = p[za], pb2 = p[zb];
+        if ((uint64_t)pa * pa < T) za++;
+        if ((uint64_t)pb2 * pb2 <= U) zb++;
+    }
+    const uint32_t oa = (px + py) & 1u, ob = oa ^ ((uint32_t)S & 1u);     // the parity of p_z in each class
+    const uint32_t ne = ev[k];
+    const uint32_t e0 = ev[y + 1], ea = ev[za], eb = ev[zb];
+    const uint32_t a0 = oa ? y + 1 - e0 : e0, a1 = oa ? za - ea : ea;
+    const uint32_t b0 = ob ? zb - eb : eb, b1 = ob ? k - ne : ne;
+    const uint32_t na = a1 - a0;
+    uint32_t nb = b1 - b0;
+    if (nb && !(S & 1) && p[k - 1] == v.rep_q[st + k - 1]) nb--;         // even S: ob is every p's parity
+    ps.sx = st | x << 16;
+    ps.ya = y | na << 16;
+    ps.ab = (st + (oa ? ne : 0) + a0) | (st + (ob ? ne : 0) + b0) << 16;
+    return na + nb;
 }
 
-// A lane's share of P5: the pairs g = gw + lane, gw + lane + 32, ... below ge of its warp's
-// contiguous block.  Neighbouring lanes take neighbouring pairs (mostly the same S), and each
-// lane finds its pair's S by one binary search, then by stepping forward.
-template <bool WRITE, bool RING = false>
-__device__ __forceinline__ uint32_t lane_pairs(const SearchArgs &a, uint32_t gw, uint32_t ge, int lane, uint32_t nI,
-                                               const uint16_t *is_off, const uint16_t *is_k,
-                                               const uint16_t *is_start, const uint32_t *is_pbase,
-                                               const uint32_t *rep_p, const uint32_t *rep_q, uint64_t S0,
-                                               uint32_t item, uint64_t out, bool store) {
-    uint32_t g = gw + (uint32_t)lane;
-    if (g >= ge) return 0;
-    uint32_t lo = 0, hi = nI;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (is_pbase[mid] <= g) lo = mid; else hi = mid;
+// The write pass of one warp step: the lanes' 4-sets (n each, places ps) are spread evenly over the
+// warp, 32 per turn, checked and dumped where asked, and queued (when `store`): the first `rem` at
+// `cur`, those after them at `next`.
+template <bool RING>
+__device__ __forceinline__ void write_sets(const SearchArgs &a, const TileView &v, uint32_t n, const PairSets &ps,
+                                           uint32_t first, uint32_t total, int lane, uint64_t S0, uint32_t item,
+                                           bool store, uint64_t cur, uint32_t rem, uint64_t next) {
+    for (uint32_t t = 0; t < total; t += 32) {
+        const uint32_t s = t + lane;
+        uint32_t o = 0;                                                  // the last lane with first <= s
+#pragma unroll
+        for (uint32_t step = 16; step; step >>= 1)
+            if (__shfl_sync(0xffffffffu, first, o + step) <= s) o += step;
+        const uint32_t f = __shfl_sync(0xffffffffu, first, o), sx = __shfl_sync(0xffffffffu, ps.sx, o),
+                       ya = __shfl_sync(0xffffffffu, ps.ya, o), ab = __shfl_sync(0xffffffffu, ps.ab, o);
+        if (s >= total) continue;
+        const uint32_t st = sx & 0xFFFFu, x = st + (sx >> 16), y = st + (ya & 0xFFFFu), na = ya >> 16;
+        uint32_t j = s - f;
+        const bool one = j >= na;                                        // class 1
+        j = one ? (ab >> 16) + j - na : (ab & 0xFFFFu) + j;
+        const uint32_t z = st + v.pp[j];
+        const uint32_t pz = v.rep_p[z], qz = v.rep_q[z];
+        uint32_t r[6];
+        r[0] = v.rep_q[x]; r[1] = v.rep_q[y]; r[4] = v.rep_p[y]; r[5] = v.rep_p[x];
+        r[2] = one ? pz : qz;
+        r[3] = one ? qz : pz;
+        if (a.flags & (PS4_F_VERIFY | PS4_F_DUMP4)) {
+            uint64_t m[4], S;
+            quad_values(r, m, S);
+            if ((a.flags & PS4_F_VERIFY) && !quad_roots_ok(m, r)) record_verify_failure(a, S, m);
+            if (a.flags & PS4_F_DUMP4) dump_quad(a, r);
+        }
+        if (store) {
+            const uint64_t pos = s < rem ? cur + s : next + (s - rem);
+            if (!RING) {
+                put_job(a.jobs, pos, r, item);
+            } else if (ring_wait_free(a, pos)) {
+                put_job(a.jobs, pos & a.ring_mask, r, item);
+                __threadfence();
+                *(volatile uint32_t *)&a.seq[pos & a.ring_mask] = (uint32_t)(pos + 1);
+            }
+        }
     }
-    uint32_t n = 0;
-    for (; g < ge; g += 32) {
-        while (lo + 1 < nI && is_pbase[lo + 1] <= g) lo++;
-        uint32_t x, y;
-        decode_pair(g - is_pbase[lo], x, y);
-        n += pair_quads<WRITE, RING>(a, is_start[lo], is_k[lo], S0 + is_off[lo], x, y, rep_p, rep_q, item, out + n,
-                                     store);
-    }
-    return n;
 }
+
+// a warp's exclusive prefix of n, and its total
+__device__ __forceinline__ uint32_t warp_prefix(uint32_t n, int lane, uint32_t &total) {
+    uint32_t i = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, i, o);
+        if (lane >= o) i += y;
+    }
+    total = __shfl_sync(0xffffffffu, i, 31);
+    return i - n;
+}
+
+// A warp's open stretch of the job queue: a.chunk records at a time are reserved (one atomic), so that
+// the tile needs no count pass and no barrier before its 4-sets are written.  What is left at the
+// kernel's end is filled with empty records, which the engine passes over.
+struct JobSpan {
+    uint64_t cur = 0;
+    uint32_t rem = 0;
+};
 
 // The segment of tile ti: the last one whose first tile is not after it.
 __device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
@@ -246,43 +306,57 @@ __device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
 }
 
 // One tile [S0, S0+n) of query item `item`: P1-P4 (from its list's parts, or by scanning when list
-// is null), the count pass, one reservation for the tile's 4-sets, the write
-// pass.  NT threads.  RING: the 4-sets go to the persistent kernel's ring and each lane publishes
-// its contiguous run after a fence.
+// is null), then P5: each warp takes a contiguous block of the tile's pairs, 32 at a time.  NT threads.
+// The tile kernel (RING false) queues what a step finds in the warp's open stretch.  The persistent
+// kernel counts first and reserves the tile's 4-sets at once (the ring's room is waited for), and
+// each 4-set is published after a fence.
 template <int TL, int NT, bool RING>
-__device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0, uint32_t n,
-                                             uint32_t item, const uint64_t *list, const uint32_t *list_n,
-                                             uint32_t parts, uint32_t cap, unsigned long long &s_base, int &s_store) {
+__device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0,
+                                             uint32_t n, uint32_t item, const uint64_t *list,
+                                             const uint32_t *list_n, uint32_t parts, uint32_t cap, JobSpan &span,
+                                             unsigned long long &s_base, int &s_store) {
     using L = TileLayout<TL>;
     constexpr int NW = NT / 32;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const bool noext = (a.flags & PS4_F_NOEXT) != 0;
     const bool need_write_pass = !noext || (a.flags & (PS4_F_DUMP4 | PS4_F_VERIFY));
     tile_reset(ts);
     __syncthreads();
-    if (!tile_reps<TL, NT>(a, ts, smem, S0, n, list, list_n, parts, cap)) { __syncthreads(); return; }
-    const uint16_t *is_off = (const uint16_t *)(smem + L::OFF_IS_OFF);
-    const uint16_t *is_k = (const uint16_t *)(smem + L::OFF_IS_K);
-    const uint16_t *is_start = (const uint16_t *)(smem + L::OFF_IS_START);
-    const uint32_t *is_pbase = (const uint32_t *)(smem + L::OFF_IS_PBASE);
-    const uint32_t *rep_p = (const uint32_t *)(smem + L::OFF_REP_P);
-    const uint32_t *rep_q = (const uint32_t *)(smem + L::OFF_REP_Q);
-    const uint32_t nI = ts.n_is, nPairs = ts.n_pairs;
-    // count pass, one reservation for the tile, write pass in the same order
-    // each warp a contiguous block of pairs (whole multiples of 32)
-    const int lane = tid & 31, wid = tid >> 5;
+    if (!tile_reps<TL, NT, true>(a, ts, smem, S0, n, list, list_n, parts, cap)) { __syncthreads(); return; }
+    TileView v;
+    v.off = (const uint16_t *)(smem + L::OFF_IS_OFF);
+    v.k = (const uint16_t *)(smem + L::OFF_IS_K);
+    v.start = (const uint16_t *)(smem + L::OFF_IS_START);
+    v.pbase = (const uint32_t *)(smem + L::OFF_IS_PBASE);
+    v.rep_p = (const uint32_t *)(smem + L::OFF_REP_P);
+    v.rep_q = (const uint32_t *)(smem + L::OFF_REP_Q);
+    v.ev = (const uint16_t *)(smem + TileIndex<TL>::OFF_EV);
+    v.pp = (const uint16_t *)(smem + TileIndex<TL>::OFF_PP);
+    v.n_is = ts.n_is;
+    const uint32_t nPairs = ts.n_pairs;
+    // each warp a contiguous block of pairs (whole multiples of 32), and the S of its first one
     const uint32_t blk = ((nPairs + NW * 32 - 1) / (NW * 32)) * 32;
     const uint32_t gw = (uint32_t)wid * blk, ge = min(nPairs, gw + blk);
-    uint32_t mine = lane_pairs<false>(a, gw, ge, lane, nI, is_off, is_k, is_start, is_pbase, rep_p, rep_q, S0, item, 0,
-                                      false);
-    uint32_t off, d1, d2, tot[3];
-    block_scan3<NT>(mine, 0u, 0u, off, d1, d2, tot, ts.wsum);
-    if (tid == 0) {
-        ts.cnt[K_SETS4] += tot[0];
-        s_base = 0;
-        s_store = 0;
-        if (!noext && tot[0]) {
-            if (RING) {
+    uint32_t lo0 = 0;
+    if (gw < ge) {
+        uint32_t hi = v.n_is;
+        while (hi - lo0 > 1) {
+            const uint32_t mid = (lo0 + hi) >> 1;
+            if (v.pbase[mid] <= gw) lo0 = mid; else hi = mid;
+        }
+    }
+    PairSets ps;
+    uint32_t mine = 0, total;
+    if (RING) {
+        const uint32_t lo_first = lo0;
+        for (uint32_t g = gw; g < ge; g += 32) mine += pair_sets(v, S0, g + lane, ge, lane, lo0, ps);
+        lo0 = lo_first;
+        uint32_t off, d1, d2, tot[3];
+        block_scan3<NT>(mine, 0u, 0u, off, d1, d2, tot, ts.wsum);
+        if (tid == 0) {
+            s_base = 0;
+            s_store = 0;
+            if (!noext && tot[0]) {
                 // room: the ring holds the reserved-but-unfinished 4-sets plus this tile's
                 WaitClock wc;
                 bool ok = true;
@@ -294,28 +368,54 @@ __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts
                     s_base = atomicAdd(&a.status->q_tail, (ull)tot[0]);
                     s_store = 1;
                 }
-            } else {
-                s_base = atomicAdd(&a.status->n_jobs, (ull)tot[0]);
-                if (s_base + tot[0] <= a.jobs_cap) s_store = 1;
-                else raise_capacity(a.status, E_QUEUE, 5, s_base + tot[0], a.jobs_cap, S0);
+            }
+        }
+        __syncthreads();
+        if (need_write_pass) {
+            uint64_t cur = s_base + __shfl_sync(0xffffffffu, off, 0);
+            for (uint32_t g = gw; g < ge; g += 32) {
+                const uint32_t m = pair_sets(v, S0, g + lane, ge, lane, lo0, ps);
+                const uint32_t first = warp_prefix(m, lane, total);
+                write_sets<true>(a, v, m, ps, first, total, lane, S0, item, s_store != 0, cur, total, 0);
+                cur += total;
+            }
+        }
+        __syncthreads();
+        if (tid == 0 && s_store && tot[0]) atomicAdd(&a.status->q_pub, (ull)tot[0]);
+    } else {
+        for (uint32_t g = gw; g < ge; g += 32) {
+            const uint32_t m = pair_sets(v, S0, g + lane, ge, lane, lo0, ps);
+            mine += m;
+            if (!need_write_pass) continue;                              // warp-uniform
+            const uint32_t first = warp_prefix(m, lane, total);
+            if (total == 0) continue;
+            uint64_t next = 0;
+            uint32_t room = 0;
+            bool store = !noext;
+            if (store && total > span.rem) {
+                room = max(a.chunk, total - span.rem);
+                if (lane == 0) next = atomicAdd(&a.status->n_jobs, (ull)room);
+                next = __shfl_sync(0xffffffffu, next, 0);
+                if (next + room > a.jobs_cap) {
+                    if (lane == 0) raise_capacity(a.status, E_QUEUE, 5, next + room, a.jobs_cap, S0);
+                    store = false;
+                }
+            }
+            write_sets<false>(a, v, m, ps, first, total, lane, S0, item, store, span.cur, span.rem, next);
+            if (store) {
+                if (room) {
+                    span.cur = next + (total - span.rem);
+                    span.rem = room - (total - span.rem);
+                } else {
+                    span.cur += total;
+                    span.rem -= total;
+                }
             }
         }
     }
+    const ull found = warp_sum((ull)mine);
+    if (lane == 0 && found) atomicAdd(&ts.cnt[K_SETS4], found);
     __syncthreads();
-    if (need_write_pass) {
-        const bool store = s_store != 0;
-        lane_pairs<true, RING>(a, gw, ge, lane, nI, is_off, is_k, is_start, is_pbase, rep_p, rep_q, S0, item,
-                               s_base + off, store);
-        if (RING && store && mine) {               // publish this lane's run [s_base+off, +mine)
-            __threadfence();
-            for (uint32_t i = 0; i < mine; i++) {
-                const uint64_t pos = s_base + off + i;
-                *(volatile uint32_t *)&a.seq[pos & a.ring_mask] = (uint32_t)(pos + 1);
-            }
-        }
-    }
-    __syncthreads();
-    if (RING && tid == 0 && s_store && tot[0]) atomicAdd(&a.status->q_pub, (ull)tot[0]);
     tile_flush_counters(a, ts, item);
     __syncthreads();
 }
@@ -327,6 +427,7 @@ template <int TL, int NT>
 __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t c0,
                                   uint64_t *lists, uint32_t *raw_n, unsigned long long &s_base, int &s_store) {
     using L = TileLayout<TL>;
+    JobSpan span;
     const uint64_t cn = min((uint64_t)SUPER_K, a.n_tiles - c0);
     uint64_t ti = a.n_tiles - c0 - cn;
     const uint64_t ti_end = a.n_tiles - c0;
@@ -345,7 +446,7 @@ __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned 
             const uint64_t S0 = SA + ((uint64_t)j << TL);
             produce_tile<TL, NT, true>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
                                        raw_n[j] <= a.raw_cap ? lists + (size_t)j * a.raw_cap : nullptr, &raw_n[j], 1,
-                                       a.raw_cap, s_base, s_store);
+                                       a.raw_cap, span, s_base, s_store);
         }
         ti = g_end;
     }
@@ -364,6 +465,7 @@ __global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const SearchArgs a) 
     __shared__ TileShared ts;
     __shared__ unsigned long long s_base, s_claim;
     __shared__ int s_store;
+    JobSpan span;
     __shared__ uint32_t s_tile, s_fit;
     // entries that this CTA's scan appended to each tile's list, and the next tile to take (CTA 0's
     // is used).  Two sets, one for each parity of the group: a set is cleared while the other one's
@@ -419,11 +521,14 @@ __global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const SearchArgs a) 
             __syncthreads();
             const uint64_t S0 = SA + ((uint64_t)j << TL);
             produce_tile<TL, NT, false>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
-                                        s_fit ? lists + (size_t)j * nc * cap : nullptr, s_n, nc, cap, s_base, s_store);
+                                        s_fit ? lists + (size_t)j * nc * cap : nullptr, s_n, nc, cap, span, s_base,
+                                        s_store);
         }
         __syncthreads();                                                 // s_tile read by all
         ti = g_end;
     }
+    const uint32_t none[6] = {0, 0, 0, 0, 0, 0};
+    for (uint32_t i = tid & 31; i < span.rem; i += 32) put_job(a.jobs, span.cur + i, none, 0);
     cluster.sync();                          // no CTA leaves while another may read its shared memory
 }
 
@@ -689,6 +794,7 @@ template <bool COH>
 __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJob &J, uint32_t (*fp)[32],
                                           int lane) {
     get_job<COH>(a.jobs, j, J.r, J.item);
+    if (J.r[0] == 0) return false;                 // an empty record (the end of a tile warp's stretch)
     quad_values(J.r, J.v, J.S);
     uint32_t best;
     choose_pair(J.v, J.r, a.ndiv, J.bi, J.bj, J.bk, best);
@@ -1212,6 +1318,11 @@ int launch_gen(SearchArgs a, int grid, void *stream) {
     const uint64_t K = std::min(fit, want), ctas = K * cl;
     const double G = std::min(std::sqrt(2 * n * scan / (double)K), std::ceil(n / (double)K));
     a.group = (uint32_t)std::min<double>(std::max<double>(G, cl), cl * SUPER_K);
+    // a warp's reservations: a sixteenth of its expected share of about 0.2 4-sets per S, so that the
+    // empty records at the end stay below a few percent, 128 at most (one atomic per 128 4-sets)
+    const double warps = (double)ctas * gen_threads(a.log2_tile) / 32;
+    const double share = 0.2 * std::ldexp(n, (int)a.log2_tile) / warps;
+    a.chunk = (uint32_t)std::min<double>(std::max<double>(share / 16, 8), 128);
     switch (a.log2_tile) {
         case 12: return launch_gen_tl<12>(a, (int)ctas, cl, s);
         case 13: return launch_gen_tl<13>(a, (int)ctas, cl, s);

@@ -85,7 +85,8 @@ struct SearchArgs {
     uint64_t *raw;             // tile and persistent kernel: per CTA, SUPER_K lists of one tile's
     uint32_t raw_cap;          //   representations, raw_cap entries each (a cluster pools its CTAs' lists)
     uint64_t s_top;            // the launch's largest S, for the tile kernel's launch shape
-    uint32_t group;            // tile kernel: tiles a cluster claims at once (set by launch_gen)
+    uint32_t group;            // tile kernel: tiles a cluster claims at once, and job records a warp
+    uint32_t chunk;            //   reserves at once (both set by launch_gen)
     // persistent kernel: jobs is a ring of jobs_cap (a power of two) slots; seq[slot] tells its state
     // for position pos = slot + lap * jobs_cap: pos = free for pos, pos + 1 = 4-set of pos written
     uint32_t *seq;

@@ -41,3 +41,24 @@ def test_shape_changes_vs_split_calls(wide, lo, width):
     assert one.lines == a.lines + b.lines
     for k in COUNTERS:
         assert one.stats[k] == a.stats[k] + b.stats[k], k
+
+
+# S with 3 .. 288 representations, odd, = 4 and = 0 mod 8 (among these some twice a square, whose last
+# representation has p = q): the list lengths at which the tile kernel's sort changes its way, and the
+# lengths of its searches
+LISTS = {3: (15317, 61268), 4: (80401, 643208), 5: (33125, 132500), 7: (180625, 1445000), 8: (2331629, 18653032),
+         9: (2588573, 10354292), 13: (1221025, 9768200), 16: (39637693, 317101544), 31: (763140625, 6105125000),
+         32: (515290009, 4122320072), 36: (3926865241, 31414921928), 63: (40446453125, 323571625000),
+         64: (87084011521, 696672092168), 96: (1480428195857, 11843425566856), 192: (8708401152100, 17416802304200),
+         288: (14234886498625,)}
+
+
+@pytest.mark.parametrize("k", sorted(LISTS))
+def test_list_lengths_vs_oracle(wide, k):
+    for S in LISTS[k]:
+        r = wide.range(S, S + 1)
+        rc, ost, olines, err = orc.search(S, S + 1)
+        assert rc == 0, err
+        assert ost["max_reps"] in (k, k + 1)          # one more for twice a square
+        assert sorted(r.lines) == sorted(olines)
+        assert_stats_equal(r.stats, ost)
