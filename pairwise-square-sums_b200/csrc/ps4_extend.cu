@@ -4,22 +4,29 @@
 //                 4-set of the tile (P5: two searches per representation pair give the z intervals)
 //                 is written to a global job queue, each warp into stretches it reserves.
 //                                                                             (s4.c:280-341)
-//   extend_jobs   the extension engine.  Each lane of a warp holds one queued 4-set; it picks
-//                 the difference to extend by and factors it.  In rounds, the warp places the
-//                 factored odd-divisor lists of as many of its 4-sets as fit in its shared
-//                 buffer, pools the candidates of those 4-sets -- the complementary divisor
-//                 pairs (f,g), f<g, of equal parity, each visited once -- and splits them into
-//                 32 equal contiguous runs, one per lane, so every lane does the same work
-//                 whatever the divisor counts; lanes whose 4-set is done take the next one from
-//                 the queue before the next round.  Residue filters mod 64/63/65 are bit tests
-//                 against per-4-set masks indexed by u's residue; the candidates that pass (the
-//                 reference's ext_sqrt) go through a warp queue and are square-tested 32 at a
-//                 time.                                                        (s4.c:160-207)
+//   extend_jobs   the extension engine.  Each lane of a warp takes one queued 4-set, picks the
+//                 difference to extend by and factors it (phase A).  The candidates of the
+//                 round's 4-sets -- the complementary divisor pairs (f,g), f<g, of equal parity,
+//                 each visited once -- are products of two short divisor lists in shared memory,
+//                 and come in rows: one divisor of the shorter list (and power of two) against
+//                 the whole longer list.  Rows are taken longest first, 32 at a time, one per
+//                 lane, so a row's factors are set up once and its candidates take two
+//                 multiplications each.  Residue filters mod 64/63/65 are bit tests against
+//                 per-4-set masks indexed by residues of f + g = 2u; the candidates that pass go
+//                 through a warp queue, where those that are the reference's ext_sqrt are
+//                 square-tested 32 at a time.                                  (s4.c:160-207)
+//
+// The engine is bound by instruction issue (67 % of issue slots busy, 28.8 of 32 threads active; DRAM 2.5 %).
+// Per [1,1e10) search its launches take 192 ms; with candidates spread over the lanes in 32 equal
+// runs, u64 lists, per-candidate member tests and IEEE double square roots they took 313 ms (25.5 -> 15.8 warp
+// instructions per S).  Rows cost a partly empty turn (30.2 turns of 32 candidates per round against
+// 24.9 full ones) and save the per-candidate bookkeeping, half of the 85 instructions of the old loop.
 //
 // Every counter and every reported line is identical to the reference's.
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -459,7 +466,7 @@ __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned 
 // by one from a common counter.  A scan costs ~0.29 sqrt(S) steps however few S it covers, and a
 // narrow call has too few tiles for one CTA each on a scan of its own, so both ends gain from sharing it.
 template <int TL, int NT>
-__global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const SearchArgs a) {
+__global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const __grid_constant__ SearchArgs a) {
     using L = TileLayout<TL>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileShared ts;
@@ -536,110 +543,170 @@ __global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const SearchArgs a) 
 
 constexpr int EBS = 256;                 // threads per CTA
 constexpr int EWARPS = EBS / 32;
-constexpr int DCAP = 416;                // divisor-list entries per warp (u64)
-constexpr int QCAP = 64;                 // square-test queue per warp
+constexpr int DCAP = 560;                // divisor-list entries per warp (u32)
+constexpr int LCAP = 128;                // divisors per list at most (longer ones take the per-lane walk)
+constexpr int QCAP = 96;                 // square-test queue per warp
 constexpr int EXCAP = 8;                 // extensions per warp and round
-constexpr int FSLOT = 16;                // prime slots per lane: m1's primes from 0, m2's from 8
+constexpr int FSIDE = 7;                 // odd primes of a number below 2^23 at most
+constexpr int ICACHE = 8;                // items whose counters a warp holds back
 
-// The odd part D_odd of a difference is kept factored: its odd primes are split into a low
-// group (the first primes of the reference's order) and a high group, with divisor lists
-// lo[0..L) and hi[0..H) in mixed-radix order.  The odd divisor with mixed-radix index
-// t = l + L*h is lo[l]*hi[h], and its complement (index ndo-1-t) is lo[L-1-l]*hi[H-1-h]:
-// L+H entries instead of ndo = L*H.
-struct __align__(16) EJob {              // one lane's 4-set, read by every lane in phase B
-    uint64_t m64, m63, m65;              // bit s: u^2 + (C - A) is a residue for both C (mod 64/63/65)
-    uint32_t rA0, rA1;                   // rA0..rA2: the roots sqrt(A + v) of the three other members
-    uint32_t uA, rAA, rA2, ncand;        // u <= uA: e <= 0; rAA = sqrt(2A) if integral, else 0;
-                                         //   e = u^2 - A is a member of the 4-set iff u is one of
-                                         //   rAA, rA0, rA1, rA2
-    uint16_t base, L, H;                 // lo list at dbuf[base..base+L), hi list right after it
-    uint8_t E2, flags;                   // flags: 1 = D even
-    uint64_t A;                          // extend by D = A - B
-    uint64_t C1, C2;                     // the other two members (square tests)
+// The odd part of a difference D = m1*m2 is kept factored as two coprime numbers below 2^32 (m1's
+// odd primes, with the powers that m2 adds to them, and m2's others; a prime moves to the other side
+// where that evens out the divisor counts).  The longer of their divisor lists is the row list x[0..L),
+// the other y[0..H), each in mixed-radix order of its primes.  The odd divisor (l, h) is x[l]*y[h], its
+// complement x[L-1-l]*y[H-1-h].  With D = 2^E2 * odd, the candidates -- complementary divisor pairs (f,
+// g) of equal parity -- are (l, h, d): f = x[l]*y[h] << s, g = the complement << E2-s, with s = d + 1, 0 <= d <
+// E2 - 1, for even D and s = 0 for odd D.  In the order l fastest, then h, then d, complements lie at
+// mirrored places, so the first half of the sequence visits each pair once: full rows of L
+// candidates, and half a row at the end when the number of rows is odd.
+struct __align__(16) EJob {              // one lane's 4-set
+    uint64_t m63, m65;                   // residue masks of f + g = 2u (see VResTabs)
+    uint32_t m64, geo;                   // geo: L | H << 8 | E2 << 16 | list place << 22
+    uint64_t A;                          // extend by D = A - B: e = u^2 - A
+    int64_t d1, d2;                      // C - A of the other two members (square tests of u^2 + (C - A))
+    uint32_t rA0, rA1, rA2;              // the roots sqrt(A + v) of the three other members: e is one of
+                                         //   them iff u is one of these
+    uint32_t item;                       // | ext_sqrt << 20 where the round's items differ (a 4-set has
+                                         //   fewer than 2^12 candidates: no number below 2^44 has 2^14 divisors)
+};
+static_assert(sizeof(EJob) == 64 && offsetof(EJob, d1) == 32 && offsetof(EJob, rA0) == 48, "vector loads of job fields");
+static_assert(LCAP <= 255 && DCAP <= 1024, "fields of geo");
+
+struct ItemCount {                       // counters of an item that the warp holds back
+    uint32_t item, mdiv;
+    ull cand, sqrt_;
 };
 
+// 6.8 KB: three CTAs take 167 KB, which leaves 92 KB of L1 for the table lookups of phase A (with 8.6 KB
+// areas it was 28 KB)
 struct WarpArea {
-    uint64_t dbuf[DCAP];
     EJob job[32];
-    uint32_t cstart[33];
-    uint32_t qidx[QCAP];                 // candidate: l | h << 12 | d2 << 24
-    uint64_t qu[QCAP];
-    uint8_t qj[QCAP];
+    uint32_t dbuf[DCAP];                 // a turn may read up to LCAP entries past a list's ends: the
+                                         //   neighbours on both sides are longer than that
+    union {                              // primes until the lists are made, then the queue
+        uint32_t fp[2 * FSIDE][32];      // each lane's odd primes of D (p | e << 24), m1's from slot 0, m2's
+                                         //   others from FSIDE, lane-minor (no bank conflicts)
+        uint64_t q[QCAP];                // candidates that pass the filters: f + g | job << 58
+    };
+    ItemCount ic[ICACHE];
     ExtEntry ext[EXCAP];
-    uint32_t fp[FSLOT][32];              // each lane's primes of D with their exponents (p | e << 24),
-                                         //   lane-minor (no bank conflicts)
-    uint32_t jsq[32];                    // ext_sqrt of each lane's 4-set in this round
     uint32_t jid[32];                    // queue index of each lane's 4-set
     uint32_t n_ext;
+    uint8_t order[32];                   // lanes by row length, longest first
 };
+static_assert(sizeof(EJob) * 32 >= 4 * LCAP && 4 * 32 * 2 * FSIDE >= 4 * LCAP, "neighbours of dbuf");
+static_assert(EWARPS * sizeof(WarpArea) + 1024 <= 164 * 1024 / 3, "three engine CTAs per SM in the 164 KB carve-out");
 
-static_assert(EWARPS * sizeof(WarpArea) + 1024 <= 228 * 1024 / 3, "three engine CTAs per SM");
-
-// Residue masks indexed by u's residue: bit w of q_m[a] is set iff w^2 + a is a square mod m.
-// A 4-set's mask for its two remaining members C1, C2 is q_m[(C1-A) mod m] & q_m[(C2-A) mod m],
-// so the filters of e + C = u^2 + (C - A) (s4.c:192-194) become one bit test per modulus on
-// u mod m.  Mod 65 has 65 residues, but 64 = -1 and 1 have the same square, so bit 64 equals
-// bit 1 and residue 64 is looked up as 1.
-struct UResTabs {
-    uint64_t q64[64], q63[63], q65[65];
+// Residue masks of a candidate's v = f + g = 2u.  e + C = u^2 + (C - A) must be a square mod 64, 63
+// and 65 for both remaining members C (s4.c:192-194): one bit test per modulus, against the AND of
+// the two members' masks q_m[(C - A) mod m].
+//  * mod 64: u^2 mod 64 depends on u mod 32, bit v/2 mod 32.
+//  * mod 63 and 65: with x = (v >> 24) + (v & 0xFFFFFF) + 32 = v + 32 (2^24 = 1 in both), bit x mod 63, and bit (x
+//    mod 65) mod 64: x = 0 and 64 mod 65 are v = -32 and 32, whose squares are equal, so 65 residues
+//    fit 64 bits.
+struct VResTabs {
+    uint64_t q63[63], q65[65];
+    uint32_t q64[64];
 };
 constexpr bool is_qr_mod(int m, int r) {
     return r < 64 ? ((qr_bits(m) >> r) & 1) != 0 : true;          // r = 64 (m = 65) is 8^2
 }
-constexpr UResTabs make_ures() {
-    UResTabs t{};
-    for (int a = 0; a < 64; a++) {
-        uint64_t x = 0;
-        for (int w = 0; w < 64; w++) if (is_qr_mod(64, (w * w + a) % 64)) x |= 1ull << w;
-        t.q64[a] = x;
-    }
-    for (int a = 0; a < 63; a++) {
-        uint64_t x = 0;
-        for (int w = 0; w < 63; w++) if (is_qr_mod(63, (w * w + a) % 63)) x |= 1ull << w;
-        t.q63[a] = x;
-    }
-    for (int a = 0; a < 65; a++) {
-        uint64_t x = 0;
-        for (int w = 0; w < 64; w++) if (is_qr_mod(65, (w * w + a) % 65)) x |= 1ull << w;
-        t.q65[a] = x;
-    }
+constexpr VResTabs make_vres() {
+    VResTabs t{};
+    for (int a = 0; a < 64; a++)
+        for (int u = 0; u < 32; u++)
+            if (is_qr_mod(64, (u * u + a) % 64)) t.q64[a] |= 1u << u;
+    for (int a = 0; a < 63; a++)
+        for (int x = 0; x < 63; x++) {
+            const int u = (x + 31) * 32 % 63;                     // (x - 32) / 2; 1/2 = 32
+            if (is_qr_mod(63, (u * u + a) % 63)) t.q63[a] |= 1ull << x;
+        }
+    for (int a = 0; a < 65; a++)
+        for (int x = 0; x < 64; x++) {
+            const int u = (x + 33) * 33 % 65;                     // (x - 32) / 2; 1/2 = 33
+            if (is_qr_mod(65, (u * u + a) % 65)) t.q65[a] |= 1ull << x;
+        }
     return t;
 }
-__device__ const UResTabs UQ = make_ures();
+__device__ const VResTabs VQ = make_vres();
 
-// (d mod 63, d mod 65) for |d| < 2^48, by folding 24-bit halves (2^24 = 1 mod 63 and mod 65)
-__device__ __forceinline__ void res6365(int64_t d, uint32_t &r63, uint32_t &r65) {
-    const uint64_t x = d < 0 ? (uint64_t)(-d) : (uint64_t)d;
-    const uint32_t r = (uint32_t)(x >> 24) + (uint32_t)(x & 0xFFFFFFu);
-    r63 = r % 63u;
-    r65 = r % 65u;
-    if (d < 0) { r63 = r63 ? 63u - r63 : 0u; r65 = r65 ? 65u - r65 : 0u; }
+// x mod 63 and mod 65 for x < 2^26, by the ceilings of 2^32/63 and 2^32/65 (exact there)
+__device__ __forceinline__ uint32_t mod63(uint32_t x) { return x - 63u * __umulhi(x, 68174085u); }
+__device__ __forceinline__ uint32_t mod65(uint32_t x) { return x - 65u * __umulhi(x, 66076420u); }
+
+// a 4-set's masks for C - A = d, |d| < 2^44
+__device__ __forceinline__ void and_masks(int64_t d, uint32_t &m64, uint64_t &m63, uint64_t &m65) {
+    const uint64_t x = (uint64_t)(d + (int64_t)(4095ull << 33));  // positive; 4095 = 63 * 65, 2^12 = 1 in both
+    const uint32_t r = (uint32_t)(x >> 24) + ((uint32_t)x & 0xFFFFFFu);
+    m64 &= __ldg(&VQ.q64[(uint32_t)d & 63u]);
+    m63 &= __ldg(&VQ.q63[mod63(r)]);
+    m65 &= __ldg(&VQ.q65[mod65(r)]);
 }
 
-// One lane's counters for the item of the 4-set it is working on, added to that item's
-// counter block whenever the item changes (queries of a batch are separate items).
-struct LaneCounters {
-    uint32_t item = 0xFFFFFFFFu;
-    ull cand = 0, sqrt_ = 0;
-    uint32_t mdiv = 0;
-    __device__ __forceinline__ void flush(const SearchArgs &a) {
-        if (item != 0xFFFFFFFFu) {
-            ull *k = a.counters + (size_t)item * K_SLOTS;
-            if (cand) atomicAdd(&k[K_EXT_CAND], cand);
-            if (sqrt_) atomicAdd(&k[K_EXT_SQRT], sqrt_);
-            if (mdiv) atomicMax(&k[K_MAX_DIVS], (ull)mdiv);
+constexpr uint32_t NO_ITEM = 0xFFFFFFFFu;
+
+__device__ __forceinline__ void count_global(const SearchArgs &a, uint32_t item, ull cand, ull sq, uint32_t mdiv) {
+    ull *k = a.counters + (size_t)item * K_SLOTS;
+    if (cand) atomicAdd(&k[K_EXT_CAND], cand);
+    if (sq) atomicAdd(&k[K_EXT_SQRT], sq);
+    if (mdiv) atomicMax(&k[K_MAX_DIVS], (ull)mdiv);
+}
+
+// A warp's counters: one item at a time (queries of a batch are separate items; the queue's
+// neighbours mostly belong to one), summed over the lanes and, when the item changes, put into the
+// warp's small cache of items, which reaches the items' counter blocks when an entry is pushed out and
+// at the end.  (Every lane's own atomics to one block took most of a small call's engine time: 2e5
+// 4-sets 0.28 -> 0.08 ms; without the cache, claims that alternate between the items in production
+// cost 64 uneven subranges 20 ms of 50 in atomics.)
+struct WarpCounters {
+    uint32_t item = NO_ITEM;                     // warp-uniform
+    uint32_t cand = 0, sqrt_ = 0, mdiv = 0;      // a lane meets 2^29 / 32 4-sets of a few dozen candidates at most
+    __device__ __forceinline__ void flush(const SearchArgs &a, WarpArea *w, int lane) {      // the whole warp
+        // sums of 32-bit values by halves (at most 32 * 65535 each)
+        const ull c = (ull)__reduce_add_sync(0xffffffffu, cand & 0xFFFFu) +
+                      ((ull)__reduce_add_sync(0xffffffffu, cand >> 16) << 16);
+        const ull s = (ull)__reduce_add_sync(0xffffffffu, sqrt_ & 0xFFFFu) +
+                      ((ull)__reduce_add_sync(0xffffffffu, sqrt_ >> 16) << 16);
+        const uint32_t d = __reduce_max_sync(0xffffffffu, mdiv);
+        if (lane == 0 && item != NO_ITEM) {
+            ItemCount &e = w->ic[item * 0x9E3779B1u >> 29];
+            if (e.item == item) {
+                e.cand += c;
+                e.sqrt_ += s;
+                e.mdiv = max(e.mdiv, d);
+            } else {
+                if (e.item != NO_ITEM) count_global(a, e.item, e.cand, e.sqrt_, e.mdiv);
+                e.item = item;
+                e.cand = c;
+                e.sqrt_ = s;
+                e.mdiv = d;
+            }
         }
         cand = 0; sqrt_ = 0; mdiv = 0;
     }
-    __device__ __forceinline__ void use(const SearchArgs &a, uint32_t it) {
-        if (it != item) { flush(a); item = it; }
+    // the whole warp: the lanes with `have` count c, s and d for their item `it`
+    __device__ __forceinline__ void add(const SearchArgs &a, WarpArea *w, int lane, bool have, uint32_t it, uint32_t c,
+                                        uint32_t s, uint32_t d) {
+        for (;;) {
+            if (have && it == item) {
+                cand += c;
+                sqrt_ += s;
+                mdiv = max(mdiv, d);
+                have = false;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, have);
+            if (!m) break;
+            flush(a, w, lane);
+            item = __shfl_sync(0xffffffffu, it, __ffs((int)m) - 1);
+        }
     }
 };
+static_assert(ICACHE == 8, "the cache index is a 3-bit hash");
 
 // Report the extensions of one warp round: group them per 4-set, emit hit / ext / six
 // records and the counters sets5 / multi / sets6 / hist5 / max_extensions (s4.c:243-277).
 template <bool COH>
-static __device__ void report_warp_exts(const SearchArgs &a, ExtEntry *el, uint32_t n) {
+static __device__ __noinline__ void report_warp_exts(const SearchArgs &a, ExtEntry *el, uint32_t n) {
     for (uint32_t x = 1; x < n; x++) {
         ExtEntry k = el[x];
         uint32_t y = x;
@@ -723,117 +790,190 @@ static __device__ void report_warp_exts(const SearchArgs &a, ExtEntry *el, uint3
     }
 }
 
-// Phase A state of one lane: its 4-set, the difference to extend by and its factorisation.
-struct LaneJob {
-    uint32_t r[6], item;
-    uint64_t v[4], S, A, C1, C2;
-    int bi, bj, bk;
-    int np;                              // distinct primes, in w->fp[0..np)[lane]
-    bool has2;
-    int E2, j0, js;                      // odd primes are pr[j0..np); the high group starts at js
-    uint32_t ndo, nd, ncand, L, H;
+// Whether the product of a lane's n prime powers from slot `first` exceeds 32 bits.
+static __device__ __noinline__ bool side_is_wide(const uint32_t (*fp)[32], int lane, uint32_t first, uint32_t n) {
+    uint64_t x = 1;
+    for (uint32_t i = first; i < first + n; i++)
+        for (uint32_t e = fp[i][lane] >> 24; e && x <= 0xFFFFFFFFull; e--) x *= fp[i][lane] & 0xFFFFFFu;
+    return x > 0xFFFFFFFFull;
+}
+
+// The odd primes of m1 and m2 (p | e << 24, from slots 0 and FSIDE): those of m2 that divide m1 too
+// add to m1's exponents.  The slow form, for numbers with more primes than a table entry holds.
+// Returns the primes and divisors of each side: na | nb << 8 | L << 16 | H << 40.
+static __device__ __noinline__ uint64_t merge_slow(const uint64_t *spfq, uint32_t m1, uint32_t m2, uint32_t (*fp)[32],
+                                                   int lane) {
+    uint32_t na = 0, nb = 0, L = 1, H = 1;
+    while (m1 > 1) {
+        const uint64_t t = __ldg(&spfq[m1]);
+        fp[na++][lane] = (uint32_t)t;                          // p | e << 24, as the table stores it
+        m1 = spf_cof(t);
+    }
+    while (m2 > 1) {
+        const uint64_t t = __ldg(&spfq[m2]);
+        const uint32_t x = (uint32_t)t, p = x & 0xFFFFFFu;
+        m2 = spf_cof(t);
+        uint32_t i = 0;
+        while (i < na && (fp[i][lane] & 0xFFFFFFu) != p) i++;
+        if (i < na) {
+            fp[i][lane] += x & 0xFF000000u;
+        } else {
+            fp[FSIDE + nb++][lane] = x;
+            H *= (x >> 24) + 1;
+        }
+    }
+    for (uint32_t i = 0; i < na; i++) L *= (fp[i][lane] >> 24) + 1;
+    return (uint64_t)na | (uint64_t)nb << 8 | (uint64_t)L << 16 | (uint64_t)H << 40;
+}
+
+struct LaneJob {                                 // a lane's 4-set in its round
+    uint32_t item, ncand, nd;
+    uint32_t L, H, rows;                         // list lengths; full rows and the last half one
+    uint32_t slots;                              // first prime slot of the row list | of the other list << 8
+    bool big;                                    // for the per-lane divisor walk
 };
 
-// Factor D = m1*m2 (m1 = ra-rb, m2 = ra+rb, both < 2^23, of equal parity).  The power of two
-// comes from counting trailing zeros; each odd part's first three primes come in one 16-byte
-// load (fac3), and the rare cofactor left over is walked through spfq (one table load per
-// distinct prime), both walks interleaved so that their dependent loads overlap.  Without fac3
-// (null) every prime is walked through spfq.  m1's primes are stored from slot 0, m2's from
-// slot 8 (each has at most 7 distinct odd primes), then m2's are merged into m1's list --
-// primes in first-seen order, as s4.c:141-147.  A new prime is written to a slot below every
-// unread slot of m2, so the merge is in place.
-__device__ __forceinline__ int factor_pair(const uint64_t *spfq, const uint4 *fac3, uint32_t m1, uint32_t m2,
-                                           uint32_t (*fp)[32], int lane) {
-    int na = 0, nb = 0;
-    if (m1 > 1 && !(m1 & 1)) {                      // both even
+// Phase A: one 4-set per lane.  Picks the difference to extend by (the fewest estimated divisors, in
+// the candidate order and with the tie-break of s4.c:163-171), factors it and writes the lane's
+// EJob.  False: an empty record, or more divisors than the cap.
+template <bool COH>
+__device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJob &J, WarpArea *w, int lane) {
+    uint32_t r[6];
+    get_job<COH>(a.jobs, j, r, J.item);
+    if (r[0] == 0) return false;                   // an empty record (the end of a tile warp's stretch)
+    // The six candidate pairs (i, j) with third member k: v_i - v_j = r_ik^2 - r_jk^2.  (0,1;2) (2,3;0)
+    // (0,2;1) (1,3;0) (0,3;1) (1,2;0), the first of the least kept.
+    uint32_t best = 0xFFFFFFFFu, rik = 0, rjk = 0;
+    auto pair = [&](int t, uint32_t x, uint32_t y) {
+        const uint32_t hi = max(x, y), lo = min(x, y);
+        const uint32_t est = (uint32_t)__ldg(&a.ndiv[hi - lo]) * (uint32_t)__ldg(&a.ndiv[hi + lo]);
+        const uint32_t key = est * 8u + t;                                       // est < 2^26
+        if (key < best) { best = key; rik = x; rjk = y; }
+    };
+    pair(0, r[1], r[3]);
+    pair(1, r[1], r[2]);
+    pair(2, r[0], r[3]);
+    pair(3, r[0], r[2]);
+    pair(4, r[0], r[4]);
+    pair(5, r[0], r[1]);
+    const uint32_t t = best & 7u;
+    // D = m1 * m2; D even => both even.  The factors are loaded while the members are worked out.
+    uint32_t m1 = max(rik, rjk) - min(rik, rjk), m2 = rik + rjk, E2 = 0;
+    if (!(m1 & 1)) {
         const uint32_t z1 = (uint32_t)__ffs((int)m1) - 1, z2 = (uint32_t)__ffs((int)m2) - 1;
-        fp[0][lane] = 2u | ((z1 + z2) << 24);
-        na = 1;
+        E2 = z1 + z2;
         m1 >>= z1;
         m2 >>= z2;
     }
-    if (fac3) {
-        const uint4 fa = m1 > 1 ? __ldg(&fac3[m1]) : make_uint4(0, 0, 0, 1);
-        const uint4 fb = m2 > 1 ? __ldg(&fac3[m2]) : make_uint4(0, 0, 0, 1);
-        if (fa.x) fp[na++][lane] = fa.x;
-        if (fa.y) fp[na++][lane] = fa.y;
-        if (fa.z) fp[na++][lane] = fa.z;
-        if (fb.x) fp[8 + nb++][lane] = fb.x;
-        if (fb.y) fp[8 + nb++][lane] = fb.y;
-        if (fb.z) fp[8 + nb++][lane] = fb.z;
-        m1 = fa.w;
-        m2 = fb.w;
+    const uint4 fa = __ldg(&a.fac[m1 >> 1]), fb = __ldg(&a.fac[m2 >> 1]);
+    EJob &E = w->job[lane];
+    {
+        uint64_t v[4];
+        const uint64_t ab = (uint64_t)r[0] * r[0], ac = (uint64_t)r[1] * r[1], ad = (uint64_t)r[2] * r[2],
+                       bc = (uint64_t)r[3] * r[3];
+        v[0] = (ab + ac - bc) >> 1; v[1] = ab - v[0]; v[2] = ac - v[0]; v[3] = ad - v[0];
+        // i = 0,2,0,1,0,1 and j = 1,3,2,3,3,2 for t = 0..5; the other two are 2,3 / 0,1 / 1,3 / 0,2 / 1,2 / 0,3
+        const bool i0 = (0x15u >> t) & 1u, i1 = (0x28u >> t) & 1u;               // i = 0; i = 1; else 2
+        const bool j3 = (0x1Au >> t) & 1u, j2 = (0x24u >> t) & 1u;               // j = 3; j = 2; else 1
+        const bool sw = rik < rjk;                                               // v_i < v_j
+        const uint64_t A = sw ? (j3 ? v[3] : j2 ? v[2] : v[1]) : (i0 ? v[0] : i1 ? v[1] : v[2]);
+        const uint64_t C1 = t == 0 ? v[2] : (0x14u >> t) & 1u ? v[1] : v[0];     // t = 2, 4: 1; t = 1, 3, 5: 0
+        const uint64_t C2 = (0x25u >> t) & 1u ? v[3] : t == 1 ? v[1] : v[2];     // t = 0, 2, 5: 3; t = 3, 4: 2
+        const uint32_t bi = sw ? (j3 ? 3u : j2 ? 2u : 1u) : (i0 ? 0u : i1 ? 1u : 2u);
+        E.A = A;
+        const int64_t d1 = (int64_t)C1 - (int64_t)A, d2 = (int64_t)C2 - (int64_t)A;
+        E.d1 = d1;
+        E.d2 = d2;
+        // the roots through member bi: r_ab r_ac r_ad / r_ab r_bc r_bd / r_ac r_bc r_cd / r_ad r_bd r_cd
+        E.rA0 = bi <= 1 ? r[0] : bi == 2 ? r[1] : r[2];
+        E.rA1 = bi == 0 ? r[1] : bi == 3 ? r[4] : r[3];
+        E.rA2 = bi == 0 ? r[2] : bi == 1 ? r[4] : r[5];
+        E.item = J.item;
+        uint32_t m64 = 0xFFFFFFFFu;
+        uint64_t m63 = ~0ull, m65 = ~0ull;
+        and_masks(d1, m64, m63, m65);
+        and_masks(d2, m64, m63, m65);
+        E.m64 = m64; E.m63 = m63; E.m65 = m65;
     }
-    uint64_t sa = m1 > 1 ? __ldg(&spfq[m1]) : 0, sb = m2 > 1 ? __ldg(&spfq[m2]) : 0;
-    while (m1 > 1 || m2 > 1) {
-        if (m1 > 1) {
-            fp[na][lane] = (uint32_t)sa;                   // p | e << 24, as the table stores it
-            na++;
-            m1 = spf_cof(sa);
-            if (m1 > 1) sa = __ldg(&spfq[m1]);
-        }
-        if (m2 > 1) {
-            fp[8 + nb][lane] = (uint32_t)sb;
-            nb++;
-            m2 = spf_cof(sb);
-            if (m2 > 1) sb = __ldg(&spfq[m2]);
-        }
-    }
-    int np = na;
-    for (int j = 0; j < nb; j++) {
-        const uint32_t x = fp[8 + j][lane], p = x & 0xFFFFFFu;
-        int i = 0;
-        while (i < na && (fp[i][lane] & 0xFFFFFFu) != p) i++;
-        if (i < na) fp[i][lane] += x & 0xFF000000u;
-        else { fp[np][lane] = x; np++; }
-    }
-    return np;
-}
-
-template <bool COH>
-__device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJob &J, uint32_t (*fp)[32],
-                                          int lane) {
-    get_job<COH>(a.jobs, j, J.r, J.item);
-    if (J.r[0] == 0) return false;                 // an empty record (the end of a tile warp's stretch)
-    quad_values(J.r, J.v, J.S);
-    uint32_t best;
-    choose_pair(J.v, J.r, a.ndiv, J.bi, J.bj, J.bk, best);
-    const uint32_t ra = pick6(J.r, pair_slot(J.bi, J.bk)), rb = pick6(J.r, pair_slot(J.bj, J.bk));
-    J.A = pick4(J.v, J.bi);
-    int o1 = -1, o2 = -1;
+    uint32_t na = 0, nb = 0, L = 1, H = 1, shared_ = 0;
+    if ((fa.w | fb.w) >> 31) {                     // more than four primes on a side
+        const uint64_t s = merge_slow(a.spfq, m1, m2, w->fp, lane);
+        na = (uint32_t)s & 0xFFu;
+        nb = (uint32_t)(s >> 8) & 0xFFu;
+        L = (uint32_t)(s >> 16) & 0xFFFFFFu;
+        H = (uint32_t)(s >> 40);
+        shared_ = 1;
+    } else {
+        uint32_t x[4] = {fa.x, fa.y, fa.z, fa.w}, y[4] = {fb.x, fb.y, fb.z, fb.w};
 #pragma unroll
-    for (int t = 0; t < 4; t++)
-        if (t != J.bi && t != J.bj) { if (o1 < 0) o1 = t; else o2 = t; }
-    J.C1 = pick4(J.v, o1);
-    J.C2 = pick4(J.v, o2);
-    J.np = factor_pair(a.spfq, a.fac3, ra - rb, ra + rb, fp, lane);
-    // D even => both factors even => 2 is the first prime and 4 | D
-    J.has2 = J.np > 0 && (fp[0][lane] & 0xFFFFFFu) == 2;
-    J.E2 = J.has2 ? fp[0][lane] >> 24 : 0;
-    J.j0 = J.has2 ? 1 : 0;
-    uint32_t ndo = 1;
-    for (int q = J.j0; q < J.np; q++) ndo *= (fp[q][lane] >> 24) + 1;
-    J.ndo = ndo;
-    // low group: the leading odd primes while their radix product stays <= sqrt(ndo)
-    uint32_t L = 1, js = J.j0;
-    while (js < J.np && L * ((fp[js][lane] >> 24) + 1) * L * ((fp[js][lane] >> 24) + 1) <= ndo)
-        L *= (fp[js++][lane] >> 24) + 1;
-    J.js = js;
-    J.L = L;
-    J.H = ndo / L;
-    const uint64_t nd = (uint64_t)ndo * (uint64_t)(J.E2 + 1);
+        for (int k = 0; k < 4; k++) {
+            const uint32_t e = y[k] & 0xFF000000u;
+            bool eq = false;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const bool s = ((x[i] ^ y[k]) & 0xFFFFFFu) == 0;     // two zeros: nothing moves
+                x[i] += s ? e : 0u;
+                eq |= s;
+            }
+            shared_ |= eq ? e : 0u;
+            y[k] = eq ? 0u : y[k];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (x[i]) w->fp[i][lane] = x[i];
+            na += x[i] != 0;
+            L += L * (x[i] >> 24);
+            if (y[i]) w->fp[FSIDE + nb][lane] = y[i];
+            nb += y[i] != 0;
+            H += H * (y[i] >> 24);
+        }
+    }
+    const uint64_t ndo = (uint64_t)L * H, nd = ndo * (E2 + 1);
+    if (nd > a.cap_divs) {
+        raise_error(a.status, E_CAP_DIVS, (uint64_t)r[0] * r[0] + (uint64_t)r[5] * r[5]);
+        return false;
+    }
     J.nd = (uint32_t)nd;
+    // the row list is the longer one; its last prime moves over while that leaves both shorter
+    uint32_t sr = 0, so = FSIDE, nr = na, no = nb;
+    if (H > L) {
+        sr = FSIDE; so = 0; nr = nb; no = na;
+        const uint32_t s = L; L = H; H = s;
+    }
+    const bool below32 = (uint64_t)m1 * m2 <= 0xFFFFFFFFull;         // then no list entry is above 32 bits
+    bool wide = false;
+    if (below32 || !shared_) {                     // else both sides are checked, and left alone
+        while (nr > 1 && no < FSIDE) {
+            const uint32_t x = w->fp[sr + nr - 1][lane], k = (x >> 24) + 1;
+            if (H * k >= L || !below32) break;
+            w->fp[so + no++][lane] = x;
+            nr--;
+            L /= k;
+            H *= k;
+        }
+        if (H > L) {
+            const uint32_t s = L, q = sr; L = H; H = s; sr = so; so = q;
+        }
+    } else {
+        wide = side_is_wide(w->fp, lane, 0, na);   // m2's side is a divisor of m2
+    }
+    J.slots = sr | so << 8;
+    J.L = L;
+    J.H = H;
     // same-parity complementary pairs with f < g: the reference's ext_cand (s4.c:191)
-    J.ncand = J.has2 ? (uint32_t)(((uint64_t)(J.E2 - 1) * ndo) >> 1) : (uint32_t)(nd >> 1);
-    if (nd > a.cap_divs) { raise_error(a.status, E_CAP_DIVS, J.S); return false; }
+    const uint32_t R = E2 ? E2 - 1 : 1;            // 2-exponents of f: 1 .. E2-1, or 0
+    J.ncand = (uint32_t)ndo * R >> 1;
+    J.rows = (H * R + (L > 1 ? 1u : 0u)) >> 1;
+    E.geo = L | H << 8 | E2 << 16;
+    // a list longer than the fields and buffers allow, or one side above 32 bits: the per-lane walk
+    J.big = wide || L > (uint32_t)LCAP;
     return true;
 }
 
 // The n divisors of prod pr[q]^ex[q], q in [q0, q1), in mixed-radix order (first prime
 // fastest), in one flat loop: prime q's block repeats the list so far ex[q] times, each copy
 // times p_q, so d[j] = d[j - cur] * p_q with cur the list length before q.
-__device__ __forceinline__ void gen_list(uint64_t *d, const uint32_t (*fp)[32], int lane,
-                                         int q0, uint32_t n) {
+__device__ __forceinline__ void gen_list(uint32_t *d, const uint32_t (*fp)[32], int lane, int q0, uint32_t n) {
     d[0] = 1;
     if (n <= 1) return;
     int q = q0;
@@ -850,294 +990,312 @@ __device__ __forceinline__ void gen_list(uint64_t *d, const uint32_t (*fp)[32], 
     }
 }
 
-// A 4-set whose factored divisor lists exceed the warp buffer: the per-lane divisor walk.
-static __device__ __noinline__ void extend_big(const SearchArgs &a, const LaneJob &J, uint32_t qid, ull &cand,
-                                               ull &sq, ExtEntry *el, uint32_t *el_n) {
-    uint32_t md = 0;
-    extend_quad(a, J.r, J.v, J.S, J.bi, J.bj, J.bk, qid, cand, sq, md, el, el_n, EXCAP);
+// A 4-set whose factored divisor lists exceed the warp buffer or 32 bits: the per-lane divisor walk.
+// Returns its ext_sqrt.
+template <bool COH>
+static __device__ __noinline__ uint32_t extend_big(const SearchArgs &a, uint64_t j, uint32_t qid, ExtEntry *el,
+                                                   uint32_t *el_n) {
+    ull cand = 0, sq = 0;
+    uint32_t r[6], item, best, md = 0;
+    uint64_t v[4], S;
+    int bi, bj, bk;
+    get_job<COH>(a.jobs, j, r, item);
+    quad_values(r, v, S);
+    choose_pair(v, r, a.ndiv, bi, bj, bk, best);
+    extend_quad(a, r, v, S, bi, bj, bk, qid, cand, sq, md, el, el_n, EXCAP);
+    return (uint32_t)sq;
 }
 
-// Square tests of queue entries [first, first+count), one per lane (s4.c:199-203); a hit
-// gets its order key, the reference's mixed-radix index of the smaller divisor.
+// Whether n = u^2 + d is a square; n > 0, u < 2^44, |d| < 2^44, n's low 64 bits given.  If n = s^2
+// then s < 2^45; the double of n is one rounding off (2^-53), and two Newton steps from the single-precision
+// reciprocal root (relative error e < 2^-22) leave 1.5 e^2, then e times that, plus roundings: below 2^-50,
+// so the root is less than 1/4 off and rounds to s.  A number r that passes r^2 = n mod 2^64 for r
+// within 1/2 of sqrt(n) has |r^2 - n| <= sqrt(n) + 1 < 2^46, so r^2 = n.  Hence the result is exact.
+__device__ __forceinline__ bool is_square_near(uint64_t u, int64_t d, uint64_t n_lo) {
+    const double two52 = 4503599627370496.0, b = 6755399441055744.0;             // 2^52, 1.5 * 2^52
+    const double ud = __longlong_as_double((long long)(u | 0x4330000000000000ull)) - two52;
+    const double dd = __longlong_as_double(0x4338000000000000ll + d) - b;
+    const double x = fma(ud, ud, dd);
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"((float)x));
+    const double y = (double)yf, h = 0.5 * y;
+    double s = x * y;
+    s = fma(fma(-s, s, x), h, s);
+    s = fma(fma(-s, s, x), h, s);
+    const uint64_t r = ((uint64_t)__double_as_longlong(s + b) & 0xFFFFFFFFFFFFFull) ^ 0x8000000000000ull;
+    return r * r == n_lo;
+}
+
+// The extension e = u^2 - A of lane jl's 4-set (rare).  Its order key is the reference's mixed-radix
+// index of the smaller divisor f = u - w, w^2 = e + B, over the primes in first-seen order: 2, m1's, then
+// m2's others (s4.c:141-156).
+static __device__ __noinline__ void record_ext(const SearchArgs &a, WarpArea *w, uint32_t jl, uint64_t u) {
+    uint32_t rt[6], item, best;
+    uint64_t v[4], S;
+    int bi, bj, bk;
+    get_job<true>(a.jobs, w->jid[jl], rt, item);
+    quad_values(rt, v, S);
+    choose_pair(v, rt, a.ndiv, bi, bj, bk, best);
+    const uint32_t ra = pick6(rt, pair_slot(bi, bk)), rb = pick6(rt, pair_slot(bj, bk));
+    uint32_t m1 = ra - rb, m2 = ra + rb, key = 0, mult = 1;
+    const u128 e = (u128)u * u - pick4(v, bi);
+    uint64_t f = u - isqrt128(e + pick4(v, bj));
+    if (!(m1 & 1)) {
+        const uint32_t z1 = (uint32_t)__ffs((int)m1) - 1, z2 = (uint32_t)__ffs((int)m2) - 1;
+        while (!(f & 1)) { f >>= 1; key++; }
+        mult = z1 + z2 + 1;
+        m1 >>= z1;
+        m2 >>= z2;
+    }
+    for (int side = 0; side < 2; side++) {
+        const uint32_t other = side ? m1 : m2;
+        for (uint32_t m = side ? m2 : m1; m > 1;) {
+            const uint64_t t = __ldg(&a.spfq[m]);
+            const uint32_t p = spf_p(t);
+            uint32_t ex = spf_e(t), o = other;
+            m = spf_cof(t);
+            if (side && o % p == 0) continue;                        // one of m1's
+            while (o % p == 0) { o /= p; ex++; }
+            while (f % p == 0) { f /= p; key += mult; }
+            mult *= ex + 1;
+        }
+    }
+    const uint32_t slot = atomicAdd(&w->n_ext, 1u);
+    if (slot < EXCAP) {
+        ExtEntry &x = w->ext[slot];
+        x.qid = w->jid[jl];
+        x.key = key;
+        x.lo = (uint64_t)e;
+        x.hi = (uint64_t)(e >> 64);
+    } else {
+        raise_capacity(a.status, E_EXTLIST, 4, slot + 1, EXCAP, 0);
+    }
+}
+
+// Queue entries [first, first+count), one per lane: those with 0 < e = u^2 - A not in the 4-set are the
+// reference's ext_sqrt (s4.c:195-198) and are square-tested (s4.c:199-203).
 __device__ __forceinline__ void process_queue(const SearchArgs &a, WarpArea *w, uint32_t first, uint32_t count,
-                                              int lane) {
+                                              int lane, WarpCounters &cnt) {
     if ((uint32_t)lane < count) {
-        const uint32_t idx = first + lane;
-        const uint64_t u = w->qu[idx];
-        const uint32_t jl = w->qj[idx];
-        const EJob &J = w->job[jl];
-        const u128 e = (u128)u * u - J.A;
-        // is_square_fast needs n < 2^100: u = (f+g)/2 <= (D+1)/2 < 2^44 and C < S < 2^44, so
-        // e + C < u^2 + C < 2^89
-        if (is_square_fast(e + J.C1) && is_square_fast(e + J.C2)) {
-            const uint32_t c = w->qidx[idx], l = c & 0xFFFu, h = (c >> 12) & 0xFFFu, d2 = c >> 24;
-            const uint64_t fo = w->dbuf[J.base + l] * w->dbuf[J.base + J.L + h];
-            const uint64_t go = w->dbuf[J.base + J.L - 1 - l] * w->dbuf[J.base + J.L + J.H - 1 - h];
-            const uint32_t to = l + J.L * h;
-            const uint32_t t = (J.flags & 1) ? d2 + (J.E2 + 1u) * to : to;
-            const uint32_t nd = (uint32_t)J.L * J.H * ((J.flags & 1) ? J.E2 + 1u : 1u);
-            const uint32_t key = (fo << d2) < (go << (J.E2 - d2)) ? t : nd - 1 - t;
-            const uint32_t slot = atomicAdd(&w->n_ext, 1u);
-            if (slot < EXCAP) {
-                ExtEntry &x = w->ext[slot];
-                x.qid = w->jid[jl];
-                x.key = key;
-                x.lo = (uint64_t)e;
-                x.hi = (uint64_t)(e >> 64);
-            } else {
-                raise_capacity(a.status, E_EXTLIST, 4, slot + 1, EXCAP, 0);
+        const uint64_t ent = w->q[first + lane];
+        const uint32_t jl = (uint32_t)(ent >> 58);
+        const uint64_t u = (ent & ((1ull << 58) - 1)) >> 1, u2 = u * u;          // u < 2^44; u2 mod 2^64
+        const EJob &E = w->job[jl];
+        const uint64_t A = E.A;
+        const uint4 ro = *(const uint4 *)&E.rA0;
+        const uint32_t ul = (uint32_t)u;
+        // u below 2^32: e > 0 iff u2 > A; e = A iff u2 = 2A; e another member iff u one of A's roots
+        if ((u >> 32) != 0 || (u2 > A && u2 != 2 * A && ul != ro.x && ul != ro.y && ul != ro.z)) {
+            if ((ro.w & 0xFFFFFu) == cnt.item) cnt.sqrt_++;
+            else atomicAdd(&w->job[jl].item, 1u << 20);
+            bool sq = true;
+#pragma unroll 1
+            for (int c = 0; c < 2 && sq; c++) {                                  // one copy of the code
+                const int64_t d = (&E.d1)[c];
+                sq = is_square_near(u, d, u2 + (uint64_t)d);
             }
+            if (sq) record_ext(a, w, jl, u);
         }
     }
 }
 
+// One candidate of a row: v = f + g = x*fy + y*gy and whether it passes the filters (bit 0).
+__device__ __forceinline__ uint32_t candidate(uint32_t x, uint32_t y, uint64_t fy, uint64_t gy, uint32_t m64,
+                                              uint64_t m63, uint64_t m65, uint64_t &v) {
+    const uint64_t lo = (uint64_t)x * (uint32_t)fy + (uint64_t)y * (uint32_t)gy;
+    const uint32_t hi = (uint32_t)(lo >> 32) + x * (uint32_t)(fy >> 32) + y * (uint32_t)(gy >> 32);
+    v = (uint64_t)hi << 32 | (uint32_t)lo;
+    const uint32_t z = (uint32_t)(v >> 24) + ((uint32_t)lo & 0xFFFFFFu) + 32u;
+    return __funnelshift_r(m64, m64, (uint32_t)lo >> 1) & (uint32_t)(m63 >> mod63(z)) &
+           (uint32_t)(m65 >> (mod65(z) & 63u));
+}
+
 // The engine loop of one warp.  Linear (RING false): the batch's queue [0, njobs), filled before
-// the launch; the loop ends when it is drained.  RING: the persistent kernel's ring; positions are
-// claimed below q_tail and waited for until published, each finished 4-set's slot is handed back
-// after the round's report, and the loop ends when a claim finds the ring empty and no lane holds
-// a 4-set.  Returns whether the warp took any 4-set.
+// the launch, taken in stretches of `stretch` 4-sets; the loop ends when it is drained.  RING: the
+// persistent kernel's ring; positions are claimed below q_tail and waited for until published, each
+// finished 4-set's slot is handed back after the round's report, and the loop ends when a claim finds
+// the ring empty and no lane holds a 4-set.  quota: lanes that hold a 4-set (32 unless the queue is too
+// short to fill every warp of the launch; the candidates of few 4-sets are still walked by all
+// lanes).  Returns whether the warp took any 4-set.
 template <bool RING>
-__device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint64_t njobs) {
+__device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint32_t njobs, uint32_t quota,
+                                            uint32_t stretch) {
     const unsigned FULL = 0xffffffffu;
     if (lane == 0) w->n_ext = 0;
-    w->jsq[lane] = 0;
+    if (lane < ICACHE) w->ic[lane].item = NO_ITEM;
     __syncwarp();
-    LaneCounters cnt;
-    LaneJob J;
-    bool pending = false, old = false, drained = false, rel = false, took = false;
+    WarpCounters cnt;
+    bool pending = false, drained = false, rel = false, took = false;
     uint32_t myjob = 0;
     uint64_t mypos = 0;
+    uint32_t st_cur = 0, st_rem = 0;               // the warp's stretch of the queue (not RING)
+    bool last = false;                             // no further stretch
 
-    // Rolling rounds: before each round every lane without a 4-set takes the next one from the
-    // queue (phase A), so every round runs with a full warp of 4-sets; a lane whose divisor
-    // lists did not fit keeps its 4-set and goes first in the next round's placement.
+    // Rounds: every lane without a 4-set takes the next one from the queue; a lane whose divisor lists
+    // did not fit keeps its 4-set, sets it up again and goes first in the next round's placement.
     for (;;) {
+        const bool old = pending;
         if (!drained) {
-            const bool need = !pending;
+            const bool need = !pending && (uint32_t)lane < quota;
             const unsigned m = __ballot_sync(FULL, need);
-            uint64_t base = 0;
-            uint32_t got = 0;
+            const uint32_t n = (uint32_t)__popc(m), rank = (uint32_t)__popc(m & ((1u << lane) - 1u));
             int stop = 0;
             if (RING) {
+                uint64_t base = 0;
+                uint32_t got = 0;
                 if (lane == 0) {
-                    if (m) base = ring_claim(a, (uint32_t)__popc(m), &got);
+                    if (m) base = ring_claim(a, n, &got);
                     stop = *(volatile ull *)&a.status->err != 0ull;
                 }
                 base = __shfl_sync(FULL, base, 0);
-            } else {
-                uint32_t b32 = 0;                  // the batch queue's counter is 32-bit
-                if (lane == 0) {
-                    if (m) b32 = atomicAdd(&a.status->ext_next, (uint32_t)__popc(m));
-                    stop = *(volatile ull *)&a.status->err != 0ull;
-                }
-                base = __shfl_sync(FULL, b32, 0);
-            }
-            stop = __shfl_sync(FULL, stop, 0);
-            if (stop) break;                                             // warp-uniform
-            if (RING) {
                 got = __shfl_sync(FULL, got, 0);
-                if (got < (uint32_t)__popc(m)) drained = true;           // the ring is empty for now
-            } else if (base + __popc(m) >= njobs) {
-                drained = true;                                          // warp-uniform
-            }
-            if (need) {
-                const uint32_t rank = __popc(m & ((1u << lane) - 1u));
-                const uint64_t jidx = base + rank;
-                bool have = RING ? rank < got : jidx < njobs;
-                if (RING && have) {
-                    have = ring_wait_ready(a, jidx);
-                    mypos = jidx;
+                stop = __shfl_sync(FULL, stop, 0);
+                if (stop) break;                                         // warp-uniform
+                if (got < n) drained = true;                             // the ring is empty for now
+                if (need && rank < got && ring_wait_ready(a, base + rank)) {
+                    pending = true;
+                    mypos = base + rank;
+                    myjob = (uint32_t)(mypos & a.ring_mask);
                 }
-                if (have) {
-                    myjob = (uint32_t)(RING ? (jidx & a.ring_mask) : jidx);
-                    old = false;
-                    took = true;
-                    // ---- phase A: one 4-set per lane
-                    pending = job_setup<RING>(a, myjob, J, w->fp, lane);
-                    const bool big = pending && J.L + J.H > (uint32_t)DCAP;
-                    if (pending) {
-                        cnt.use(a, J.item);
-                        if (J.nd > cnt.mdiv) cnt.mdiv = J.nd;
-                        if (!big) cnt.cand += J.ncand;
+                took |= pending;
+            } else {
+                uint32_t nx = 0, avail = 0;
+                if (st_rem < n && !last) {                               // a new stretch behind the old one
+                    if (lane == 0) {
+                        nx = atomicAdd(&a.status->ext_next, stretch);
+                        stop = *(volatile ull *)&a.status->err != 0ull;
                     }
-                    if (big) {               // extremely rare: its factored lists exceed the buffer
-                        extend_big(a, J, myjob, cnt.cand, cnt.sqrt_, w->ext, &w->n_ext);
-                        pending = false;
-                    }
-                    if (RING && !pending) rel = true;                  // done in phase A: freed after the report
+                    nx = __shfl_sync(FULL, nx, 0);
+                    stop = __shfl_sync(FULL, stop, 0);
+                    if (stop) break;                                     // warp-uniform
+                    avail = nx < njobs ? min(stretch, njobs - nx) : 0u;
+                    last = avail < stretch;
                 }
+                if (need && rank < st_rem + avail) {
+                    pending = true;
+                    myjob = rank < st_rem ? st_cur + rank : nx + (rank - st_rem);
+                }
+                const uint32_t used = min(n, st_rem + avail);
+                if (used < st_rem) {
+                    st_cur += used;
+                    st_rem -= used;
+                } else {
+                    st_cur = nx + (used - st_rem);
+                    st_rem = st_rem + avail - used;
+                }
+                drained = last && st_rem == 0;                           // warp-uniform
             }
         }
+        // ---- phase A: one 4-set per lane
+        LaneJob J;
+        J.item = J.ncand = J.nd = 0;
+        J.big = false;
+        const bool mine = pending;
+        uint32_t bsq = 0;
+        if (pending) {
+            pending = job_setup<RING>(a, myjob, J, w, lane);
+            if (pending && J.big) {                                      // rare
+                bsq = extend_big<RING>(a, myjob, myjob, w->ext, &w->n_ext);
+                pending = false;
+            }
+        }
+        if (RING && mine && !pending) rel = true;                        // done: freed after the report
+        const bool fresh = mine && !old && (pending || J.big);           // counted once
+        cnt.add(a, w, lane, fresh, J.item, J.ncand, bsq, J.nd);
         const bool round = __any_sync(FULL, pending);
         if (round) {
             // place the factored divisor lists of as many pending lanes as fit: lanes left over
             // from the last round first, then the new ones, each in lane order
             const uint32_t want = pending ? J.L + J.H : 0;
-            uint32_t io = old ? want : 0, in = old ? 0 : want;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t yo = __shfl_up_sync(FULL, io, o), yn = __shfl_up_sync(FULL, in, o);
-                if (lane >= o) { io += yo; in += yn; }
-            }
-            const uint32_t tot_old = __shfl_sync(FULL, io, 31);           // every lane takes part
-            const uint32_t incl = old ? io : tot_old + in;
-            const uint32_t base = incl - want;
-            const bool fits = pending && incl <= (uint32_t)DCAP;
-            if (fits) w->jid[lane] = myjob;
+            uint32_t tot_old = 0, tot_new, base = 0;
+            if (__any_sync(FULL, old)) base = warp_prefix(old ? want : 0, lane, tot_old);
+            const uint32_t bn = warp_prefix(old ? 0 : want, lane, tot_new);
+            if (!old) base = tot_old + bn;
+            const bool fits = pending && base + want <= (uint32_t)DCAP;
             if (fits) {
-                gen_list(w->dbuf + base, w->fp, lane, J.j0, J.L);               // lo: L entries
-                gen_list(w->dbuf + base + J.L, w->fp, lane, J.js, J.H);         // hi: H entries
-                EJob &E = w->job[lane];
-                E.A = J.A; E.C1 = J.C1; E.C2 = J.C2;
-                const int64_t dd1 = (int64_t)J.C1 - (int64_t)J.A, dd2 = (int64_t)J.C2 - (int64_t)J.A;
-                uint32_t a63, a65, b63, b65;
-                res6365(dd1, a63, a65);
-                res6365(dd2, b63, b65);
-                E.m64 = UQ.q64[(uint32_t)dd1 & 63u] & UQ.q64[(uint32_t)dd2 & 63u];
-                E.m63 = UQ.q63[a63] & UQ.q63[b63];
-                E.m65 = UQ.q65[a65] & UQ.q65[b65];
-                E.uA = isqrt_lt2p46(J.A);                        // < 2^22 (A < 2^44)
-                const uint32_t r2A = isqrt_lt2p46(2 * J.A);      // < 2^23
-                E.rAA = (uint64_t)r2A * r2A == 2 * J.A ? r2A : 0u;
-                // the three roots through A, r[pair_slot(bi, x)]^2 = A + v_x (the member test takes
-                // them as a set): slots 0,1,2 through index 0; 0,3,4 through 1; 1,3,5 through 2;
-                // 2,4,5 through 3
-                const int bi = J.bi;
-                E.rA0 = bi <= 1 ? J.r[0] : (bi == 2 ? J.r[1] : J.r[2]);
-                E.rA1 = bi == 0 ? J.r[1] : (bi == 3 ? J.r[4] : J.r[3]);
-                E.rA2 = bi == 0 ? J.r[2] : (bi == 1 ? J.r[4] : J.r[5]);
-                E.ncand = J.ncand;
-                E.base = (uint16_t)base; E.L = (uint16_t)J.L; E.H = (uint16_t)J.H;
-                E.E2 = (uint8_t)J.E2;
-                E.flags = (uint8_t)(J.has2 ? 1 : 0);
+                w->jid[lane] = myjob;
+                w->job[lane].geo |= base << 22;
+                gen_list(w->dbuf + base, w->fp, lane, J.slots & 0xFFu, J.L);             // rows: L entries
+                gen_list(w->dbuf + base + J.L, w->fp, lane, J.slots >> 8, J.H);          // H entries
             }
-            // ---- phase B: the pooled candidates, 32 equal contiguous runs
-            const uint32_t nc = fits ? J.ncand : 0;
-            const unsigned nonempty = __ballot_sync(FULL, nc != 0);          // jobs with candidates
-            uint32_t ci = nc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, ci, o);
-                if (lane >= o) ci += y;
-            }
-            w->cstart[lane] = ci - nc;
-            const uint32_t C = __shfl_sync(FULL, ci, 31);
-            if (lane == 31) w->cstart[32] = C;
-            __syncwarp();
-            const uint32_t g0 = (uint32_t)(((uint64_t)lane * C) >> 5);
-            const uint32_t g1 = (uint32_t)(((uint64_t)(lane + 1) * C) >> 5);
-            const uint32_t iters = (C + 31) >> 5;
-            uint32_t jl = 0;
+            // rows by length, longest first, so that the 32 rows of a turn are about equally long:
+            // each lane's rank by (length, lane), then the rows' prefix in rank order
+            const uint32_t rows = fits ? J.rows : 0;
+            uint32_t rank = 0;
             {
-                uint32_t lo = 0, hi = 32;                 // last job with cstart <= g0
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (w->cstart[mid] <= g0) lo = mid; else hi = mid;
+                const uint32_t key = rows ? min(J.L, 31u) : 0u;
+                unsigned eq = FULL;
+#pragma unroll
+                for (int b = 4; b >= 0; b--) {
+                    const unsigned m = __ballot_sync(FULL, key >> b & 1u);
+                    if (key >> b & 1u) eq &= m;
+                    else { rank += __popc(eq & m); eq &= ~m; }
                 }
-                jl = lo;
+                rank += __popc(eq & ((1u << lane) - 1u));
             }
-            // the current job of this lane's run, in registers
-            uint64_t m64 = 0, m63 = 0, m65 = 0, hv = 0, hc = 0;
-            uint32_t uA = 0, rAA = 0, rA0 = 0, rA1 = 0, rA2 = 0;
-            uint32_t ncand = 0, jb = 0, L = 1, H = 1, E2 = 0, flg = 0, R = 1, dlo = 0, dhi = 0;
-            uint32_t cc = 0, l = 0, h = 0, d2 = 0;
-            // hv/hc are reloaded only for a new row h or a new job: the loads of the lanes that keep
-            // their row are predicated off, so fewer divisor-buffer wavefronts (engine -1.8 % per
-            // [1,1e10) step; the same for the lo values, which change every candidate of odd D, +3 %)
-            bool hre = true;
-            // job fields in four vector loads; entering a job at its first candidate needs no division
-            auto load_job = [&](uint32_t j) {
-                const ulonglong2 x0 = *(const ulonglong2 *)&w->job[j].m64;
-                const ulonglong2 x1 = *(const ulonglong2 *)&w->job[j].m65;    // m65, rA0 | rA1 << 32
-                const uint4 y = *(const uint4 *)&w->job[j].uA;
-                const uint2 z = *(const uint2 *)&w->job[j].base;
-                m64 = x0.x; m63 = x0.y; m65 = x1.x;
-                rA0 = (uint32_t)x1.y; rA1 = (uint32_t)(x1.y >> 32);
-                uA = y.x; rAA = y.y; rA2 = y.z; ncand = y.w;
-                jb = z.x & 0xFFFFu; L = z.x >> 16; H = z.y & 0xFFFFu; E2 = (z.y >> 16) & 0xFFu; flg = z.y >> 24;
-                R = (flg & 1) ? E2 - 1 : 1;
-                dlo = flg & 1; dhi = (flg & 1) ? E2 - 1 : 0;      // 2-exponents of f: [1, E2-1] or {0}
-                cc = 0; l = 0; h = 0; d2 = (flg & 1) ? 1u : 0u;
-            };
-            if (g0 < g1) {
-                load_job(jl);
-                const uint32_t cidx = g0 - w->cstart[jl];
-                const uint32_t to = (flg & 1) ? cidx / R : cidx;
-                d2 = (flg & 1) ? 1 + cidx % R : 0;
-                h = to / L;
-                l = to - h * L;
-                cc = cidx;
-            }
-            uint32_t qn = 0, sq_run = 0;
-            for (uint32_t it = 0; it < iters; it++) {
-                bool pass = false;
-                uint64_t u = 0;
-                uint32_t cidx = 0, jcur = jl;              // the job of THIS candidate
-                if (it < g1 - g0) {
-                    if (hre) {
-                        hv = w->dbuf[jb + L + h];
-                        hc = w->dbuf[jb + L + H - 1 - h];
-                    }
-                    // f = 2^d2 * lo[l]*hi[h], g = 2^(E2-d2) * lo[L-1-l]*hi[H-1-h]: complementary divisors
-                    const uint64_t fo = w->dbuf[jb + l] * hv, go = w->dbuf[jb + L - 1 - l] * hc;
-                    u = ((fo << d2) + (go << (E2 - d2))) >> 1;
-                    // e + C = u^2 + (C - A): residues mod 64, 63, 65 for both C (s4.c:192-194), as
-                    // bits of the 4-set's u-indexed masks
-                    const uint32_t w64 = (uint32_t)u & 63u;
-                    const uint32_t rr = (uint32_t)(u >> 24) + ((uint32_t)u & 0xFFFFFFu);   // 2^24 = 1 mod 63, 65
-                    const uint32_t w63 = rr % 63u, w65r = rr % 65u;
-                    const uint32_t w65 = w65r == 64u ? 1u : w65r;     // 64^2 = 1^2 mod 65: same bit
-                    // e = u^2 - A in v (s4.c:197) iff u^2 = A + v_i: u is one of the 4-set's roots
-                    // through A (all below 2^23, so u's low word decides once u < 2^32)
-                    const uint32_t ul = (uint32_t)u;
-                    const bool member = (u >> 32) == 0 && (ul == rA0 || ul == rA1 || ul == rA2 || ul == rAA);
-                    pass = ((m64 >> w64) & (m63 >> w63) & (m65 >> w65) & 1u) && u > uA && !member;
-                    if (pass) { sq_run++; cidx = l | (h << 12) | (d2 << 24); }
-                    // next candidate of this lane's run
-                    {                                          // (l, h, d2) advance, branch-free
-                        d2++;
-                        const uint32_t wd = d2 > dhi ? 1u : 0u;
-                        d2 = wd ? dlo : d2;
-                        l += wd;
-                        const uint32_t wl = l == L ? 1u : 0u;
-                        l = wl ? 0u : l;
-                        h += wl;
-                        hre = wl != 0;
-                    }
-                    if (++cc == ncand && it + 1 < g1 - g0) {
-                        if (sq_run) atomicAdd(&w->jsq[jl], sq_run);
-                        sq_run = 0;
-                        jl = min((uint32_t)__ffs(nonempty & (0xFFFFFFFEu << jl)) - 1u, 31u);
-                        load_job(jl);
-                        hre = true;
+            w->order[rank] = (uint8_t)lane;
+            __syncwarp();                                                // lists, records and order written
+            const uint32_t olane = w->order[lane];
+            uint32_t T;
+            const uint32_t orows = __shfl_sync(FULL, rows, olane);
+            uint32_t rstart = warp_prefix(orows, lane, T);
+            if (!orows) rstart = NO_ITEM;                                // no row: after every row
+            // ---- phase B: 32 rows at a time, one per lane, two candidates of each per turn
+            uint32_t qn = 0;
+            for (uint32_t g0 = 0; g0 < T; g0 += 32) {
+                // the job of row g: the last one (in rank order) that starts at or before it; starts
+                // within these rows as a bit mask
+                const uint32_t rel0 = rstart - g0;
+                const unsigned before = __ballot_sync(FULL, rstart < g0);
+                const unsigned starts = __reduce_or_sync(FULL, rel0 < 32u ? 1u << rel0 : 0u);
+                const int o = __popc(before) + __popc(starts & (0xFFFFFFFFu >> (31 - lane))) - 1;
+                const uint32_t r = g0 + lane - __shfl_sync(FULL, rstart, o), jl = __shfl_sync(FULL, olane, o);
+                const ulonglong2 mm = *(const ulonglong2 *)&w->job[jl].m63;
+                const uint2 jj = *(const uint2 *)&w->job[jl].m64;        // m64, geo
+                const uint32_t L = jj.y & 0xFFu, H = jj.y >> 8 & 0xFFu, E2 = jj.y >> 16 & 0x3Fu;
+                // row r = (h, d), h fastest.  (r + 1/2) / H is 1/(2H) >= 2^-9 from an integer, and below
+                // R/2 + 1 < 32: far more than the division's error (2^-21 relative)
+                const uint32_t d = (uint32_t)__fdividef((float)r + 0.5f, (float)H), h = r - d * H;
+                const uint32_t sf = E2 ? d + 1 : 0, sg = E2 - sf;
+                const uint32_t full = H * (E2 ? E2 - 1 : 1) >> 1;        // full rows
+                const bool live = g0 + lane < T;
+                const int len = live ? (int)(r < full ? L : L >> 1) : 0;
+                const uint32_t x0 = jj.y >> 22;
+                const uint64_t fy = live ? (uint64_t)w->dbuf[x0 + L + h] << sf : 0;
+                const uint64_t gy = live ? (uint64_t)w->dbuf[x0 + L + H - 1 - h] << sg : 0;
+                const int turns = (int)__reduce_max_sync(FULL, (unsigned)len);
+                const uint32_t tag = jl << 26;
+                // a lane past the end of its row reads on, within the warp's area, and passes nothing
+                const uint32_t *xf = w->dbuf + (live ? x0 : 0), *xg = w->dbuf + (live ? x0 + L - 1 : 0);
+#pragma unroll 1
+                for (int l = 0; l < turns; l += 2) {
+                    uint64_t v0, v1;
+                    const uint32_t p0 = candidate(xf[0], xg[0], fy, gy, jj.x, mm.x, mm.y, v0);
+                    const uint32_t p1 = candidate(xf[1], xg[-1], fy, gy, jj.x, mm.x, mm.y, v1);
+                    xf += 2;
+                    xg -= 2;
+                    const bool b0 = l < len && (p0 & 1u), b1 = l + 1 < len && (p1 & 1u);
+                    const unsigned a0 = __ballot_sync(FULL, b0), a1 = __ballot_sync(FULL, b1);
+                    const unsigned below = (1u << lane) - 1u;
+                    const uint32_t n0 = __popc(a0);
+                    if (b0) w->q[qn + __popc(a0 & below)] = v0 | (uint64_t)tag << 32;
+                    if (b1) w->q[qn + n0 + __popc(a1 & below)] = v1 | (uint64_t)tag << 32;
+                    qn += n0 + __popc(a1);
+                    // the queue is emptied 32 at a time, and whole after the round's last turn
+                    const uint32_t least = l + 2 >= turns && g0 + 32 >= T ? 1u : 32u;
+                    while (qn >= least) {
+                        const uint32_t n = min(qn, 32u);
+                        qn -= n;
+                        __syncwarp();
+                        process_queue(a, w, qn, n, lane, cnt);
+                        __syncwarp();
                     }
                 }
-                const unsigned m = __ballot_sync(FULL, pass);
-                if (pass) {
-                    const uint32_t pos = qn + __popc(m & ((1u << lane) - 1u));
-                    w->qu[pos] = u;
-                    w->qidx[pos] = cidx;
-                    w->qj[pos] = (uint8_t)jcur;
-                }
-                qn += __popc(m);
-                __syncwarp();
-                if (qn >= 32) {
-                    process_queue(a, w, qn - 32, 32, lane);
-                    qn -= 32;
-                    __syncwarp();
-                }
             }
-            if (sq_run) atomicAdd(&w->jsq[jl], sq_run);
-            if (qn) process_queue(a, w, 0, qn, lane);
-            __syncwarp();
-            if (fits) {                        // this lane's 4-set is done: its ext_sqrt into its item
-                cnt.use(a, J.item);
-                cnt.sqrt_ += w->jsq[lane];
-                w->jsq[lane] = 0;
-                if (RING) rel = true;
-            }
-            pending = pending && !fits;
-            old = pending;
+            const bool other = fits && J.item != cnt.item;               // counted with its 4-set
+            if (__any_sync(FULL, other)) cnt.add(a, w, lane, other, J.item, 0, w->job[lane].item >> 20, 0);
+            if (fits) pending = false;
+            if (RING && fits) rel = true;
         }
         __syncwarp();
         if (lane == 0 && w->n_ext) {          // this round's extensions (and any from the per-lane path)
@@ -1153,16 +1311,25 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
         }
         if (!round && drained) break;          // warp-uniform
     }
-    cnt.flush(a);
+    cnt.flush(a, w, lane);
+    __syncwarp();
+    if (lane < ICACHE && w->ic[lane].item != NO_ITEM)
+        count_global(a, w->ic[lane].item, w->ic[lane].cand, w->ic[lane].sqrt_, w->ic[lane].mdiv);
+    __syncwarp();
     return RING ? __any_sync(FULL, took) : false;
 }
 
-__global__ void __launch_bounds__(EBS, 3) extend_jobs(const SearchArgs a) {
+__global__ void __launch_bounds__(EBS, 3) extend_jobs(const __grid_constant__ SearchArgs a) {
     extern __shared__ __align__(16) unsigned char esmem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     WarpArea *w = (WarpArea *)(esmem + (size_t)wid * sizeof(WarpArea));
-    const uint64_t njobs = min(*(volatile ull *)&a.status->n_jobs, (ull)a.jobs_cap);
-    engine_loop<false>(a, w, lane, njobs);
+    const uint32_t njobs = (uint32_t)min(*(volatile ull *)&a.status->n_jobs, (ull)a.jobs_cap);
+    if (njobs == 0) return;
+    const uint32_t warps = gridDim.x * EWARPS;
+    const uint32_t quota = min((njobs + warps - 1) / warps, 32u);                // 1 at least
+    // a stretch is a 32nd of a warp's share, 32 to 256 4-sets (one atomic each)
+    const uint32_t stretch = quota < 32 ? quota : 32u * min(max(njobs / (warps * 1024), 1u), 8u);
+    engine_loop<false>(a, w, lane, njobs, quota, stretch);
 }
 
 // ================================================================== the persistent kernel
@@ -1188,7 +1355,7 @@ static_assert(P_TS_OFF + sizeof(TileShared) <= PWARPS * sizeof(WarpArea),
               "the tile layout and tile state fit in the engine's warp areas");
 static_assert(PWARPS * sizeof(WarpArea) + 1024 + 128 <= 228 * 1024 / 3, "three persistent CTAs per SM");
 
-__global__ void __launch_bounds__(PBS, 3) search_persist(const SearchArgs a) {
+__global__ void __launch_bounds__(PBS, 3) search_persist(const __grid_constant__ SearchArgs a) {
     using L = TileLayout<PTL>;
     extern __shared__ __align__(16) unsigned char smem[];
     TileShared &ts = *reinterpret_cast<TileShared *>(smem + P_TS_OFF);
@@ -1236,7 +1403,7 @@ __global__ void __launch_bounds__(PBS, 3) search_persist(const SearchArgs a) {
             }
         } else {
             WarpArea *w = (WarpArea *)(smem + (size_t)wid * sizeof(WarpArea));
-            if (engine_loop<true>(a, w, lane, 0) && lane == 0) s_busy = 1;
+            if (engine_loop<true>(a, w, lane, 0u, 32u, 0u) && lane == 0) s_busy = 1;
             __syncthreads();
             if (tid == 0) {
                 if (s_busy) {

@@ -69,7 +69,7 @@ struct SearchArgs {
     const uint64_t *spfq;      // spf | quot << 32, m < tab_n
     const uint16_t *ndiv;      // divisor counts, m < tab_n
     uint64_t tab_n;
-    const uint4 *fac3;         // odd m: up to three odd primes (p | e << 24, ascending) and the cofactor
+    const uint4 *fac;          // fac[m >> 1] of odd m: up to four primes (p | e << 24, ascending)
     unsigned long long *counters;   // [n_items][K_SLOTS]
     ps4_hit *hits;   uint32_t hits_cap;
     ps4_ext *exts;   uint32_t exts_cap;
@@ -149,7 +149,7 @@ void canonical_order_into(const ps4_hit *hits, uint64_t nh, const ps4_ext *exts,
 struct CtxView {
     const uint64_t *spfq;
     const uint16_t *ndiv;
-    const uint4 *fac3;
+    const uint4 *fac;
     uint64_t tab_n, s_hi_max;
     uint32_t cap_reps, cap_divs, cap_ext, flags;
     int device, num_sms;
@@ -158,9 +158,12 @@ struct CtxView {
 int ctx_view(ps4_ctx *c, CtxView *v);
 int ctx_fail(ps4_ctx *c, int code, const char *msg);
 
+// entries of the odd numbers' factor table next to tables of m < tab_n
+inline uint64_t fac_n(uint64_t tab_n) { return (tab_n + 1) / 2; }
+
 // Launchers (ps4_kernels.cu).  Return a cudaError_t value.
 int launch_tables(uint64_t *spfq, uint16_t *ndiv, uint64_t tab_n, void *stream);
-int launch_fac3(uint4 *fac3, uint64_t tab_n, void *stream);
+int launch_fac(uint4 *fac, uint64_t n, void *stream);
 // two-kernel pipeline (ps4_extend.cu): 4-set generation into the job queue, then extension
 int launch_gen(SearchArgs a, int grid, void *stream);
 int launch_ext(const SearchArgs &a, int grid, void *stream);
