@@ -577,8 +577,6 @@ struct ItemCount {                       // counters of an item that the warp ho
     ull cand, sqrt_;
 };
 
-// 6.8 KB: three CTAs take 167 KB, which leaves 92 KB of L1 for the table lookups of phase A (with 8.6 KB
-// areas it was 28 KB)
 struct WarpArea {
     EJob job[32];
     uint32_t dbuf[DCAP];                 // a turn may read up to LCAP entries past a list's ends: the
@@ -591,11 +589,14 @@ struct WarpArea {
     ItemCount ic[ICACHE];
     ExtEntry ext[EXCAP];
     uint32_t jid[32];                    // queue index of each lane's 4-set
+    // the loop's own state, out of the registers between its claims (the same for all lanes)
+    uint32_t njobs, quota, stretch;      // queue length; lanes that hold a 4-set; 4-sets per stretch
+    uint32_t st_cur, st_rem, last;       // the stretch at hand; whether it is the last
     uint32_t n_ext;
     uint8_t order[32];                   // lanes by row length, longest first
 };
 static_assert(sizeof(EJob) * 32 >= 4 * LCAP && 4 * 32 * 2 * FSIDE >= 4 * LCAP, "neighbours of dbuf");
-static_assert(EWARPS * sizeof(WarpArea) + 1024 <= 164 * 1024 / 3, "three engine CTAs per SM in the 164 KB carve-out");
+static_assert(EWARPS * sizeof(WarpArea) + 1024 <= 228 * 1024 / 3, "three engine CTAs per SM");
 
 // Residue masks of a candidate's v = f + g = 2u.  e + C = u^2 + (C - A) must be a square mod 64, 63
 // and 65 for both remaining members C (s4.c:192-194): one bit test per modulus, against the AND of
@@ -829,7 +830,7 @@ static __device__ __noinline__ uint64_t merge_slow(const uint64_t *spfq, uint32_
 struct LaneJob {                                 // a lane's 4-set in its round
     uint32_t item, ncand, nd;
     uint32_t L, H, rows;                         // list lengths; full rows and the last half one
-    uint32_t slots;                              // first prime slot of the row list | of the other list << 8
+    uint32_t slots;                              // row list: first prime slot | primes << 8, the other << 16
     bool big;                                    // for the per-lane divisor walk
 };
 
@@ -948,16 +949,18 @@ __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJ
             if (H * k >= L || !below32) break;
             w->fp[so + no++][lane] = x;
             nr--;
-            L /= k;
+            L = (uint32_t)(__fdividef((float)L, (float)k) + 0.5f);   // exact: k divides L < 2^14
             H *= k;
         }
         if (H > L) {
-            const uint32_t s = L, q = sr; L = H; H = s; sr = so; so = q;
+            uint32_t s = L; L = H; H = s;
+            s = sr; sr = so; so = s;
+            s = nr; nr = no; no = s;
         }
     } else {
         wide = side_is_wide(w->fp, lane, 0, na);   // m2's side is a divisor of m2
     }
-    J.slots = sr | so << 8;
+    J.slots = sr | nr << 8 | so << 16 | no << 24;
     J.L = L;
     J.H = H;
     // same-parity complementary pairs with f < g: the reference's ext_cand (s4.c:191)
@@ -970,36 +973,29 @@ __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJ
     return true;
 }
 
-// The n divisors of prod pr[q]^ex[q], q in [q0, q1), in mixed-radix order (first prime
-// fastest), in one flat loop: prime q's block repeats the list so far ex[q] times, each copy
-// times p_q, so d[j] = d[j - cur] * p_q with cur the list length before q.
-__device__ __forceinline__ void gen_list(uint32_t *d, const uint32_t (*fp)[32], int lane, int q0, uint32_t n) {
+// The divisors of the n prime powers from slot q, in mixed-radix order (first prime fastest): prime
+// after prime, the list so far is repeated e times, each copy p times the one before.
+__device__ __forceinline__ void gen_list(uint32_t *d, const uint32_t (*fp)[32], int lane, uint32_t q, uint32_t n) {
     d[0] = 1;
-    if (n <= 1) return;
-    int q = q0;
-    uint32_t x = fp[q][lane];
-    uint32_t p = x & 0xFFFFFFu, cur = 1, end = (x >> 24) + 1;
-    for (uint32_t j = 1; j < n; j++) {
-        if (j == end) {
-            cur = end;
-            x = fp[++q][lane];
-            p = x & 0xFFFFFFu;
-            end = cur * ((x >> 24) + 1);
-        }
-        d[j] = d[j - cur] * p;
+    uint32_t cur = 1;
+    for (uint32_t i = 0; i < n; i++) {
+        const uint32_t x = fp[q + i][lane], p = x & 0xFFFFFFu, add = cur * (x >> 24);
+#pragma unroll 1
+        for (uint32_t j = 0; j < add; j++) d[cur + j] = d[j] * p;
+        cur += add;
     }
 }
 
 // A 4-set whose factored divisor lists exceed the warp buffer or 32 bits: the per-lane divisor walk.
 // Returns its ext_sqrt.
 template <bool COH>
-static __device__ __noinline__ uint32_t extend_big(const SearchArgs &a, uint64_t j, uint32_t qid, ExtEntry *el,
+static __device__ __noinline__ uint32_t extend_big(const SearchArgs &a, uint32_t qid, ExtEntry *el,
                                                    uint32_t *el_n) {
     ull cand = 0, sq = 0;
     uint32_t r[6], item, best, md = 0;
     uint64_t v[4], S;
     int bi, bj, bk;
-    get_job<COH>(a.jobs, j, r, item);
+    get_job<COH>(a.jobs, qid, r, item);
     quad_values(r, v, S);
     choose_pair(v, r, a.ndiv, bi, bj, bk, best);
     extend_quad(a, r, v, S, bi, bj, bk, qid, cand, sq, md, el, el_n, EXCAP);
@@ -1121,22 +1117,23 @@ template <bool RING>
 __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint32_t njobs, uint32_t quota,
                                             uint32_t stretch) {
     const unsigned FULL = 0xffffffffu;
-    if (lane == 0) w->n_ext = 0;
+    if (lane == 0) {
+        w->n_ext = 0;
+        w->njobs = njobs; w->quota = quota; w->stretch = stretch;
+        w->st_cur = w->st_rem = w->last = 0;
+    }
     if (lane < ICACHE) w->ic[lane].item = NO_ITEM;
     __syncwarp();
     WarpCounters cnt;
     bool pending = false, drained = false, rel = false, took = false;
-    uint32_t myjob = 0;
     uint64_t mypos = 0;
-    uint32_t st_cur = 0, st_rem = 0;               // the warp's stretch of the queue (not RING)
-    bool last = false;                             // no further stretch
 
     // Rounds: every lane without a 4-set takes the next one from the queue; a lane whose divisor lists
     // did not fit keeps its 4-set, sets it up again and goes first in the next round's placement.
     for (;;) {
         const bool old = pending;
         if (!drained) {
-            const bool need = !pending && (uint32_t)lane < quota;
+            const bool need = !pending && (uint32_t)lane < w->quota;
             const unsigned m = __ballot_sync(FULL, need);
             const uint32_t n = (uint32_t)__popc(m), rank = (uint32_t)__popc(m & ((1u << lane) - 1u));
             int stop = 0;
@@ -1155,35 +1152,36 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
                 if (need && rank < got && ring_wait_ready(a, base + rank)) {
                     pending = true;
                     mypos = base + rank;
-                    myjob = (uint32_t)(mypos & a.ring_mask);
+                    w->jid[lane] = (uint32_t)(mypos & a.ring_mask);
                 }
                 took |= pending;
             } else {
+                const uint32_t cur = w->st_cur, rem = w->st_rem, size = w->stretch;
+                bool last = w->last != 0;
                 uint32_t nx = 0, avail = 0;
-                if (st_rem < n && !last) {                               // a new stretch behind the old one
+                if (rem < n && !last) {                                  // a new stretch behind the old one
                     if (lane == 0) {
-                        nx = atomicAdd(&a.status->ext_next, stretch);
+                        nx = atomicAdd(&a.status->ext_next, size);
                         stop = *(volatile ull *)&a.status->err != 0ull;
                     }
                     nx = __shfl_sync(FULL, nx, 0);
                     stop = __shfl_sync(FULL, stop, 0);
                     if (stop) break;                                     // warp-uniform
-                    avail = nx < njobs ? min(stretch, njobs - nx) : 0u;
-                    last = avail < stretch;
+                    avail = nx < w->njobs ? min(size, w->njobs - nx) : 0u;
+                    last = avail < size;
                 }
-                if (need && rank < st_rem + avail) {
+                if (need && rank < rem + avail) {
                     pending = true;
-                    myjob = rank < st_rem ? st_cur + rank : nx + (rank - st_rem);
+                    w->jid[lane] = rank < rem ? cur + rank : nx + (rank - rem);
                 }
-                const uint32_t used = min(n, st_rem + avail);
-                if (used < st_rem) {
-                    st_cur += used;
-                    st_rem -= used;
-                } else {
-                    st_cur = nx + (used - st_rem);
-                    st_rem = st_rem + avail - used;
+                const uint32_t used = min(n, rem + avail);
+                __syncwarp();                                            // read by all
+                if (lane == 0) {
+                    w->st_cur = used < rem ? cur + used : nx + (used - rem);
+                    w->st_rem = rem + avail - used;
+                    w->last = last;
                 }
-                drained = last && st_rem == 0;                           // warp-uniform
+                drained = last && rem + avail == used;                   // warp-uniform
             }
         }
         // ---- phase A: one 4-set per lane
@@ -1193,9 +1191,9 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
         const bool mine = pending;
         uint32_t bsq = 0;
         if (pending) {
-            pending = job_setup<RING>(a, myjob, J, w, lane);
+            pending = job_setup<RING>(a, w->jid[lane], J, w, lane);
             if (pending && J.big) {                                      // rare
-                bsq = extend_big<RING>(a, myjob, myjob, w->ext, &w->n_ext);
+                bsq = extend_big<RING>(a, w->jid[lane], w->ext, &w->n_ext);
                 pending = false;
             }
         }
@@ -1213,10 +1211,9 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
             if (!old) base = tot_old + bn;
             const bool fits = pending && base + want <= (uint32_t)DCAP;
             if (fits) {
-                w->jid[lane] = myjob;
                 w->job[lane].geo |= base << 22;
-                gen_list(w->dbuf + base, w->fp, lane, J.slots & 0xFFu, J.L);             // rows: L entries
-                gen_list(w->dbuf + base + J.L, w->fp, lane, J.slots >> 8, J.H);          // H entries
+                gen_list(w->dbuf + base, w->fp, lane, J.slots & 0xFFu, J.slots >> 8 & 0xFFu);      // rows: L entries
+                gen_list(w->dbuf + base + J.L, w->fp, lane, J.slots >> 16 & 0xFFu, J.slots >> 24); // H entries
             }
             // rows by length, longest first, so that the 32 rows of a turn are about equally long:
             // each lane's rank by (length, lane), then the rows' prefix in rank order
@@ -1292,8 +1289,9 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
                     }
                 }
             }
-            const bool other = fits && J.item != cnt.item;               // counted with its 4-set
-            if (__any_sync(FULL, other)) cnt.add(a, w, lane, other, J.item, 0, w->job[lane].item >> 20, 0);
+            const uint32_t it = w->job[lane].item;
+            const bool other = fits && (it & 0xFFFFFu) != cnt.item;      // counted with its 4-set
+            if (__any_sync(FULL, other)) cnt.add(a, w, lane, other, it & 0xFFFFFu, 0, it >> 20, 0);
             if (fits) pending = false;
             if (RING && fits) rel = true;
         }
