@@ -38,14 +38,18 @@ struct ps4_ctx {
     uint4 *d_fac = nullptr;
     // working buffers (grown on demand)
     Item *d_items = nullptr; uint32_t items_cap = 0;
-    unsigned long long *d_counters = nullptr; uint32_t counters_items = 0;
+    // one block holds the status and the items' counters, so that both are cleared and copied back at
+    // once; a call of few items has its segments behind them, and clears and uploads in one copy
+    unsigned char *d_block = nullptr; uint64_t block_cap = 0;
+    unsigned char *h_block = nullptr; uint64_t h_block_cap = 0;      // pinned: where the block lands
+    unsigned char *h_stage = nullptr; uint64_t h_stage_cap = 0;      // pinned: zeros and segments to upload
+    Status *d_status = nullptr;
+    unsigned long long *d_counters = nullptr;
     ps4_hit *d_hits = nullptr; uint32_t hits_cap = 0;
     ps4_ext *d_exts = nullptr; uint32_t exts_cap = 0;
     ps4_six *d_sixes = nullptr; uint32_t sixes_cap = 0;
     ps4_quad *d_quads = nullptr; uint64_t quads_cap = 0;
     uint32_t *d_scratch = nullptr; size_t scratch_words = 0;
-    Status *d_status = nullptr;
-    Status *h_status = nullptr;          // pinned
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
     uint64_t last_launches = 0;
@@ -72,8 +76,7 @@ struct ps4_ctx {
     uint64_t jobs_cap_max = 1ull << 29;      // largest job queue (entries; 2^29 = 12.9 GB): fewer,
                                              //   longer batches, fewer launch tails
     double tuned_rate = 0.0;
-    // pinned staging of the segments, and the kept CUDA graph of a multi-batch call
-    Item *h_segs = nullptr; uint64_t h_segs_cap = 0;
+    // the kept CUDA graph of a multi-batch call
     // pinned landing buffers of the result records (copied back at full speed, then ordered into the
     // caller's buffers)
     ps4_hit *h_hits = nullptr; uint64_t h_hits_cap = 0;
@@ -86,11 +89,11 @@ struct ps4_ctx {
     std::vector<cudaEvent_t> kev;
     size_t kev_used = 0;
     double gen_ms = 0.0, ext_ms = 0.0;
-    // triple extension (grown on demand)
+    // triple extension (grown on demand): the members in; counters, states and records out in one block
     uint64_t *d_tri_in = nullptr; uint64_t tri_in_cap = 0;
-    uint8_t *d_tri_state = nullptr; uint64_t tri_state_cap = 0;
-    ps4_tri_ext *d_tri_out = nullptr; uint64_t tri_out_cap = 0;
-    unsigned long long *d_tri_cnt = nullptr; uint64_t tri_cnt_cap = 0;   // n_out, n_cand, n_sqrt
+    unsigned char *d_tri = nullptr; uint64_t tri_cap = 0;
+    unsigned char *h_tri = nullptr; uint64_t h_tri_cap = 0;          // pinned
+    uint64_t tri_out_cap = 0;                                        // records the device block holds
     std::string err;
 };
 
@@ -143,6 +146,18 @@ static int grow_pinned(ps4_ctx *c, T *&ptr, uint64_t &cap, uint64_t need) {
     return 0;
 }
 
+// The block of a call: status, counters of n_items, then (small calls) n_segs segments.
+static const size_t BLOCK_HEAD = (sizeof(Status) + 255) & ~(size_t)255;
+static size_t block_bytes(uint64_t n_items) { return BLOCK_HEAD + (size_t)n_items * K_SLOTS * sizeof(unsigned long long); }
+static const uint32_t SMALL_ITEMS = 16, SMALL_SEGS = 64;             // uploaded together with their zeros
+static int reserve_block(ps4_ctx *c, uint32_t n_items) {
+    if (grow(c, c->d_block, c->block_cap, std::max<uint64_t>(c->block_cap, block_bytes(n_items) + SMALL_SEGS * sizeof(Item))))
+        return PS4_ERR_CUDA;
+    c->d_status = reinterpret_cast<Status *>(c->d_block);
+    c->d_counters = reinterpret_cast<unsigned long long *>(c->d_block + BLOCK_HEAD);
+    return grow_pinned(c, c->h_block, c->h_block_cap, block_bytes(n_items));
+}
+
 static uint64_t isqrt_host(uint64_t n) {
     uint64_t r = (uint64_t)std::sqrt((double)n);
     while (r * r > n) r--;
@@ -160,13 +175,14 @@ extern "C" uint64_t ps4_last_launches(const ps4_ctx *ctx) { return ctx ? ctx->la
 
 extern "C" void ps4_destroy(ps4_ctx *c) {
     if (!c) return;
-    cudaFree(c->d_spfq); cudaFree(c->d_ndiv); cudaFree(c->d_items); cudaFree(c->d_counters);
+    cudaFree(c->d_spfq); cudaFree(c->d_ndiv); cudaFree(c->d_items); cudaFree(c->d_block);
     cudaFree(c->d_hits); cudaFree(c->d_exts); cudaFree(c->d_sixes); cudaFree(c->d_quads);
-    cudaFree(c->d_scratch); cudaFree(c->d_status); cudaFree(c->d_jobs); cudaFree(c->d_raw); cudaFree(c->d_seq);
+    cudaFree(c->d_scratch); cudaFree(c->d_jobs); cudaFree(c->d_raw); cudaFree(c->d_seq);
     cudaFree(c->d_fac);
-    cudaFree(c->d_tri_in); cudaFree(c->d_tri_state); cudaFree(c->d_tri_out); cudaFree(c->d_tri_cnt);
-    if (c->h_status) cudaFreeHost(c->h_status);
-    if (c->h_segs) cudaFreeHost(c->h_segs);
+    cudaFree(c->d_tri_in); cudaFree(c->d_tri);
+    if (c->h_block) cudaFreeHost(c->h_block);
+    if (c->h_stage) cudaFreeHost(c->h_stage);
+    if (c->h_tri) cudaFreeHost(c->h_tri);
     if (c->h_hits) cudaFreeHost(c->h_hits);
     if (c->h_exts) cudaFreeHost(c->h_exts);
     if (c->h_sixes) cudaFreeHost(c->h_sixes);
@@ -221,8 +237,6 @@ extern "C" int ps4_create(const ps4_config *cfg, ps4_ctx **out) {
     c->tab_n = 2 * isqrt_host(c->cfg.s_hi_max) + 64;      // s4.c:440
     CUDA_TRY(c, cudaMalloc((void **)&c->d_spfq, c->tab_n * sizeof(uint64_t)));
     CUDA_TRY(c, cudaMalloc((void **)&c->d_ndiv, c->tab_n * sizeof(uint16_t)));
-    CUDA_TRY(c, cudaMalloc((void **)&c->d_status, sizeof(Status)));
-    CUDA_TRY(c, cudaMallocHost((void **)&c->h_status, sizeof(Status)));
     CUDA_TRY(c, (cudaError_t)launch_tables(c->d_spfq, c->d_ndiv, c->tab_n, c->stream));
     CUDA_TRY(c, cudaMalloc((void **)&c->d_fac, fac_n(c->tab_n) * sizeof(uint4)));
     CUDA_TRY(c, (cudaError_t)launch_fac(c->d_fac, fac_n(c->tab_n), c->stream));
@@ -425,12 +439,11 @@ static int enqueue_items(ps4_ctx *c) {
 
     // every allocation before any launch (a captured call may allocate nothing)
     if (grow32(c, c->d_items, c->items_cap, std::max<size_t>(segs.size(), 1))) return PS4_ERR_CUDA;
-    if (c->h_segs_cap < segs.size() || !c->h_segs) {
-        if (c->h_segs) cudaFreeHost(c->h_segs);
-        c->h_segs = nullptr;
-        c->h_segs_cap = std::max<uint64_t>(segs.size(), 1024);
-        CUDA_TRY(c, cudaMallocHost((void **)&c->h_segs, c->h_segs_cap * sizeof(Item)));
-    }
+    // a call of few items uploads its zeros and segments in one copy, to one place
+    const bool small = n_items <= SMALL_ITEMS && segs.size() <= SMALL_SEGS;
+    const size_t blk = block_bytes(n_items), segs_bytes = segs.size() * sizeof(Item);
+    if (grow_pinned(c, c->h_stage, c->h_stage_cap, (small ? blk : 0) + segs_bytes)) return PS4_ERR_CUDA;
+    Item *const dev_items = small ? reinterpret_cast<Item *>(c->d_block + blk) : c->d_items;
     if (kernel == PS4_KERNEL_BATCHED && c->d_jobs_words < 6 * c->jobs_cap)
         if (grow(c, c->d_jobs, c->d_jobs_words, 6 * c->jobs_cap)) return PS4_ERR_CUDA;
     // gen_ctas counts 512 threads per SM: one or two 512-thread CTAs on 2^14-S tiles, twice as
@@ -511,11 +524,13 @@ static int enqueue_items(ps4_ctx *c) {
         for (size_t b : batch_start) key_add(key, b);
         key_add(key, a);
         key_add(key, kernel); key_add(key, n_items); key_add(key, grid); key_add(key, g_gen); key_add(key, g_ext);
-        key_add(key, stage_cap); key_add(key, c->d_scratch); key_add(key, c->h_segs); key_add(key, c->d_items);
+        key_add(key, stage_cap); key_add(key, c->d_scratch); key_add(key, c->h_stage); key_add(key, dev_items);
+        key_add(key, c->h_block);
         key_add(key, c->stream);
     }
-    if (!segs.empty()) memcpy(c->h_segs, segs.data(), segs.size() * sizeof(Item));
-    c->h2d_bytes += segs.size() * sizeof(Item);
+    if (small) memset(c->h_stage, 0, blk);
+    if (!segs.empty()) memcpy(c->h_stage + (small ? blk : 0), segs.data(), segs_bytes);
+    c->h2d_bytes += (small ? blk : 0) + segs_bytes;
     CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
     if (graph && c->graph_exec && key == c->graph_key) {
         CUDA_TRY(c, cudaGraphLaunch(c->graph_exec, c->stream));
@@ -526,20 +541,22 @@ static int enqueue_items(ps4_ctx *c) {
         const uint64_t launches0 = c->last_launches;
         int rc = PS4_OK;
         cudaError_t e = cudaSuccess;
-        if (!segs.empty())
-            e = cudaMemcpyAsync(c->d_items, c->h_segs, segs.size() * sizeof(Item), cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(c->d_counters, 0, (size_t)n_items * K_SLOTS * sizeof(unsigned long long), c->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(Status), c->stream);
+        if (small) {
+            e = cudaMemcpyAsync(c->d_block, c->h_stage, blk + segs_bytes, cudaMemcpyHostToDevice, c->stream);
+        } else {
+            if (!segs.empty())
+                e = cudaMemcpyAsync(c->d_items, c->h_stage, segs_bytes, cudaMemcpyHostToDevice, c->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(c->d_block, 0, blk, c->stream);
+        }
         if (e == cudaSuccess && kernel == PS4_KERNEL_BATCHED) {
             for (size_t b = 0; b < batch_start.size() && e == cudaSuccess; b++) {
                 const size_t s0 = batch_start[b], s1 = b + 1 < batch_start.size() ? batch_start[b + 1] : segs.size();
-                a.items = c->d_items + s0;
+                a.items = dev_items + s0;
                 a.n_items = (uint32_t)(s1 - s0);
                 a.n_tiles = batch_tiles[b];
                 a.s_top = segs[s1 - 1].hi;                   // a batch's segments ascend by their end
-                // n_jobs, tile_next, ext_next: the per-batch tail of the status block
-                e = cudaMemsetAsync(&c->d_status->n_jobs, 0, 2 * sizeof(unsigned long long), c->stream);
+                // n_jobs, tile_next, ext_next: the per-batch tail of the status block (clear for the first)
+                if (b > 0) e = cudaMemsetAsync(&c->d_status->n_jobs, 0, 2 * sizeof(unsigned long long), c->stream);
                 if (timed && e == cudaSuccess) e = cudaEventRecord(c->kev[4 * b], c->stream);
                 if (e == cudaSuccess) e = (cudaError_t)launch_gen(a, g_gen, c->stream);
                 if (timed && e == cudaSuccess) e = cudaEventRecord(c->kev[4 * b + 1], c->stream);
@@ -553,12 +570,12 @@ static int enqueue_items(ps4_ctx *c) {
                 if (timed) c->kev_used = 4 * (b + 1);
             }
         } else if (e == cudaSuccess && persist && tiles_total > 0) {
-            a.items = c->d_items; a.n_items = (uint32_t)segs.size(); a.n_tiles = tiles_total;
+            a.items = dev_items; a.n_items = (uint32_t)segs.size(); a.n_tiles = tiles_total;
             e = (cudaError_t)launch_ring_init(c->d_seq, c->ring_cap, c->stream);
             if (e == cudaSuccess) e = (cudaError_t)launch_persist(a, g_persist, c->stream);
             c->last_launches += 2;
         } else if (e == cudaSuccess && tiles_total > 0) {
-            a.items = c->d_items; a.n_items = (uint32_t)segs.size(); a.n_tiles = tiles_total;
+            a.items = dev_items; a.n_items = (uint32_t)segs.size(); a.n_tiles = tiles_total;
             a.scratch = c->d_scratch; a.stage_cap = stage_cap;
             // launch_search's selector: PS4_KERNEL_BATCHED there is the fused persistent kernel
             e = (cudaError_t)launch_search(a, kernel == PS4_KERNEL_PLAIN ? PS4_KERNEL_PLAIN : PS4_KERNEL_BATCHED, grid,
@@ -587,7 +604,8 @@ static int enqueue_items(ps4_ctx *c) {
         if (rc) return rc;
     }
     CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-    CUDA_TRY(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(Status), cudaMemcpyDeviceToHost, c->stream));
+    // the status and every item's counters, in one copy that the result's wait covers
+    CUDA_TRY(c, cudaMemcpyAsync(c->h_block, c->d_block, blk, cudaMemcpyDeviceToHost, c->stream));
     return PS4_OK;
 }
 
@@ -612,8 +630,7 @@ static int begin_items(ps4_ctx *c, const uint64_t *lo, const uint64_t *hi, uint3
         p.items[i].hi = b;
         p.items[i].id = i;
     }
-    if (grow32(c, c->d_items, c->items_cap, n_items)) return PS4_ERR_CUDA;
-    if (grow32(c, c->d_counters, c->counters_items, (uint64_t)n_items * K_SLOTS)) return PS4_ERR_CUDA;
+    if (reserve_block(c, n_items)) return PS4_ERR_CUDA;
     p.dump = (c->cfg.flags & PS4_F_DUMP4) && want_dump && dump_cap > 0;
     if (p.dump && grow(c, c->d_quads, c->quads_cap, dump_cap)) return PS4_ERR_CUDA;
     // result buffers sized up front from the call's width (4-sets with an extension stay below
@@ -644,7 +661,7 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
             if (rc) return rc;
         }
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        c->d2h_bytes += sizeof(Status);
+        c->d2h_bytes += block_bytes(n_items);
         if (p.tiles > 0) {
             float ms = 0.f;
             cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -659,7 +676,7 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
                 c->ext_ms += x;
             }
         }
-        const Status &st = *c->h_status;
+        const Status &st = *reinterpret_cast<const Status *>(c->h_block);
         const unsigned code = (unsigned)(st.err & 0xFF);
         const unsigned long long errS = st.err >> 8;
         if (code == E_QUEUE) {                   // a batch outgrew the job queue: narrower batches
@@ -722,9 +739,7 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
                                (unsigned long long)res->quads_cap, st.n_quads);
             }
         }
-        std::vector<unsigned long long> k((size_t)n_items * K_SLOTS);
-        CUDA_TRY(c, cudaMemcpyAsync(k.data(), c->d_counters, k.size() * sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, c->stream));
+        const unsigned long long *k = reinterpret_cast<const unsigned long long *>(c->h_block + BLOCK_HEAD);
         const bool fits = res && st.n_hits <= res->hits_cap && st.n_exts <= res->exts_cap &&
                           st.n_sixes <= res->sixes_cap;
         if (fits) {                              // the records land in pinned buffers, then go in order to res
@@ -745,9 +760,9 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
         if (res && p.dump && st.n_quads)
             CUDA_TRY(c, cudaMemcpyAsync(res->quads, c->d_quads, st.n_quads * sizeof(ps4_quad), cudaMemcpyDeviceToHost,
                                         c->stream));
-        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        c->d2h_bytes += k.size() * sizeof(unsigned long long) +
-                        (fits ? st.n_hits * sizeof(ps4_hit) + st.n_exts * sizeof(ps4_ext) +
+        if ((fits && (st.n_hits || st.n_exts || st.n_sixes)) || (res && p.dump && st.n_quads))
+            CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        c->d2h_bytes += (fits ? st.n_hits * sizeof(ps4_hit) + st.n_exts * sizeof(ps4_ext) +
                                     st.n_sixes * sizeof(ps4_six)
                               : 0) +
                         ((res && p.dump) ? st.n_quads * sizeof(ps4_quad) : 0);
@@ -981,65 +996,80 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
     if (n == 0) return PS4_OK;
     if (!abc) return set_err(c, PS4_ERR_ARG, "ps4_extend_triples: no input");
     if (dmax > (1ull << 62)) return set_err(c, PS4_ERR_ARG, "dmax %llu exceeds 2^62", (unsigned long long)dmax);
-    if (grow(c, c->d_tri_in, c->tri_in_cap, 3 * (uint64_t)n)) return PS4_ERR_CUDA;
-    if (grow(c, c->d_tri_state, c->tri_state_cap, n)) return PS4_ERR_CUDA;
-    if (grow(c, c->d_tri_cnt, c->tri_cnt_cap, 3)) return PS4_ERR_CUDA;
-    if (grow(c, c->d_tri_out, c->tri_out_cap, std::max<uint64_t>(c->tri_out_cap, std::max<uint64_t>(out_cap, 1u << 16))))
-        return PS4_ERR_CUDA;
-    CUDA_TRY(c, cudaMemcpyAsync(c->d_tri_in, abc, 3 * (size_t)n * sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
-    c->h2d_bytes += 3 * (uint64_t)n * sizeof(uint64_t);
-    unsigned long long cnt[3];
+    // device block: counters n_out, n_cand, n_sqrt (32 bytes), a state per triple, the records
+    const uint64_t off_out = (32 + (uint64_t)n + 15) & ~15ull;
+    const uint64_t FIRST = 1024;                      // records copied back with the states
+    if (grow(c, c->d_tri_in, c->tri_in_cap, std::max<uint64_t>(c->tri_in_cap, 3 * (uint64_t)n))) return PS4_ERR_CUDA;
+    c->tri_out_cap = std::max<uint64_t>(c->tri_out_cap, std::max<uint64_t>(out_cap, 1u << 16));
+    auto reserve = [&]() {
+        return grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, off_out + c->tri_out_cap * sizeof(ps4_tri_ext)));
+    };
+    if (reserve()) return PS4_ERR_CUDA;
+    if (grow_pinned(c, c->h_tri, c->h_tri_cap, off_out + FIRST * sizeof(ps4_tri_ext))) return PS4_ERR_CUDA;
+    const uint64_t in_bytes = 3 * (uint64_t)n * sizeof(uint64_t);
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_tri_in, abc, in_bytes, cudaMemcpyHostToDevice, c->stream));
+    c->h2d_bytes += in_bytes;
+    const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(c->h_tri);
+    uint64_t first = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
-        CUDA_TRY(c, cudaMemsetAsync(c->d_tri_cnt, 0, 3 * sizeof(unsigned long long), c->stream));
+        unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(c->d_tri);
+        CUDA_TRY(c, cudaMemsetAsync(d_cnt, 0, 32, c->stream));
         TriArgs t;
         t.abc = c->d_tri_in; t.n = n; t.dmax = dmax;
         t.spfq = c->d_spfq; t.ndiv = c->d_ndiv; t.tab_n = c->tab_n;
-        t.state = c->d_tri_state;
-        t.out = c->d_tri_out; t.out_cap = c->tri_out_cap;
-        t.n_out = c->d_tri_cnt; t.n_cand = c->d_tri_cnt + 1; t.n_sqrt = c->d_tri_cnt + 2;
+        t.state = c->d_tri + 32;
+        t.out = reinterpret_cast<ps4_tri_ext *>(c->d_tri + off_out); t.out_cap = c->tri_out_cap;
+        t.n_out = d_cnt; t.n_cand = d_cnt + 1; t.n_sqrt = d_cnt + 2;
         t.item_base = 0;
         t.cand_per = t.sqrt_per = nullptr;
         CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
         CUDA_TRY(c, (cudaError_t)launch_triples(t, c->stream));
         CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
         c->last_launches++;
-        CUDA_TRY(c, cudaMemcpyAsync(cnt, c->d_tri_cnt, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
+        first = std::min<uint64_t>(FIRST, c->tri_out_cap);
+        CUDA_TRY(c, cudaMemcpyAsync(c->h_tri, c->d_tri, off_out + first * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost,
+                                    c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        c->d2h_bytes += sizeof cnt;
+        c->d2h_bytes += off_out + first * sizeof(ps4_tri_ext);
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev0, c->ev1);
         c->last_ms = ms;
         if (cnt[0] <= c->tri_out_cap) break;
         // more records than the device buffer holds: grow it and run again (results do not
         // depend on the buffer)
-        if (grow(c, c->d_tri_out, c->tri_out_cap, cnt[0] * 3 / 2 + 1024)) return PS4_ERR_CUDA;
+        c->tri_out_cap = cnt[0] * 3 / 2 + 1024;
+        if (reserve()) return PS4_ERR_CUDA;
     }
-    std::vector<uint8_t> st(n);
-    CUDA_TRY(c, cudaMemcpyAsync(st.data(), c->d_tri_state, n, cudaMemcpyDeviceToHost, c->stream));
-    std::vector<ps4_tri_ext> recs(cnt[0]);
-    if (cnt[0])
-        CUDA_TRY(c, cudaMemcpyAsync(recs.data(), c->d_tri_out, cnt[0] * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost,
-                                    c->stream));
-    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    c->d2h_bytes += n + cnt[0] * sizeof(ps4_tri_ext);
-    uint64_t n_invalid = 0;
+    const uint8_t *st = c->h_tri + 32;
+    const uint64_t n_rec = cnt[0];
+    std::vector<ps4_tri_ext> recs(n_rec);
+    if (n_rec) memcpy(recs.data(), c->h_tri + off_out, std::min(n_rec, first) * sizeof(ps4_tri_ext));
+    if (n_rec > first) {
+        CUDA_TRY(c, cudaMemcpyAsync(recs.data() + first, c->d_tri + off_out + first * sizeof(ps4_tri_ext),
+                                    (n_rec - first) * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        c->d2h_bytes += (n_rec - first) * sizeof(ps4_tri_ext);
+    }
+    uint64_t n_invalid = 0, n_range = 0;
     for (uint32_t i = 0; i < n; i++) {
-        if (st[i] == TRI_RANGE)
-            return set_err(c, PS4_ERR_ARG,
-                           "triple %u (%llu, %llu, %llu) is beyond the context's factor tables (s_hi_max %llu)", i,
-                           (unsigned long long)abc[3 * i], (unsigned long long)abc[3 * i + 1],
-                           (unsigned long long)abc[3 * i + 2], (unsigned long long)c->cfg.s_hi_max);
         n_invalid += st[i] == TRI_INVALID;
+        n_range += st[i] == TRI_RANGE;
     }
-    if (state) memcpy(state, st.data(), n);
+    if (n_range) {
+        const uint32_t i = (uint32_t)((const uint8_t *)memchr(st, TRI_RANGE, n) - st);
+        return set_err(c, PS4_ERR_ARG, "triple %u (%llu, %llu, %llu) is beyond the context's factor tables (s_hi_max %llu)", i,
+                       (unsigned long long)abc[3 * (size_t)i], (unsigned long long)abc[3 * (size_t)i + 1],
+                       (unsigned long long)abc[3 * (size_t)i + 2], (unsigned long long)c->cfg.s_hi_max);
+    }
+    if (state) memcpy(state, st, n);
     std::sort(recs.begin(), recs.end(), [](const ps4_tri_ext &x, const ps4_tri_ext &y) {
         return x.item != y.item ? x.item < y.item : x.d < y.d;
     });
-    if (n_out) *n_out = cnt[0];
-    if (cnt[0] > out_cap)
+    if (n_out) *n_out = n_rec;
+    if (n_rec > out_cap)
         return set_err(c, PS4_ERR_OUTPUT_FULL, "triple output holds %llu records, %llu needed",
-                       (unsigned long long)out_cap, cnt[0]);
-    if (cnt[0]) memcpy(out, recs.data(), cnt[0] * sizeof(ps4_tri_ext));
+                       (unsigned long long)out_cap, (unsigned long long)n_rec);
+    if (n_rec) memcpy(out, recs.data(), n_rec * sizeof(ps4_tri_ext));
     if (stats) {
         stats->triples += n - n_invalid;
         stats->invalid += n_invalid;

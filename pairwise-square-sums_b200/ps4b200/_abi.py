@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from pathlib import Path
 
 PKG_ROOT = Path(__file__).resolve().parent.parent          # pairwise-square-sums_b200/
@@ -52,6 +53,11 @@ COUNTER_NAMES = ("S_done", "pairs", "S_ge3", "triples", "sets4", "sets5", "sets6
                  "ext_cand", "ext_sqrt")
 
 
+# the fields of Stats, in order: a batch turns thousands of blocks into dicts
+_COUNTERS, _HIST, _MAXIMA = struct.Struct(f"={len(COUNTER_NAMES)}Q"), struct.Struct("=100Q"), struct.Struct("=3Q")
+_NO_HIST = bytes(_HIST.size)
+
+
 class Config(C.Structure):
     _fields_ = [("device", C.c_int), ("s_hi_max", C.c_uint64), ("cap_reps", C.c_uint32),
                 ("cap_divs", C.c_uint32), ("cap_ext", C.c_uint32), ("flags", C.c_uint32),
@@ -73,11 +79,11 @@ class Stats(C.Structure):
         ("max_extensions", C.c_uint64)]
 
     def as_dict(self) -> dict:
-        d = {n: int(getattr(self, n)) for n in COUNTER_NAMES}
-        d["hist5"] = {i: int(v) for i, v in enumerate(self.hist5) if v}
-        d["max_reps"] = int(self.max_reps)
-        d["max_divisors"] = int(self.max_divisors)
-        d["max_extensions"] = int(self.max_extensions)
+        raw = bytes(self)
+        d = dict(zip(COUNTER_NAMES, _COUNTERS.unpack_from(raw)))
+        hist = raw[_COUNTERS.size:_COUNTERS.size + _HIST.size]
+        d["hist5"] = {} if hist == _NO_HIST else {i: v for i, v in enumerate(_HIST.unpack(hist)) if v}
+        d["max_reps"], d["max_divisors"], d["max_extensions"] = _MAXIMA.unpack_from(raw, _COUNTERS.size + _HIST.size)
         return d
 
 

@@ -256,7 +256,7 @@ class Search:
 
     def _collect(self, out: RangeResult):
         r = self._res
-        buf = C.create_string_buffer(_LINE_CAP)
+        buf = C.create_string_buffer(_LINE_CAP) if r.n_sixes or (self.dump4 and r.n_quads) else None
         if r.n_hits:
             # every hit's lines in one call (ps4_format_hits), grown once if the estimate is short
             # (the text buffer is kept between calls and only the bytes written are copied out)
