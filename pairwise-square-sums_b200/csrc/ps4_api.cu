@@ -41,8 +41,11 @@ struct ps4_ctx {
     // one block holds the status and the items' counters, so that both are cleared and copied back at
     // once; a call of few items has its segments behind them, and clears and uploads in one copy
     unsigned char *d_block = nullptr; uint64_t block_cap = 0;
-    unsigned char *h_block = nullptr; uint64_t h_block_cap = 0;      // pinned: where the block lands
-    unsigned char *h_stage = nullptr; uint64_t h_stage_cap = 0;      // pinned: zeros and segments to upload
+    unsigned char *h_block = nullptr;    // pinned: where the block lands
+    unsigned char *h_stage = nullptr;    // pinned: zeros and segments to upload
+    unsigned char *h_pin = nullptr;      // one pinned allocation, in whose halves both lie while they fit
+    unsigned char *h_big_block = nullptr; uint64_t h_big_block_cap = 0;
+    unsigned char *h_big_stage = nullptr; uint64_t h_big_stage_cap = 0;
     Status *d_status = nullptr;
     unsigned long long *d_counters = nullptr;
     ps4_hit *d_hits = nullptr; uint32_t hits_cap = 0;
@@ -92,7 +95,6 @@ struct ps4_ctx {
     // triple extension (grown on demand): the members in; counters, states and records out in one block
     uint64_t *d_tri_in = nullptr; uint64_t tri_in_cap = 0;
     unsigned char *d_tri = nullptr; uint64_t tri_cap = 0;
-    unsigned char *h_tri = nullptr; uint64_t h_tri_cap = 0;          // pinned
     uint64_t tri_out_cap = 0;                                        // records the device block holds
     std::string err;
 };
@@ -150,12 +152,24 @@ static int grow_pinned(ps4_ctx *c, T *&ptr, uint64_t &cap, uint64_t need) {
 static const size_t BLOCK_HEAD = (sizeof(Status) + 255) & ~(size_t)255;
 static size_t block_bytes(uint64_t n_items) { return BLOCK_HEAD + (size_t)n_items * K_SLOTS * sizeof(unsigned long long); }
 static const uint32_t SMALL_ITEMS = 16, SMALL_SEGS = 64;             // uploaded together with their zeros
+static const size_t PIN_HALF = 32768;
 static int reserve_block(ps4_ctx *c, uint32_t n_items) {
     if (grow(c, c->d_block, c->block_cap, std::max<uint64_t>(c->block_cap, block_bytes(n_items) + SMALL_SEGS * sizeof(Item))))
         return PS4_ERR_CUDA;
     c->d_status = reinterpret_cast<Status *>(c->d_block);
     c->d_counters = reinterpret_cast<unsigned long long *>(c->d_block + BLOCK_HEAD);
-    return grow_pinned(c, c->h_block, c->h_block_cap, block_bytes(n_items));
+    c->h_block = c->h_pin + PIN_HALF;
+    if (block_bytes(n_items) <= PIN_HALF) return 0;
+    if (grow_pinned(c, c->h_big_block, c->h_big_block_cap, block_bytes(n_items))) return PS4_ERR_CUDA;
+    c->h_block = c->h_big_block;
+    return 0;
+}
+static int reserve_stage(ps4_ctx *c, size_t bytes) {
+    c->h_stage = c->h_pin;
+    if (bytes <= PIN_HALF) return 0;
+    if (grow_pinned(c, c->h_big_stage, c->h_big_stage_cap, bytes)) return PS4_ERR_CUDA;
+    c->h_stage = c->h_big_stage;
+    return 0;
 }
 
 static uint64_t isqrt_host(uint64_t n) {
@@ -180,9 +194,9 @@ extern "C" void ps4_destroy(ps4_ctx *c) {
     cudaFree(c->d_scratch); cudaFree(c->d_jobs); cudaFree(c->d_raw); cudaFree(c->d_seq);
     cudaFree(c->d_fac);
     cudaFree(c->d_tri_in); cudaFree(c->d_tri);
-    if (c->h_block) cudaFreeHost(c->h_block);
-    if (c->h_stage) cudaFreeHost(c->h_stage);
-    if (c->h_tri) cudaFreeHost(c->h_tri);
+    if (c->h_pin) cudaFreeHost(c->h_pin);
+    if (c->h_big_block) cudaFreeHost(c->h_big_block);
+    if (c->h_big_stage) cudaFreeHost(c->h_big_stage);
     if (c->h_hits) cudaFreeHost(c->h_hits);
     if (c->h_exts) cudaFreeHost(c->h_exts);
     if (c->h_sixes) cudaFreeHost(c->h_sixes);
@@ -237,6 +251,7 @@ extern "C" int ps4_create(const ps4_config *cfg, ps4_ctx **out) {
     c->tab_n = 2 * isqrt_host(c->cfg.s_hi_max) + 64;      // s4.c:440
     CUDA_TRY(c, cudaMalloc((void **)&c->d_spfq, c->tab_n * sizeof(uint64_t)));
     CUDA_TRY(c, cudaMalloc((void **)&c->d_ndiv, c->tab_n * sizeof(uint16_t)));
+    CUDA_TRY(c, cudaMallocHost((void **)&c->h_pin, 2 * PIN_HALF));
     CUDA_TRY(c, (cudaError_t)launch_tables(c->d_spfq, c->d_ndiv, c->tab_n, c->stream));
     CUDA_TRY(c, cudaMalloc((void **)&c->d_fac, fac_n(c->tab_n) * sizeof(uint4)));
     CUDA_TRY(c, (cudaError_t)launch_fac(c->d_fac, fac_n(c->tab_n), c->stream));
@@ -442,7 +457,7 @@ static int enqueue_items(ps4_ctx *c) {
     // a call of few items uploads its zeros and segments in one copy, to one place
     const bool small = n_items <= SMALL_ITEMS && segs.size() <= SMALL_SEGS;
     const size_t blk = block_bytes(n_items), segs_bytes = segs.size() * sizeof(Item);
-    if (grow_pinned(c, c->h_stage, c->h_stage_cap, (small ? blk : 0) + segs_bytes)) return PS4_ERR_CUDA;
+    if (reserve_stage(c, (small ? blk : 0) + segs_bytes)) return PS4_ERR_CUDA;
     Item *const dev_items = small ? reinterpret_cast<Item *>(c->d_block + blk) : c->d_items;
     if (kernel == PS4_KERNEL_BATCHED && c->d_jobs_words < 6 * c->jobs_cap)
         if (grow(c, c->d_jobs, c->d_jobs_words, 6 * c->jobs_cap)) return PS4_ERR_CUDA;
@@ -996,29 +1011,31 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
     if (n == 0) return PS4_OK;
     if (!abc) return set_err(c, PS4_ERR_ARG, "ps4_extend_triples: no input");
     if (dmax > (1ull << 62)) return set_err(c, PS4_ERR_ARG, "dmax %llu exceeds 2^62", (unsigned long long)dmax);
-    // device block: counters n_out, n_cand, n_sqrt (32 bytes), a state per triple, the records
-    const uint64_t off_out = (32 + (uint64_t)n + 15) & ~15ull;
-    const uint64_t FIRST = 1024;                      // records copied back with the states
+    // device block: counters n_out, n_cand, n_sqrt (32 bytes), the records, a state per triple
+    const uint64_t FIRST = 1024;                      // records copied back with the counters
+    static_assert(32 + FIRST * sizeof(ps4_tri_ext) <= PIN_HALF, "they land in the pinned buffer");
     if (grow(c, c->d_tri_in, c->tri_in_cap, std::max<uint64_t>(c->tri_in_cap, 3 * (uint64_t)n))) return PS4_ERR_CUDA;
     c->tri_out_cap = std::max<uint64_t>(c->tri_out_cap, std::max<uint64_t>(out_cap, 1u << 16));
     auto reserve = [&]() {
-        return grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, off_out + c->tri_out_cap * sizeof(ps4_tri_ext)));
+        return grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, 32 + c->tri_out_cap * sizeof(ps4_tri_ext) + n));
     };
     if (reserve()) return PS4_ERR_CUDA;
-    if (grow_pinned(c, c->h_tri, c->h_tri_cap, off_out + FIRST * sizeof(ps4_tri_ext))) return PS4_ERR_CUDA;
     const uint64_t in_bytes = 3 * (uint64_t)n * sizeof(uint64_t);
     CUDA_TRY(c, cudaMemcpyAsync(c->d_tri_in, abc, in_bytes, cudaMemcpyHostToDevice, c->stream));
     c->h2d_bytes += in_bytes;
-    const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(c->h_tri);
-    uint64_t first = 0;
+    unsigned char *const land = c->h_pin + PIN_HALF;
+    const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(land);
+    const bool few = 32 + FIRST * sizeof(ps4_tri_ext) + n <= PIN_HALF;         // the states land there too
+    std::vector<uint8_t> st_buf(few ? 0 : n);
+    const uint8_t *st = few ? land + 32 + FIRST * sizeof(ps4_tri_ext) : st_buf.data();
     for (int attempt = 0; attempt < 2; attempt++) {
         unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(c->d_tri);
         CUDA_TRY(c, cudaMemsetAsync(d_cnt, 0, 32, c->stream));
         TriArgs t;
         t.abc = c->d_tri_in; t.n = n; t.dmax = dmax;
-        t.spfq = c->d_spfq; t.ndiv = c->d_ndiv; t.tab_n = c->tab_n;
-        t.state = c->d_tri + 32;
-        t.out = reinterpret_cast<ps4_tri_ext *>(c->d_tri + off_out); t.out_cap = c->tri_out_cap;
+        t.spfq = c->d_spfq; t.ndiv = c->d_ndiv; t.fac = c->d_fac; t.tab_n = c->tab_n;
+        t.out = reinterpret_cast<ps4_tri_ext *>(c->d_tri + 32); t.out_cap = c->tri_out_cap;
+        t.state = c->d_tri + 32 + c->tri_out_cap * sizeof(ps4_tri_ext);
         t.n_out = d_cnt; t.n_cand = d_cnt + 1; t.n_sqrt = d_cnt + 2;
         t.item_base = 0;
         t.cand_per = t.sqrt_per = nullptr;
@@ -1026,11 +1043,11 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
         CUDA_TRY(c, (cudaError_t)launch_triples(t, c->stream));
         CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
         c->last_launches++;
-        first = std::min<uint64_t>(FIRST, c->tri_out_cap);
-        CUDA_TRY(c, cudaMemcpyAsync(c->h_tri, c->d_tri, off_out + first * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost,
-                                    c->stream));
+        const uint64_t head = 32 + std::min<uint64_t>(FIRST, c->tri_out_cap) * sizeof(ps4_tri_ext);
+        CUDA_TRY(c, cudaMemcpyAsync(land, c->d_tri, head, cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(c, cudaMemcpyAsync(const_cast<uint8_t *>(st), t.state, n, cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        c->d2h_bytes += off_out + first * sizeof(ps4_tri_ext);
+        c->d2h_bytes += head + n;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev0, c->ev1);
         c->last_ms = ms;
@@ -1040,12 +1057,11 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
         c->tri_out_cap = cnt[0] * 3 / 2 + 1024;
         if (reserve()) return PS4_ERR_CUDA;
     }
-    const uint8_t *st = c->h_tri + 32;
-    const uint64_t n_rec = cnt[0];
+    const uint64_t n_rec = cnt[0], first = std::min<uint64_t>(n_rec, FIRST);
     std::vector<ps4_tri_ext> recs(n_rec);
-    if (n_rec) memcpy(recs.data(), c->h_tri + off_out, std::min(n_rec, first) * sizeof(ps4_tri_ext));
+    if (first) memcpy(recs.data(), land + 32, first * sizeof(ps4_tri_ext));
     if (n_rec > first) {
-        CUDA_TRY(c, cudaMemcpyAsync(recs.data() + first, c->d_tri + off_out + first * sizeof(ps4_tri_ext),
+        CUDA_TRY(c, cudaMemcpyAsync(recs.data() + first, c->d_tri + 32 + first * sizeof(ps4_tri_ext),
                                     (n_rec - first) * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         c->d2h_bytes += (n_rec - first) * sizeof(ps4_tri_ext);

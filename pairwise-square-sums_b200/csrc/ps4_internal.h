@@ -121,6 +121,7 @@ struct TriArgs {
     uint64_t dmax;             // extensions d <= dmax
     const uint64_t *spfq;
     const uint16_t *ndiv;
+    const uint4 *fac;
     uint64_t tab_n;
     uint8_t *state;            // per triple: TRI_OK / TRI_INVALID / TRI_RANGE
     ps4_tri_ext *out;

@@ -560,7 +560,7 @@ int launch_step(ps4_server *s, StepBuf &b) {
         TriArgs t;
         memset(&t, 0, sizeof t);
         t.abc = b.d_abc; t.n = n_tri; t.dmax = 0;
-        t.spfq = s->v.spfq; t.ndiv = s->v.ndiv; t.tab_n = s->v.tab_n;
+        t.spfq = s->v.spfq; t.ndiv = s->v.ndiv; t.fac = s->v.fac; t.tab_n = s->v.tab_n;
         t.state = b.d_tri_state;
         t.out = b.d_tri_out; t.out_cap = b.tri_out_cap;
         t.n_out = b.d_tri_cnt; t.n_cand = b.d_tri_cnt + 1; t.n_sqrt = b.d_tri_cnt + 2;

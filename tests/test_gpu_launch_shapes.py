@@ -10,7 +10,7 @@ import pytest
 
 from conftest import COUNTERS, assert_stats_equal
 from oracle import orc
-from ps4b200 import Search
+from ps4b200 import Search, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +62,27 @@ def test_list_lengths_vs_oracle(wide, k):
         assert ost["max_reps"] in (k, k + 1)          # one more for twice a square
         assert sorted(r.lines) == sorted(olines)
         assert_stats_equal(r.stats, ost)
+
+
+@pytest.mark.parametrize("S0", [4205, 5785, 6205])
+def test_differences_with_a_large_square_vs_oracle(wide, S0):
+    """4-sets that are 49999^2 times a small one: both factors of their differences share a large prime,
+    so that divisor lists would leave 32 bits and the per-lane divisor walk takes over."""
+    S = S0 * 49999 ** 2
+    r = wide.range(S, S + 1)
+    rc, ost, olines, err = orc.search(S, S + 1)
+    assert rc == 0 and ost["sets4"] > 0, err
+    assert sorted(r.lines) == sorted(olines)
+    assert_stats_equal(r.stats, ost)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 4736, 4737, 9473])
+@pytest.mark.parametrize("scale", [1, 65537 ** 2])
+def test_triple_counts_and_scales_vs_oracle(wide, n, scale):
+    """One triple per warp up to a full device, then several; scaled ones share a large prime (as above)."""
+    abc = workloads.triples(n, seed=n, xmax=40 if scale > 1 else 2000) * scale
+    got, state, st = wide.extend_triples(abc, 10 ** 15)
+    assert not state.any() and st["triples"] == n
+    check = range(n) if n < 100 else range(0, n, 97)
+    for i in check:
+        assert got[i] == orc.extend_triple(*(int(v) for v in abc[i]), 10 ** 15), i
