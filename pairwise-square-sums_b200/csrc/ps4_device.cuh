@@ -385,19 +385,9 @@ __device__ __forceinline__ uint32_t isqrt_lt2p46(uint64_t x) {
     return r;
 }
 
-// p = ceil(sqrt(m)) for 0 < m < 2^44, and over = p^2 - m.  The estimate's relative error is below
-// 2^-23 (sqrt.approx) + 2^-25 (half the conversion's), so for a root below 2^22 it is off by less than
-// 0.7 and its floor by at most one either way: one exact correction step, without branches.
-__device__ __forceinline__ uint32_t ceil_sqrt_lt2p44(uint64_t m, uint32_t &over) {
-    float f;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"((float)m));
-    uint32_t r = (uint32_t)f;
-    int32_t d = (int32_t)(m - (uint64_t)r * r);            // |d| < 2^24: the difference's low word
-    if (d < 0) { r--; d += 2 * (int32_t)r + 1; }           // floor(root) or one below it from here on
-    if (d > 2 * (int32_t)r) { d -= 2 * (int32_t)r + 1; r++; }
-    over = d > 0 ? 2 * r + 1 - (uint32_t)d : 0u;
-    return d > 0 ? r + 1 : r;
-}
+// a counter of a selected S holds, from P2 on, this bit and the next place in its list; the others
+// keep their counts (below 2^15)
+constexpr uint32_t SELECTED = 0x8000u;
 
 // P1 / P3: scan every representation S = p^2 + q^2, 1 <= p <= q, S in [S0, S0+n).
 // q-major: q runs over [ceil(sqrt(S0/2)), isqrt(S1-2)] (strided over the threads), p from
@@ -424,9 +414,8 @@ __device__ __forceinline__ uint32_t scan_reps(uint64_t S0, uint32_t n, uint32_t 
                 atomicAdd(&cnt32[w], 1u << sh);
                 found++;
             } else {
-                const uint32_t cur = (((volatile uint32_t *)cnt32)[w] >> sh) & 0xFFFFu;
-                if (cur == 0xFFFFu) continue;          // S not selected
-                const uint32_t pos = (atomicAdd(&cnt32[w], 1u << sh) >> sh) & 0xFFFFu;
+                if (!(((volatile uint32_t *)cnt32)[w] >> sh & SELECTED)) continue;
+                const uint32_t pos = (atomicAdd(&cnt32[w], 1u << sh) >> sh) & (SELECTED - 1);
                 rep_p[pos] = p;
                 rep_q[pos] = q;
             }
@@ -436,64 +425,99 @@ __device__ __forceinline__ uint32_t scan_reps(uint64_t S0, uint32_t n, uint32_t 
 }
 
 constexpr uint32_t SCAN_RUN = 24;      // a q with more p than this is walked by a whole warp
+constexpr int SCAN_ILP = 4;            // q per lane and turn: their roots are independent chains
 
 // The scan of scan_reps over a group of adjacent tiles [SS0, SS1) of one segment, done once by
 // `parts` CTAs together (this one takes every parts-th q, from `part`): every representation goes
 // to its tile's list (offset in the tile | p << 14 | q << 36; p <= q < 2^22, offset < 2^14), each CTA
 // into its own part of the list, `cap` entries long, counted in cnt[tile] (one shared-memory atomic
-// per representation).  A count above cap means the part overflowed; that tile then scans for itself.
+// per representation, or per tile that a warp's turn of a long run meets).  A count above cap means the
+// part overflowed; that tile then scans for itself.
+//
+// First p of a q: p = ceil(sqrt(m)), m = SS0 - q^2.  With qt = floor(sqrt(SS0)) and k = qt - q, m = (SS0 - qt^2) +
+// k (2 qt - k): k, 2 qt - k and SS0 - qt^2 <= 2 qt are below 2^24, exact in single precision, so one fused
+// multiply-add gives m to half a unit (2^-24 relative) and sqrt.approx (2^-23) the root, below 2^22, to
+// 2/3: its floor is off by one at most, and the difference m - r^2, below 2^24, comes from 32-bit products.
+// (A 64-bit conversion and 64-bit products per q: 680 cycles a turn of one q on a narrow call.)
 template <int NT>
 __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned TLv, uint64_t *lists, uint32_t cap,
                                            uint32_t *cnt, uint32_t part, uint32_t parts) {
     uint32_t qmin = (uint32_t)ceil_sqrt64((SS0 + 1) >> 1);
     if (qmin < 1) qmin = 1;
-    const uint32_t qmax = SS1 >= 2 ? (uint32_t)isqrt64(SS1 - 2) : 0;
-    const uint32_t width = (uint32_t)(SS1 - SS0), wmask = (1u << TLv) - 1u;
+    const uint32_t qmax = SS1 >= 2 ? (uint32_t)isqrt64(SS1 - 2) : 0, qt = (uint32_t)isqrt64(SS0);
+    const uint32_t width = (uint32_t)(SS1 - SS0), wmask = (1u << TLv) - 1u, lo0 = (uint32_t)SS0;
+    const float ft = (float)(uint32_t)(SS0 - (uint64_t)qt * qt);
     // long runs need 2 * SCAN_RUN * p < width, so p < pc and q^2 >= SS0 - pc^2: below qc there are none
     const uint64_t pc = width / (2 * SCAN_RUN);
     const uint32_t qc = pc * pc < SS0 ? (uint32_t)isqrt64(SS0 - pc * pc) : 0u;
     const int lane = threadIdx.x & 31;
     lists += (size_t)part * cap;
-    auto put = [&](uint32_t q, uint32_t p, uint32_t i) {                 // S = SS0 + i
-        const uint32_t j = i >> TLv;
-        const uint32_t pos = atomicAdd(&cnt[j], 1u);
+    auto store = [&](uint32_t q, uint32_t p, uint32_t i, uint32_t j, uint32_t pos) {    // S = SS0 + i, in tile j
         if (pos < cap)
             lists[(size_t)(j * parts) * cap + pos] = (uint64_t)(i & wmask) | ((uint64_t)p << 14) | ((uint64_t)q << 36);
     };
-    for (uint32_t qw = qmin + part + parts * (threadIdx.x - lane); qw <= qmax; qw += parts * NT) {   // warp-uniform
-        const uint32_t q = qw + parts * lane;
-        const uint64_t q2 = (uint64_t)q * q;
-        uint32_t p = 1, i = 0;                             // i = p^2 + q^2 - SS0, below width where it counts
-        bool live = q <= qmax;
-        if (SS0 > q2 + 1) {
-            p = ceil_sqrt_lt2p44(SS0 - q2, i);
-        } else {
-            live = live && q2 + 1 - SS0 < width;
-            i = (uint32_t)(q2 + 1 - SS0);
+    for (uint32_t qw = qmin + part + parts * (threadIdx.x - lane); qw <= qmax; qw += parts * NT * SCAN_ILP) {  // warp-uniform
+        uint32_t p[SCAN_ILP], i[SCAN_ILP];                 // i = p^2 + q^2 - SS0, below width where it counts
+#pragma unroll
+        for (int u = 0; u < SCAN_ILP; u++) {
+            const uint32_t q = qw + parts * (lane + NT * u), k = qt - q;
+            float f;
+            asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"(fmaf((float)k, (float)(qt + q), ft)));
+            uint32_t r = (uint32_t)f;
+            int32_t d = (int32_t)(lo0 - q * q - r * r);    // m - r^2, where q <= qt
+            if (d < 0) { r--; d += 2 * (int32_t)r + 1; }   // floor(root) or one below it from here on
+            if (d > 2 * (int32_t)r) { d -= 2 * (int32_t)r + 1; r++; }
+            p[u] = d > 0 ? r + 1 : r;
+            i[u] = d > 0 ? 2 * r + 1 - (uint32_t)d : 0u;
+            const bool top = q > qt || p[u] == 0;          // q^2 >= SS0: p from 1
+            if (top) {
+                p[u] = 1;
+                i[u] = q * q + 1 - lo0;                    // below 2^32 where q <= qmax: q^2 + 1 < SS1
+            }
+            if (q > qmax || p[u] > q) i[u] = 0xFFFFFFFFu;
         }
-        live = live && p <= q && i < width;
-        // a q with a long run of p (the top of the q range: p small against the width) is walked
-        // by the whole warp, the others by their lanes
-        if (qw + 31 * parts >= qc) {                       // warp-uniform
-            unsigned coop = __ballot_sync(0xffffffffu, live && i + SCAN_RUN * (2 * p + SCAN_RUN) < width);
-            if (coop >> lane & 1u) live = false;
-            while (coop) {
-                const int o = __ffs((int)coop) - 1;
-                coop &= coop - 1;
-                const uint32_t cq = __shfl_sync(0xffffffffu, q, o), p0 = __shfl_sync(0xffffffffu, p, o);
-                const uint32_t i0 = __shfl_sync(0xffffffffu, i, o);
-                // p^2 - p0^2 = (p - p0)(p + p0); p < p0 + 32 + width / (2 p0), within 32 bits by width < 2^21
-                for (uint32_t k = lane;; k += 32) {
-                    const uint64_t ck = (uint64_t)k * (k + 2 * p0) + i0;
-                    if (p0 + k > cq || ck >= width) break;
-                    put(cq, p0 + k, (uint32_t)ck);
+#pragma unroll
+        for (int u = 0; u < SCAN_ILP; u++) {
+            const uint32_t q = qw + parts * (lane + NT * u);
+            bool live = i[u] < width;
+            // a q with a long run of p (the top of the q range: p small against the width) is walked
+            // by the whole warp, the others by their lanes
+            if (qw + parts * (31 + NT * u) >= qc) {        // warp-uniform
+                unsigned coop = __ballot_sync(0xffffffffu, live && i[u] + SCAN_RUN * (2 * p[u] + SCAN_RUN) < width);
+                if (coop >> lane & 1u) live = false;
+                while (coop) {
+                    const int o = __ffs((int)coop) - 1;
+                    coop &= coop - 1;
+                    const uint32_t cq = __shfl_sync(0xffffffffu, q, o), p0 = __shfl_sync(0xffffffffu, p[u], o);
+                    const uint32_t i0 = __shfl_sync(0xffffffffu, i[u], o);
+                    // p^2 - p0^2 = (p - p0)(p + p0), ascending over the lanes: lanes of one tile are
+                    // neighbours, and its first lane counts them all
+                    for (uint32_t k0 = 0;; k0 += 32) {
+                        const uint32_t k = k0 + lane;
+                        const uint64_t ck = (uint64_t)k * (k + 2 * p0) + i0;
+                        const bool in = p0 + k <= cq && ck < width;
+                        const uint32_t j = in ? (uint32_t)ck >> TLv : 0xFFFFFFFFu;
+                        const uint32_t before = __shfl_up_sync(0xffffffffu, j, 1);
+                        const unsigned heads = __ballot_sync(0xffffffffu, in && (lane == 0 || before != j));
+                        const unsigned all = __ballot_sync(0xffffffffu, in);
+                        if (!all) break;
+                        const int head = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));     // of this lane's tile
+                        const unsigned after = heads & ~(0xFFFFFFFFu >> (31 - lane));
+                        uint32_t pos = 0;
+                        if (in && head == lane)
+                            pos = atomicAdd(&cnt[j], (uint32_t)((after ? __ffs((int)after) - 1 : __popc(all)) - lane));
+                        pos = __shfl_sync(0xffffffffu, pos, head & 31) + (uint32_t)(lane - head);
+                        if (in) store(cq, p0 + k, (uint32_t)ck, j, pos);
+                        if (all != 0xFFFFFFFFu) break;
+                    }
                 }
             }
-        }
-        for (; live; live = p <= q && i < width) {
-            put(q, p, i);
-            i += 2 * p + 1;
-            p++;
+            for (uint32_t pu = p[u], iu = i[u]; live; live = pu <= q && iu < width) {
+                const uint32_t j = iu >> TLv;
+                store(q, pu, iu, j, atomicAdd(&cnt[j], 1u));
+                iu += 2 * pu + 1;
+                pu++;
+            }
         }
     }
 }
@@ -646,6 +670,23 @@ __device__ __forceinline__ void sort_lists(unsigned char *smem, uint32_t n_is) {
     }
 }
 
+// f(entry) for every entry of a tile's list; four loads in flight per thread (they come from L2)
+template <int NT, class F>
+__device__ __forceinline__ void for_entries(const uint64_t *list, const uint32_t *list_n, uint32_t parts, uint32_t cap,
+                                            F f) {
+    for (uint32_t w = 0; w < parts; w++, list += cap) {
+        const uint32_t n = list_n[w];
+        for (uint32_t o = threadIdx.x; o < n; o += 4 * NT) {
+            uint64_t e[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) e[u] = o + u * NT < n ? __ldcg(list + o + u * NT) : 0;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (o + u * NT < n) f(e[u]);
+        }
+    }
+}
+
 // P1-P4 for one tile.  Returns false if the tile was abandoned (error raised).  With `list` (the
 // tile's representations from scan_group, list_n[w] entries in part w of `parts`, `cap` apart; other
 // CTAs of the cluster may have written them: read through L2) P1 and P3 read the list; without,
@@ -669,14 +710,11 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
     // P1: count, from the list or by scanning
     uint32_t found = 0;
     if (list) {
-        for (uint32_t w = 0; w < parts; w++) {
-            const uint32_t cw = list_n[w];
-            for (uint32_t o = tid; o < cw; o += NT) {
-                const uint32_t i = (uint32_t)__ldcg(list + (size_t)w * cap + o) & 0x3FFFu;
-                atomicAdd(&cnt32[i >> 1], 1u << ((i & 1) * 16));
-                found++;
-            }
-        }
+        for_entries<NT>(list, list_n, parts, cap, [&](uint64_t e) {
+            const uint32_t i = (uint32_t)e & 0x3FFFu;
+            atomicAdd(&cnt32[i >> 1], 1u << ((i & 1) * 16));
+            found++;
+        });
     } else {
         found = scan_reps<false, NT>(S0, n, cnt32, rep_p, rep_q);
     }
@@ -686,30 +724,33 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
 
     // P2: select S with >= 3 representations and S != 2 (mod 4).  A thread owns SEG consecutive
     // S, i.e. WT counter words, and visits them from a lane-dependent rotation so that the lanes
-    // of a warp touch 32 different banks (in plain order they would all hit the same two)
+    // of a warp touch 32 different banks (in plain order they would all hit the same two).  Two
+    // counters are compared at once (k + 0x7FFD has bit 15 iff k >= 3); the few selected ones (1 in 30) are
+    // then taken one by one.  (A test of every S in both passes: 17 % of the tile kernel.)
     constexpr uint32_t SEG = L::W / NT;
     constexpr uint32_t WT = SEG / 2;
-    static_assert(WT >= 1 && WT <= 32 && (WT & (WT - 1)) == 0, "counter words per thread: a power of two");
+    static_assert(WT >= 1 && WT <= 16 && (WT & (WT - 1)) == 0, "counter words per thread: a power of two, 32 S at most");
     const uint32_t i0 = tid * SEG, w0 = tid * WT;
     const uint32_t rot = (((uint32_t)tid & 31u) * WT / 32u) & (WT - 1);
-    uint32_t nI = 0, nR = 0, nP = 0, kmax = 0;
+    uint32_t nI = 0, nR = 0, nP = 0, sel = 0, kmax2 = 0;
     ull trip = 0;
     bool over = false;
+#pragma unroll
     for (uint32_t it = 0; it < WT; it++) {
         const uint32_t wi = (it + rot) & (WT - 1);
-        const uint32_t word = cnt32[w0 + wi];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint32_t i = i0 + 2 * wi + h;
-            const uint32_t k = (word >> (h * 16)) & 0xFFFFu;
-            if (i >= n) continue;
-            kmax = max(kmax, k);
-            if (k >= 3 && ((S0 + i) & 3) != 2) {
-                nI++; nR += k; nP += (k - 1) * (k - 2) / 2;      // pairs (x,y) with a z above y
-                trip += (ull)k * (k - 1) * (k - 2) / 6;
-                if (k > a.cap_reps) over = true;
-            }
-        }
+        const uint32_t word = cnt32[w0 + wi], t = (word + 0x7FFD7FFDu) & 0x80008000u;
+        kmax2 = __vmaxu2(kmax2, word);
+        sel |= ((t >> 15 | t >> 30) & 3u) << (2 * wi);
+    }
+    sel &= ~(0x11111111u << ((2u - (uint32_t)(S0 + i0)) & 3u));          // S = 2 mod 4
+    const uint32_t kmax = max(kmax2 & 0xFFFFu, kmax2 >> 16);
+    const uint16_t *cnt16 = (const uint16_t *)cnt32;
+    for (uint32_t m = sel; m; m &= m - 1) {
+        const uint32_t k = cnt16[i0 + (uint32_t)__ffs((int)m) - 1];
+        const uint32_t kp = (k - 1) * (k - 2) / 2;                       // pairs (x,y) with a z above y
+        nI++; nR += k; nP += kp;
+        trip += (ull)k * kp / 3u;
+        if (k > a.cap_reps) over = true;
     }
     if (over) raise_error(a.status, E_CAP_REPS, S0);
     uint32_t bI, bR, bP, tot[3];
@@ -735,42 +776,23 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
         ts.cnt[K_S_GE3] += tot[0];
         is_pbase[tot[0]] = tot[2];
     }
-    for (uint32_t it = 0; it < WT; it++) {
-        const uint32_t wi = (it + rot) & (WT - 1);
-        const uint32_t i = i0 + 2 * wi, cw = cnt32[w0 + wi];
-        uint32_t word = 0;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint32_t ii = i + h;
-            uint32_t val = 0xFFFFu;
-            if (ii < n) {
-                const uint32_t k = (cw >> (h * 16)) & 0xFFFFu;
-                if (k >= 3 && ((S0 + ii) & 3) != 2) {
-                    is_off[bI] = (uint16_t)ii; is_k[bI] = (uint16_t)k; is_start[bI] = (uint16_t)bR;
-                    is_pbase[bI] = bP;
-                    val = bR;
-                    bI++; bR += k; bP += (k - 1) * (k - 2) / 2;
-                }
-            }
-            word |= val << (h * 16);
-        }
-        cnt32[i >> 1] = word;
+    for (uint32_t m = sel; m; m &= m - 1) {
+        const uint32_t i = i0 + (uint32_t)__ffs((int)m) - 1, k = cnt16[i];
+        is_off[bI] = (uint16_t)i; is_k[bI] = (uint16_t)k; is_start[bI] = (uint16_t)bR;
+        is_pbase[bI] = bP;
+        ((uint16_t *)cnt32)[i] = (uint16_t)(SELECTED | bR);
+        bI++; bR += k; bP += (k - 1) * (k - 2) / 2;
     }
     __syncthreads();
     // P3: fill, from the list or by scanning again
     if (list) {
-        for (uint32_t w = 0; w < parts; w++) {
-            const uint32_t cw = list_n[w];
-            for (uint32_t o = tid; o < cw; o += NT) {
-                const uint64_t e = __ldcg(list + (size_t)w * cap + o);
-                const uint32_t i = (uint32_t)e & 0x3FFFu, wd = i >> 1, sh = (i & 1) * 16;
-                const uint32_t cur = (((volatile uint32_t *)cnt32)[wd] >> sh) & 0xFFFFu;
-                if (cur == 0xFFFFu) continue;          // S not selected
-                const uint32_t pos = (atomicAdd(&cnt32[wd], 1u << sh) >> sh) & 0xFFFFu;
-                rep_p[pos] = (uint32_t)(e >> 14) & 0x3FFFFFu;
-                rep_q[pos] = (uint32_t)(e >> 36);
-            }
-        }
+        for_entries<NT>(list, list_n, parts, cap, [&](uint64_t e) {
+            const uint32_t i = (uint32_t)e & 0x3FFFu, wd = i >> 1, sh = (i & 1) * 16;
+            if (!(((volatile uint32_t *)cnt32)[wd] >> sh & SELECTED)) return;
+            const uint32_t pos = (atomicAdd(&cnt32[wd], 1u << sh) >> sh) & (SELECTED - 1);
+            rep_p[pos] = (uint32_t)(e >> 14) & 0x3FFFFFu;
+            rep_q[pos] = (uint32_t)(e >> 36);
+        });
     } else {
         scan_reps<true, NT>(S0, n, cnt32, rep_p, rep_q);
     }
