@@ -286,7 +286,7 @@ __device__ inline void extend_quad(const SearchArgs &a, const uint32_t r[6], con
 // exclusive block scan of three u32 values over NT threads; returns totals in tot[3]
 template <int NT = BS>
 __device__ __forceinline__ void block_scan3(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t &e0, uint32_t &e1,
-                                            uint32_t &e2, uint32_t tot[3], uint32_t *wsum /* 3*NWARP; 3*NT/32 used */) {
+                                            uint32_t &e2, uint32_t tot[3], uint32_t *wsum /* 3*NT/32 */) {
     constexpr int NW = NT / 32;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t i0 = x0, i1 = x1, i2 = x2;
@@ -332,7 +332,7 @@ __device__ __forceinline__ uint32_t warp_max(uint32_t x) {
 
 struct TileShared {
     ull cnt[16];               // per-tile counters (K_* slots 0..12)
-    uint32_t wsum[3 * NWARP];
+    uint32_t wsum[3 * 32];     // block scans of up to 32 warps
     uint32_t n_is, n_rep, n_pairs, n_quads;
     uint32_t n_staged, flushed;    // 4-sets staged for extension / already extended in this tile
     uint32_t elist_n, work;
@@ -424,7 +424,7 @@ __device__ __forceinline__ uint32_t scan_reps(uint64_t S0, uint32_t n, uint32_t 
     return found;
 }
 
-constexpr uint32_t SCAN_RUN = 24;      // a q with more p than this is walked by a whole warp
+constexpr uint32_t SCAN_RUN = 24;       // a q with more p than this is walked by a whole warp
 constexpr int SCAN_ILP = 4;            // q per lane and turn: their roots are independent chains
 
 // The scan of scan_reps over a group of adjacent tiles [SS0, SS1) of one segment, done once by
@@ -456,11 +456,15 @@ __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned 
         if (pos < cap)
             lists[(size_t)(j * parts) * cap + pos] = (uint64_t)(i & wmask) | ((uint64_t)p << 14) | ((uint64_t)q << 36);
     };
-    for (uint32_t qw = qmin + part + parts * (threadIdx.x - lane); qw <= qmax; qw += parts * NT * SCAN_ILP) {  // warp-uniform
+    // Lanes of a warp take neighbouring q, whose runs are alike; a range that the CTAs pass in one turn
+    // goes round the warps instead, so that the long runs at its top are spread over them.
+    const bool spread = qmax - qmin < parts * NT * SCAN_ILP;
+    const uint32_t by_lane = parts * (spread ? NT / 32 : 1), by_warp = parts * (spread ? 1 : 32);
+    for (uint32_t qw = qmin + part + by_warp * (threadIdx.x >> 5); qw <= qmax; qw += parts * NT * SCAN_ILP) {  // warp-uniform
         uint32_t p[SCAN_ILP], i[SCAN_ILP];                 // i = p^2 + q^2 - SS0, below width where it counts
 #pragma unroll
         for (int u = 0; u < SCAN_ILP; u++) {
-            const uint32_t q = qw + parts * (lane + NT * u), k = qt - q;
+            const uint32_t q = qw + by_lane * lane + parts * NT * u, k = qt - q;
             float f;
             asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"(fmaf((float)k, (float)(qt + q), ft)));
             uint32_t r = (uint32_t)f;
@@ -478,11 +482,11 @@ __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned 
         }
 #pragma unroll
         for (int u = 0; u < SCAN_ILP; u++) {
-            const uint32_t q = qw + parts * (lane + NT * u);
+            const uint32_t q = qw + by_lane * lane + parts * NT * u;
             bool live = i[u] < width;
             // a q with a long run of p (the top of the q range: p small against the width) is walked
             // by the whole warp, the others by their lanes
-            if (qw + parts * (31 + NT * u) >= qc) {        // warp-uniform
+            if (qw + by_lane * 31 + parts * NT * u >= qc) {        // warp-uniform
                 unsigned coop = __ballot_sync(0xffffffffu, live && i[u] + SCAN_RUN * (2 * p[u] + SCAN_RUN) < width);
                 if (coop >> lane & 1u) live = false;
                 while (coop) {
@@ -512,11 +516,24 @@ __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned 
                     }
                 }
             }
-            for (uint32_t pu = p[u], iu = i[u]; live; live = pu <= q && iu < width) {
-                const uint32_t j = iu >> TLv;
-                store(q, pu, iu, j, atomicAdd(&cnt[j], 1u));
-                iu += 2 * pu + 1;
-                pu++;
+            if (!live) i[u] = 0xFFFFFFFFu;                 // nothing left to do
+        }
+        // the first entries of the lanes' q together (their places are independent), then the rest
+        uint32_t pos[SCAN_ILP];
+#pragma unroll
+        for (int u = 0; u < SCAN_ILP; u++)
+            pos[u] = i[u] < width ? atomicAdd(&cnt[i[u] >> TLv], 1u) : 0u;
+#pragma unroll
+        for (int u = 0; u < SCAN_ILP; u++) {
+            const uint32_t q = qw + by_lane * lane + parts * NT * u;
+            if (i[u] < width) {
+                store(q, p[u], i[u], i[u] >> TLv, pos[u]);
+                uint32_t iu = i[u] + 2 * p[u] + 1;
+                for (uint32_t pu = p[u] + 1; pu <= q && iu < width; pu++) {
+                    const uint32_t j = iu >> TLv;
+                    store(q, pu, iu, j, atomicAdd(&cnt[j], 1u));
+                    iu += 2 * pu + 1;
+                }
             }
         }
     }

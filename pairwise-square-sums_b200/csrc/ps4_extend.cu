@@ -455,7 +455,7 @@ __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned 
 // by one from a common counter.  A scan costs ~0.29 sqrt(S) steps however few S it covers, and a
 // narrow call has too few tiles for one CTA each on a scan of its own, so both ends gain from sharing it.
 template <int TL, int NT>
-__global__ void __launch_bounds__(NT, BS / NT * 2) gen_jobs(const __grid_constant__ SearchArgs a) {
+__global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const __grid_constant__ SearchArgs a) {
     using L = TileLayout<TL>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileShared ts;
@@ -1195,25 +1195,18 @@ __global__ void ring_init(uint32_t *seq, uint64_t n) {
 
 // ================================================================== launchers
 
-// the tile layout up to its extension-list area, which the tile kernel does not use
-template <int TL>
-static int setup_gen(size_t &smem) {
-    smem = TileLayout<TL>::OFF_ELIST;
-    return (int)cudaFuncSetAttribute(gen_jobs<TL, gen_threads(TL)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
-}
-
 // the tile kernel's full residency for 2^TL-S tiles
 int gen_grid(int num_sms, unsigned TL) { return num_sms * (BS / gen_threads(TL)) * 2; }
 int ext_grid(int num_sms) { return num_sms * 3; }
 
-template <int TL>
+template <int TL, int NT>
 static int launch_gen_tl(const SearchArgs &a, int grid, uint32_t cluster, cudaStream_t s) {
-    size_t smem;
-    if (const int e = setup_gen<TL>(smem)) return e;
+    const size_t smem = TileLayout<TL>::OFF_ELIST;       // up to the extension-list area, which it does not use
+    const int e = (int)cudaFuncSetAttribute(gen_jobs<TL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(gen_threads(TL));
+    cfg.blockDim = dim3(NT);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at;
@@ -1222,15 +1215,17 @@ static int launch_gen_tl(const SearchArgs &a, int grid, uint32_t cluster, cudaSt
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, gen_jobs<TL, gen_threads(TL)>, a);
+    return (int)cudaLaunchKernelEx(&cfg, gen_jobs<TL, NT>, a);
 }
 
+// up to this many tiles each has an SM to itself, and CTAs of 1024 threads
+constexpr uint64_t FEW_TILES = 128;
+
 // Launch shape of the tile kernel.  A group's scan visits 0.29 sqrt(S) q, as much work as s tiles
-// (68,000 q cost what a tile of 2^13 S does: 2.7 ps against 183 ns of the whole device at S = 1e12).
-//  * Cluster: 8 CTAs where scans weigh, i.e. for high S and for calls with few tiles, else 2 (a
-//    cluster of 8 costs 8 % in barriers and in CTAs that fit no GPC; of 2, nothing).  Measured, tile
-//    kernel with 8 / 2 / 1 CTAs: [1,1e10) 155.6 / 141.1 / 140.4 ms; 2e8 S at 1e12 4.95 / 6.27 / 8.32; 3e7 S
-//    at 1.2e13 2.81 / 5.71 / 9.75; 2e4 S at 4e11 0.079 / 0.140 / 0.220; 2e6 S at 1e9 0.103 / 0.109 / 0.129.
+// (34,000 q cost about what a tile of 2^13 S does).
+//  * Cluster: 8 CTAs where scans weigh, i.e. for high S and for calls with few tiles, else 2.  Measured,
+//    tile kernel with 8 / 2 / 1 CTAs: [1,1e10) 98.9 / 80.9 / 80.0 ms; 2e8 S at 1e12 2.79 / 3.05 / 3.82; 3e7 S at
+//    1.2e13 1.05 / 1.65 / 2.45; 64 subranges below 1e11 10.3 / 9.0 / 9.3; 2e4 S at 4e11 0.042 / 0.066 / 0.096.
 //  * Tiles per claim: n tiles in groups of G on K clusters take n + s n / G of work and about G K / 2 of
 //    idling at the end, least at G = sqrt(2 n s / K).
 // `grid`: the CTAs that the lists of a.raw are sized for; whole clusters of them are launched, no more
@@ -1238,21 +1233,24 @@ static int launch_gen_tl(const SearchArgs &a, int grid, uint32_t cluster, cudaSt
 int launch_gen(SearchArgs a, int grid, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const double n = (double)std::max<uint64_t>(a.n_tiles, 1);
-    const double scan = 0.29 * std::sqrt((double)a.s_top) / (68e3 * std::ldexp(1.0, (int)a.log2_tile - 13));
-    const uint32_t cl = n < 23e3 * scan || grid < 16 ? GEN_CLUSTER : 2;
+    const double scan = 0.29 * std::sqrt((double)a.s_top) / (34e3 * std::ldexp(1.0, (int)a.log2_tile - 13));
+    const uint32_t cl = n < 11e3 * scan || grid < 16 ? GEN_CLUSTER : 2;
     const uint64_t fit = std::max<uint64_t>((uint64_t)grid / cl, 1), want = ((uint64_t)n + cl - 1) / cl;
     const uint64_t K = std::min(fit, want), ctas = K * cl;
     const double G = std::min(std::sqrt(2 * n * scan / (double)K), std::ceil(n / (double)K));
     a.group = (uint32_t)std::min<double>(std::max<double>(G, cl), cl * SUPER_K);
     // a warp's reservations: a sixteenth of its expected share of about 0.2 4-sets per S, so that the
     // empty records at the end stay below a few percent, 128 at most (one atomic per 128 4-sets)
-    const double warps = (double)ctas * gen_threads(a.log2_tile) / 32;
+    const bool few = a.log2_tile == 12 && a.n_tiles <= FEW_TILES;
+    const double warps = (double)ctas * (few ? 1024 : gen_threads(a.log2_tile)) / 32;
     const double share = 0.2 * std::ldexp(n, (int)a.log2_tile) / warps;
     a.chunk = (uint32_t)std::min<double>(std::max<double>(share / 16, 8), 128);
     switch (a.log2_tile) {
-        case 12: return launch_gen_tl<12>(a, (int)ctas, cl, s);
-        case 13: return launch_gen_tl<13>(a, (int)ctas, cl, s);
-        default: return launch_gen_tl<14>(a, (int)ctas, cl, s);
+        case 12:
+            if (few) return launch_gen_tl<12, 1024>(a, (int)ctas, cl, s);
+            return launch_gen_tl<12, gen_threads(12)>(a, (int)ctas, cl, s);
+        case 13: return launch_gen_tl<13, gen_threads(13)>(a, (int)ctas, cl, s);
+        default: return launch_gen_tl<14, gen_threads(14)>(a, (int)ctas, cl, s);
     }
 }
 

@@ -31,9 +31,10 @@ def test_narrow_calls_vs_oracle(wide, lo, width):
     assert_stats_equal(r.stats, ost)
 
 
-# 592 tile CTAs: one tile of 2^13 S each and a little less or more; several groups per cluster
+# 128 tiles of 2^12 S (CTAs of 1024 threads up to there); 592 tile CTAs: one tile of 2^13 S each and a
+# little less or more; several groups per cluster
 @pytest.mark.parametrize("lo", [1, 10 ** 9, 10 ** 12])
-@pytest.mark.parametrize("width", [592 * 8192 - 1, 592 * 8192 + 1, 592 * 3 * 8192 + 4097])
+@pytest.mark.parametrize("width", [128 * 4096, 128 * 4096 + 1, 592 * 8192 - 1, 592 * 8192 + 1, 592 * 3 * 8192 + 4097])
 def test_shape_changes_vs_split_calls(wide, lo, width):
     one = wide.range(lo, lo + width)
     cut = lo + width // 3 + 1
