@@ -92,8 +92,7 @@ struct ps4_ctx {
     std::vector<cudaEvent_t> kev;
     size_t kev_used = 0;
     double gen_ms = 0.0, ext_ms = 0.0;
-    // triple extension (grown on demand): the members in; counters, states and records out in one block
-    uint64_t *d_tri_in = nullptr; uint64_t tri_in_cap = 0;
+    // triple extension (grown on demand): members, counters, states and records in one block
     unsigned char *d_tri = nullptr; uint64_t tri_cap = 0;
     uint64_t tri_out_cap = 0;                                        // records the device block holds
     std::string err;
@@ -193,7 +192,7 @@ extern "C" void ps4_destroy(ps4_ctx *c) {
     cudaFree(c->d_hits); cudaFree(c->d_exts); cudaFree(c->d_sixes); cudaFree(c->d_quads);
     cudaFree(c->d_scratch); cudaFree(c->d_jobs); cudaFree(c->d_raw); cudaFree(c->d_seq);
     cudaFree(c->d_fac);
-    cudaFree(c->d_tri_in); cudaFree(c->d_tri);
+    cudaFree(c->d_tri);
     if (c->h_pin) cudaFreeHost(c->h_pin);
     if (c->h_big_block) cudaFreeHost(c->h_big_block);
     if (c->h_big_stage) cudaFreeHost(c->h_big_stage);
@@ -471,7 +470,7 @@ static int enqueue_items(ps4_ctx *c) {
     const uint64_t raw_need = (uint64_t)g_gen * SUPER_K * raw_cap_for(TL);
     if (kernel == PS4_KERNEL_BATCHED && c->raw_words < raw_need)
         if (grow(c, c->d_raw, c->raw_words, raw_need)) return PS4_ERR_CUDA;
-    const int g_persist = c->num_sms * persist_ctas_per_sm();
+    const int g_persist = persist ? c->num_sms * persist_ctas_per_sm() : 0;
     const uint32_t raw_cap_persist = RAW_PER_TILE / 2;           // 2^13-S tiles: half the representations
     if (persist) {
         if (c->d_jobs_words < 6 * c->ring_cap && grow(c, c->d_jobs, c->d_jobs_words, 6 * c->ring_cap))
@@ -1011,31 +1010,40 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
     if (n == 0) return PS4_OK;
     if (!abc) return set_err(c, PS4_ERR_ARG, "ps4_extend_triples: no input");
     if (dmax > (1ull << 62)) return set_err(c, PS4_ERR_ARG, "dmax %llu exceeds 2^62", (unsigned long long)dmax);
-    // device block: counters n_out, n_cand, n_sqrt (32 bytes), the records, a state per triple
-    const uint64_t FIRST = 1024;                      // records copied back with the counters
-    static_assert(32 + FIRST * sizeof(ps4_tri_ext) <= PIN_HALF, "they land in the pinned buffer");
-    if (grow(c, c->d_tri_in, c->tri_in_cap, std::max<uint64_t>(c->tri_in_cap, 3 * (uint64_t)n))) return PS4_ERR_CUDA;
+    // One device block: the members, the counters n_out, n_cand, n_sqrt (32 bytes), a state per triple, the
+    // records.  A call of few triples uploads members and cleared counters in one copy, and gets
+    // counters, states and first records back in one.
+    const uint64_t FIRST = 256;                       // records copied back with the counters
+    const uint64_t in_bytes = 3 * (uint64_t)n * sizeof(uint64_t), off_cnt = (in_bytes + 31) & ~31ull, off_state = off_cnt + 32;
+    const uint64_t off_out = (off_state + n + 15) & ~15ull;
+    const uint64_t head = off_out - off_cnt + FIRST * sizeof(ps4_tri_ext);
+    const bool few = off_cnt + 32 <= PIN_HALF && head <= PIN_HALF;
     c->tri_out_cap = std::max<uint64_t>(c->tri_out_cap, std::max<uint64_t>(out_cap, 1u << 16));
     auto reserve = [&]() {
-        return grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, 32 + c->tri_out_cap * sizeof(ps4_tri_ext) + n));
+        return grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, off_out + c->tri_out_cap * sizeof(ps4_tri_ext)));
     };
-    if (reserve()) return PS4_ERR_CUDA;
-    const uint64_t in_bytes = 3 * (uint64_t)n * sizeof(uint64_t);
-    CUDA_TRY(c, cudaMemcpyAsync(c->d_tri_in, abc, in_bytes, cudaMemcpyHostToDevice, c->stream));
-    c->h2d_bytes += in_bytes;
     unsigned char *const land = c->h_pin + PIN_HALF;
-    const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(land);
-    const bool few = 32 + FIRST * sizeof(ps4_tri_ext) + n <= PIN_HALF;         // the states land there too
     std::vector<uint8_t> st_buf(few ? 0 : n);
-    const uint8_t *st = few ? land + 32 + FIRST * sizeof(ps4_tri_ext) : st_buf.data();
+    const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(land);
+    const ps4_tri_ext *first_recs = reinterpret_cast<const ps4_tri_ext *>(land + (few ? off_out - off_cnt : 32));
+    const uint8_t *st = few ? land + 32 : st_buf.data();
     for (int attempt = 0; attempt < 2; attempt++) {
-        unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(c->d_tri);
-        CUDA_TRY(c, cudaMemsetAsync(d_cnt, 0, 32, c->stream));
+        if (reserve()) return PS4_ERR_CUDA;
+        unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(c->d_tri + off_cnt);
+        if (few) {
+            memcpy(c->h_pin, abc, in_bytes);
+            memset(c->h_pin + in_bytes, 0, off_cnt + 32 - in_bytes);
+            CUDA_TRY(c, cudaMemcpyAsync(c->d_tri, c->h_pin, off_cnt + 32, cudaMemcpyHostToDevice, c->stream));
+        } else {
+            CUDA_TRY(c, cudaMemcpyAsync(c->d_tri, abc, in_bytes, cudaMemcpyHostToDevice, c->stream));
+            CUDA_TRY(c, cudaMemsetAsync(d_cnt, 0, 32, c->stream));
+        }
+        c->h2d_bytes += in_bytes;
         TriArgs t;
-        t.abc = c->d_tri_in; t.n = n; t.dmax = dmax;
+        t.abc = reinterpret_cast<const uint64_t *>(c->d_tri); t.n = n; t.dmax = dmax;
         t.spfq = c->d_spfq; t.ndiv = c->d_ndiv; t.fac = c->d_fac; t.tab_n = c->tab_n;
-        t.out = reinterpret_cast<ps4_tri_ext *>(c->d_tri + 32); t.out_cap = c->tri_out_cap;
-        t.state = c->d_tri + 32 + c->tri_out_cap * sizeof(ps4_tri_ext);
+        t.state = c->d_tri + off_state;
+        t.out = reinterpret_cast<ps4_tri_ext *>(c->d_tri + off_out); t.out_cap = c->tri_out_cap;
         t.n_out = d_cnt; t.n_cand = d_cnt + 1; t.n_sqrt = d_cnt + 2;
         t.item_base = 0;
         t.cand_per = t.sqrt_per = nullptr;
@@ -1043,11 +1051,15 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
         CUDA_TRY(c, (cudaError_t)launch_triples(t, c->stream));
         CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
         c->last_launches++;
-        const uint64_t head = 32 + std::min<uint64_t>(FIRST, c->tri_out_cap) * sizeof(ps4_tri_ext);
-        CUDA_TRY(c, cudaMemcpyAsync(land, c->d_tri, head, cudaMemcpyDeviceToHost, c->stream));
-        CUDA_TRY(c, cudaMemcpyAsync(const_cast<uint8_t *>(st), t.state, n, cudaMemcpyDeviceToHost, c->stream));
+        if (few) {
+            CUDA_TRY(c, cudaMemcpyAsync(land, d_cnt, head, cudaMemcpyDeviceToHost, c->stream));
+        } else {
+            CUDA_TRY(c, cudaMemcpyAsync(land, d_cnt, 32, cudaMemcpyDeviceToHost, c->stream));
+            CUDA_TRY(c, cudaMemcpyAsync(land + 32, t.out, FIRST * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost, c->stream));
+            CUDA_TRY(c, cudaMemcpyAsync(st_buf.data(), t.state, n, cudaMemcpyDeviceToHost, c->stream));
+        }
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        c->d2h_bytes += head + n;
+        c->d2h_bytes += 32 + n + FIRST * sizeof(ps4_tri_ext);
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev0, c->ev1);
         c->last_ms = ms;
@@ -1055,13 +1067,12 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
         // more records than the device buffer holds: grow it and run again (results do not
         // depend on the buffer)
         c->tri_out_cap = cnt[0] * 3 / 2 + 1024;
-        if (reserve()) return PS4_ERR_CUDA;
     }
     const uint64_t n_rec = cnt[0], first = std::min<uint64_t>(n_rec, FIRST);
     std::vector<ps4_tri_ext> recs(n_rec);
-    if (first) memcpy(recs.data(), land + 32, first * sizeof(ps4_tri_ext));
+    if (first) memcpy(recs.data(), first_recs, first * sizeof(ps4_tri_ext));
     if (n_rec > first) {
-        CUDA_TRY(c, cudaMemcpyAsync(recs.data() + first, c->d_tri + 32 + first * sizeof(ps4_tri_ext),
+        CUDA_TRY(c, cudaMemcpyAsync(recs.data() + first, c->d_tri + off_out + first * sizeof(ps4_tri_ext),
                                     (n_rec - first) * sizeof(ps4_tri_ext), cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         c->d2h_bytes += (n_rec - first) * sizeof(ps4_tri_ext);
