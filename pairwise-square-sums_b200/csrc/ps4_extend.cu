@@ -570,6 +570,7 @@ struct WarpArea {
     // the loop's own state, out of the registers between its claims (the same for all lanes)
     uint32_t njobs, quota, stretch;      // queue length; lanes that hold a 4-set; 4-sets per stretch
     uint32_t st_cur, st_rem, last;       // the stretch at hand; whether it is the last
+    uint32_t claimed;                    // 4-sets in the warps' first stretches
     uint32_t n_ext;
     uint8_t order[32];                   // lanes by row length, longest first
 };
@@ -909,15 +910,22 @@ __device__ __forceinline__ void process_queue(const SearchArgs &a, WarpArea *w, 
 // finished 4-set's slot is handed back after the round's report, and the loop ends when a claim finds
 // the ring empty and no lane holds a 4-set.  quota: lanes that hold a 4-set (32 unless the queue is too
 // short to fill every warp of the launch; the candidates of few 4-sets are still walked by all
-// lanes).  Returns whether the warp took any 4-set.
+// lanes).  The first `claimed` stretches belong to the warps in order, this one is number `first`.  Returns
+// whether the warp took any 4-set.
 template <bool RING>
 __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint32_t njobs, uint32_t quota,
-                                            uint32_t stretch) {
+                                            uint32_t stretch, uint32_t first, uint32_t claimed) {
     const unsigned FULL = 0xffffffffu;
     if (lane == 0) {
         w->n_ext = 0;
         w->njobs = njobs; w->quota = quota; w->stretch = stretch;
-        w->st_cur = w->st_rem = w->last = 0;
+        // the warp's first stretch is its own place in the grid (a short queue needs no atomics, whose turns
+        // on one address took 12 of a small call's 29 us), the later ones are claimed behind them
+        const uint32_t at = min(first * stretch, njobs);
+        w->st_cur = at;
+        w->st_rem = RING ? 0 : min(stretch, njobs - at);
+        w->last = (uint64_t)claimed * stretch >= njobs;
+        w->claimed = claimed * stretch;
     }
     if (lane < ICACHE) w->ic[lane].item = NO_ITEM;
     __syncwarp();
@@ -958,7 +966,7 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
                 uint32_t nx = 0, avail = 0;
                 if (rem < n && !last) {                                  // a new stretch behind the old one
                     if (lane == 0) {
-                        nx = atomicAdd(&a.status->ext_next, size);
+                        nx = w->claimed + atomicAdd(&a.status->ext_next, size);
                         stop = *(volatile ull *)&a.status->err != 0ull;
                     }
                     nx = __shfl_sync(FULL, nx, 0);
@@ -1088,7 +1096,7 @@ __global__ void __launch_bounds__(EBS, 3) extend_jobs(const __grid_constant__ Se
     const uint32_t quota = min((njobs + warps - 1) / warps, 32u);                // 1 at least
     // a stretch is a 32nd of a warp's share, 32 to 256 4-sets (one atomic each)
     const uint32_t stretch = quota < 32 ? quota : 32u * min(max(njobs / (warps * 1024), 1u), 8u);
-    engine_loop<false>(a, w, lane, njobs, quota, stretch);
+    engine_loop<false>(a, w, lane, njobs, quota, stretch, blockIdx.x * EWARPS + wid, warps);
 }
 
 // ================================================================== the persistent kernel
@@ -1162,7 +1170,7 @@ __global__ void __launch_bounds__(PBS, 3) search_persist(const __grid_constant__
             }
         } else {
             WarpArea *w = (WarpArea *)(smem + (size_t)wid * sizeof(WarpArea));
-            if (engine_loop<true>(a, w, lane, 0u, 32u, 0u) && lane == 0) s_busy = 1;
+            if (engine_loop<true>(a, w, lane, 0u, 32u, 0u, 0u, 0u) && lane == 0) s_busy = 1;
             __syncthreads();
             if (tid == 0) {
                 if (s_busy) {
