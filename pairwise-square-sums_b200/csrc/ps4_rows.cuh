@@ -141,13 +141,12 @@ __device__ __forceinline__ void gen_list(uint32_t *d, const uint32_t (*fp)[32], 
     }
 }
 
-// Residue masks of a candidate's v = f + g = 2u.  e + C = u^2 + (C - A) must be a square mod 64, 63
-// and 65 for both remaining members C (s4.c:192-194): one bit test per modulus, against the AND of
-// the two members' masks q_m[(C - A) mod m].
-//  * mod 64: u^2 mod 64 depends on u mod 32, bit v/2 mod 32.
-//  * mod 63 and 65: with x = (v >> 24) + (v & 0xFFFFFF) + 32 = v + 32 (2^24 = 1 in both), bit x mod 63, and bit (x
-//    mod 65) mod 64: x = 0 and 64 mod 65 are v = -32 and 32, whose squares are equal, so 65 residues
-//    fit 64 bits.
+// Residue masks of a candidate's w = f + g + 32 = 2u + 32.  e + C = u^2 + (C - A) must be a square mod
+// 64, 63 and 65 for every remaining member C (s4.c:192-194): one bit test per modulus, against the AND of
+// the members' masks q_m[(C - A) mod m].
+//  * mod 64: u^2 mod 64 depends on u mod 32, bit w/2 mod 32.
+//  * mod 63 and 65: bit w mod 63, and bit (w mod 65) mod 64: w = 0 and 64 mod 65 are 2u = -32 and 32, whose
+//    squares are equal, so 65 residues fit 64 bits.
 struct VResTabs {
     uint64_t q63[63], q65[65];
     uint32_t q64[64];
@@ -159,7 +158,7 @@ constexpr VResTabs make_vres() {
     VResTabs t{};
     for (int a = 0; a < 64; a++)
         for (int u = 0; u < 32; u++)
-            if (is_qr_mod(64, (u * u + a) % 64)) t.q64[a] |= 1u << u;
+            if (is_qr_mod(64, (u * u + a) % 64)) t.q64[a] |= 1u << ((u + 16) % 32);
     for (int a = 0; a < 63; a++)
         for (int x = 0; x < 63; x++) {
             const int u = (x + 31) * 32 % 63;                     // (x - 32) / 2; 1/2 = 32
@@ -187,16 +186,19 @@ __device__ __forceinline__ void and_masks(int64_t d, uint32_t &m64, uint64_t &m6
     m65 &= __ldg(&VQ.q65[mod65(r)]);
 }
 
-// One candidate of a row: v = f + g = x*fy + y*gy and whether it passes the filters (bit 0).
-__device__ __forceinline__ uint32_t candidate(uint32_t x, uint32_t y, uint64_t fy, uint64_t gy, uint32_t m64,
-                                              uint64_t m63, uint64_t m65, uint64_t &v) {
-    const uint64_t lo = (uint64_t)x * (uint32_t)fy + (uint64_t)y * (uint32_t)gy;
-    const uint32_t hi = (uint32_t)(lo >> 32) + x * (uint32_t)(fy >> 32) + y * (uint32_t)(gy >> 32);
-    v = (uint64_t)hi << 32 | (uint32_t)lo;
-    const uint32_t z = (uint32_t)(v >> 24) + ((uint32_t)lo & 0xFFFFFFu) + 32u;
-    return __funnelshift_r(m64, m64, (uint32_t)lo >> 1) & (uint32_t)(m63 >> mod63(z)) &
-           (uint32_t)(m65 >> (mod65(z) & 63u));
+// One candidate of a row: w = f + g + c = x*fy + y*gy + c, and whether it passes the filters (bit 0).  c is 32
+// with a tag from bit 58 up, which the sum (below 2^46) does not reach: an entry for the queue as it is.
+// The filters' index is w folded at 24 bits, lo - (lo >> 24)(2^24 - 1) + 256 hi (2^24 = 2^12 = 1 mod 63 and 65), in
+// multiplications, which have a pipe to themselves, and modulo 2^32, where the tag times 256 vanishes.
+__device__ __forceinline__ uint32_t candidate(uint32_t x, uint32_t y, uint64_t fy, uint64_t gy, uint64_t c, uint32_t m64,
+                                              uint64_t m63, uint64_t m65, uint64_t &w) {
+    const uint64_t s = (uint64_t)y * (uint32_t)gy + ((uint64_t)x * (uint32_t)fy + c);
+    const uint32_t lo = (uint32_t)s, hi = y * (uint32_t)(gy >> 32) + (x * (uint32_t)(fy >> 32) + (uint32_t)(s >> 32));
+    w = (uint64_t)hi << 32 | lo;
+    const uint32_t z = (lo >> 24) * (1u - (1u << 24)) + (hi * 256u + lo);        // below 2^25
+    return __funnelshift_r(m64, m64, lo >> 1) & (uint32_t)(m63 >> mod63(z)) & (uint32_t)(m65 >> (mod65(z) & 63u));
 }
+constexpr uint64_t W_SUM = (1ull << 58) - 1;                 // f + g + 32 of an entry
 
 // Whether n = u^2 + d is a square; n > 0, u < 2^44, |d| < 2^44, n's low 64 bits given.  If n = s^2
 // then s < 2^45; the double of n is one rounding off (2^-53), and two Newton steps from the single-precision

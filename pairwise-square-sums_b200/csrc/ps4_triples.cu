@@ -27,7 +27,7 @@ constexpr int TBS = 128;                 // threads per CTA of the triple kernel
 constexpr int TDCAP = 640;               // divisor-list entries per warp (u32)
 
 struct __align__(16) TJob {              // one lane's triple: d = u^2 - A
-    uint64_t m63, m65;                   // residue masks of f + g = 2u for the third member
+    uint64_t m63, m65;                   // residue masks of f + g + 32 for the third member
     uint32_t m64, geo;                   // geo: L | H << 8 | E2 << 16 | list place << 22
     uint64_t A, B, C;
     uint64_t uA, umax;                   // u <= uA: d <= 0; u > umax: d > dmax
@@ -82,8 +82,9 @@ static __device__ __noinline__ uint32_t tri_walk(const TriArgs &t, const TJob &j
             if (2 * todd + 1 == ndo && 2 * d2 >= E2) break;       // self-complementary half already seen
             const uint64_t v = (fo << d2) + (go << (E2 - d2)), u = v >> 1;
             if (u <= j.uA || u > j.umax) continue;
-            const uint32_t z = (uint32_t)(v >> 24) + ((uint32_t)v & 0xFFFFFFu) + 32u;
-            if (__funnelshift_r(m64, m64, (uint32_t)v >> 1) & (uint32_t)(j.m63 >> mod63(z)) &
+            const uint64_t w = v + 32;
+            const uint32_t z = (uint32_t)(w >> 24) + ((uint32_t)w & 0xFFFFFFu);
+            if (__funnelshift_r(m64, m64, (uint32_t)w >> 1) & (uint32_t)(j.m63 >> mod63(z)) &
                 (uint32_t)(j.m65 >> (mod65(z) & 63u)) & 1u)
                 nsq += tri_test(t, j, u);
         }
@@ -198,10 +199,10 @@ __global__ void __launch_bounds__(TBS) extend_triples_kernel(const __grid_consta
                 const int turns = (int)__reduce_max_sync(FULL, (unsigned)row.len);
                 for (int l = 0; l < turns; l++) {
                     uint64_t v;
-                    const uint32_t p = candidate(*row.xf, *row.xg, row.fy, row.gy, m64, m63, m65, v);
+                    const uint32_t p = candidate(*row.xf, *row.xg, row.fy, row.gy, 32u, m64, m63, m65, v);
                     row.xf++;
                     row.xg--;
-                    const uint64_t u = v >> 1;
+                    const uint64_t u = (v - 32) >> 1;
                     if (l < row.len && (p & 1u) && u > uA && u <= umax && tri_test(t, j, u))
                         atomicAdd(&w->job[jl].nsq, 1u);
                 }
