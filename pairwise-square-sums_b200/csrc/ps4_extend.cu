@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const 
 constexpr int EBS = 256;                 // threads per CTA
 constexpr int EWARPS = EBS / 32;
 constexpr int DCAP = 640;                // divisor-list entries per warp (u32)
-constexpr int QCAP = 96;                 // square-test queue per warp
+constexpr int QCAP = 128;                // square-test queue per warp
 constexpr int EXCAP = 8;                 // extensions per warp and round
 constexpr int ICACHE = 8;                // items whose counters a warp holds back
 
@@ -879,31 +879,40 @@ static __device__ __noinline__ void record_ext(const SearchArgs &a, WarpArea *w,
     }
 }
 
-// Queue entries [first, first+count), one per lane: those with 0 < e = u^2 - A not in the 4-set are the
-// reference's ext_sqrt (s4.c:195-198) and are square-tested (s4.c:199-203).
+// Queue entries [first, first+count), two per lane (their chains of double arithmetic overlap): those
+// with 0 < e = u^2 - A not in the 4-set are the reference's ext_sqrt (s4.c:195-198) and are
+// square-tested (s4.c:199-203).
 __device__ __forceinline__ void process_queue(const SearchArgs &a, WarpArea *w, uint32_t first, uint32_t count,
                                               int lane, WarpCounters &cnt) {
-    if ((uint32_t)lane < count) {
-        const uint64_t ent = w->q[first + lane];
-        const uint32_t jl = (uint32_t)(ent >> 58);
-        const uint64_t u = ((ent & W_SUM) - 32) >> 1, u2 = u * u;          // u < 2^44; u2 mod 2^64
-        const EJob &E = w->job[jl];
+    uint32_t jl[2];
+    uint64_t u[2], u2[2];
+    bool hit[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const uint32_t at = lane + 32 * k;
+        const uint64_t ent = w->q[first + (at < count ? at : 0)];
+        jl[k] = (uint32_t)(ent >> 58);
+        u[k] = ((ent & W_SUM) - 32) >> 1;                                        // below 2^44
+        u2[k] = u[k] * u[k];                                                     // mod 2^64
+        const EJob &E = w->job[jl[k]];
         const uint64_t A = E.A;
         const uint4 ro = *(const uint4 *)&E.rA0;
-        const uint32_t ul = (uint32_t)u;
+        const int64_t d1 = E.d1;
+        const uint32_t ul = (uint32_t)u[k];
         // u below 2^32: e > 0 iff u2 > A; e = A iff u2 = 2A; e another member iff u one of A's roots
-        if ((u >> 32) != 0 || (u2 > A && u2 != 2 * A && ul != ro.x && ul != ro.y && ul != ro.z)) {
-            if ((ro.w & 0xFFFFFu) == cnt.item) cnt.sqrt_++;
-            else atomicAdd(&w->job[jl].item, 1u << 20);
-            bool sq = true;
-#pragma unroll 1
-            for (int c = 0; c < 2 && sq; c++) {                                  // one copy of the code
-                const int64_t d = (&E.d1)[c];
-                sq = is_square_near(u, d, u2 + (uint64_t)d);
-            }
-            if (sq) record_ext(a, w, jl, u);
-        }
+        const bool test = at < count && ((u[k] >> 32) != 0 || (u2[k] > A && u2[k] != 2 * A && ul != ro.x &&
+                                                               ul != ro.y && ul != ro.z));
+        const bool here = (ro.w & 0xFFFFFu) == cnt.item;
+        cnt.sqrt_ += test && here;
+        if (test && !here) atomicAdd(&w->job[jl[k]].item, 1u << 20);
+        hit[k] = is_square_near(u[k], d1, u2[k] + (uint64_t)d1) && test;
     }
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        if (hit[k]) {                                                            // rare
+            const int64_t d2 = w->job[jl[k]].d2;
+            if (is_square_near(u[k], d2, u2[k] + (uint64_t)d2)) record_ext(a, w, jl[k], u[k]);
+        }
 }
 
 // The engine loop of one warp.  Linear (RING false): the batch's queue [0, njobs), filled before
@@ -1049,10 +1058,10 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
                     if (b0) w->q[qn + __popc(a0 & below)] = v0;
                     if (b1) w->q[qn + n0 + __popc(a1 & below)] = v1;
                     qn += n0 + __popc(a1);
-                    // the queue is emptied 32 at a time, and whole after the round's last turn
-                    const uint32_t least = l + 2 >= turns && g0 + 32 >= plan.total ? 1u : 32u;
+                    // the queue is emptied 64 at a time, and whole after the round's last turn
+                    const uint32_t least = l + 2 >= turns && g0 + 32 >= plan.total ? 1u : 64u;
                     while (qn >= least) {
-                        const uint32_t n = min(qn, 32u);
+                        const uint32_t n = min(qn, 64u);
                         qn -= n;
                         __syncwarp();
                         process_queue(a, w, qn, n, lane, cnt);

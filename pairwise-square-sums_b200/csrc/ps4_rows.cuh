@@ -129,14 +129,24 @@ __device__ __forceinline__ void split_pair(const uint64_t *spfq, uint4 fa, uint4
 }
 
 // The divisors of the n prime powers from slot q, in mixed-radix order (first prime fastest): prime
-// after prime, the list so far is repeated e times, each copy p times the one before.
+// after prime, the list so far is repeated e times, each copy p times the one before.  After the first
+// prime two entries at a time, whose loads do not wait for each other's stores.
 __device__ __forceinline__ void gen_list(uint32_t *d, const uint32_t (*fp)[32], int lane, uint32_t q, uint32_t n) {
     d[0] = 1;
+    if (n == 0) return;
     uint32_t cur = 1;
-    for (uint32_t i = 0; i < n; i++) {
+    {
+        const uint32_t x = fp[q][lane], p = x & 0xFFFFFFu, e = x >> 24;
+        for (uint32_t v = p; cur <= e; v *= p) d[cur++] = v;
+    }
+    for (uint32_t i = 1; i < n; i++) {
         const uint32_t x = fp[q + i][lane], p = x & 0xFFFFFFu, add = cur * (x >> 24);
 #pragma unroll 1
-        for (uint32_t j = 0; j < add; j++) d[cur + j] = d[j] * p;
+        for (uint32_t j = 0; j < add; j += 2) {
+            const uint32_t a = d[j] * p, b = d[j + 1] * p;
+            d[cur + j] = a;
+            if (j + 1 < add) d[cur + j + 1] = b;
+        }
         cur += add;
     }
 }
