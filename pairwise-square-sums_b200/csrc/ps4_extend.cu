@@ -14,7 +14,7 @@
 //                 multiplications each.  Residue filters mod 64/63/65 are bit tests against
 //                 per-4-set masks indexed by residues of f + g = 2u; the candidates that pass go
 //                 through a warp queue, where those that are the reference's ext_sqrt are
-//                 square-tested 32 at a time.                                  (s4.c:160-207)
+//                 square-tested 64 at a time.                                  (s4.c:160-207)
 //
 // The engine is bound by instruction issue (67 % of issue slots busy, 28.8 of 32 threads active; DRAM 2.5 %).
 // Per [1,1e10) search its launches take 192 ms; with candidates spread over the lanes in 32 equal
@@ -196,13 +196,13 @@ __device__ __forceinline__ uint32_t pair_sets(const TileView &v, uint64_t S0, ui
                                               uint32_t &lo0, PairSets &ps) {
     // every selected S has a pair at least, so 32 consecutive pairs lie in 32 consecutive ones
     const uint32_t pb = lo0 + lane < v.n_is ? v.pbase[lo0 + lane] : 0xFFFFFFFFu;
-    uint32_t o = 0;
-#pragma unroll
-    for (uint32_t step = 16; step; step >>= 1)
-        if (__shfl_sync(0xffffffffu, pb, o + step) <= g) o += step;
+    const uint32_t rel = pb - (g - lane);                  // starts behind the first pair, as a bit mask
+    const unsigned upto = __popc(__ballot_sync(0xffffffffu, pb <= g - lane));
+    const unsigned starts = __reduce_or_sync(0xffffffffu, rel - 1u < 31u ? 1u << rel : 0u);
+    const uint32_t o = upto + __popc(starts & (0xFFFFFFFFu >> (31 - lane))) - 1;
     const uint32_t base = __shfl_sync(0xffffffffu, pb, o);
     const uint32_t lo = lo0 + o;
-    lo0 = __shfl_sync(0xffffffffu, lo, 31);
+    lo0 += upto + __popc(starts) - 1;
     if (g >= ge) return 0;
     const uint32_t st = v.start[lo], k = v.k[lo];
     const uint64_t S = S0 + v.off[lo];
@@ -533,7 +533,9 @@ __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const 
 constexpr int EBS = 256;                 // threads per CTA
 constexpr int EWARPS = EBS / 32;
 constexpr int DCAP = 640;                // divisor-list entries per warp (u32)
-constexpr int QCAP = 128;                // square-test queue per warp
+constexpr int CPT = 4;                   // candidates of a row per turn: independent chains (4 / 3 / 2: 175.5 / 181.8 /
+                                         //   179.2 ms per [1,1e10) search)
+constexpr int QCAP = 64 + 32 * CPT;      // square-test queue per warp
 constexpr int EXCAP = 8;                 // extensions per warp and round
 constexpr int ICACHE = 8;                // items whose counters a warp holds back
 
@@ -559,7 +561,7 @@ struct ItemCount {                       // counters of an item that the warp ho
 
 struct WarpArea {
     EJob job[32];
-    uint32_t dbuf[DCAP];                 // a turn may read up to LCAP entries past a list's ends: the
+    uint32_t dbuf[DCAP];                 // turns may read LCAP + CPT entries past a list's ends: the
                                          //   neighbours on both sides are longer than that
     union {                              // primes until the lists are made, then the queue
         uint32_t fp[2 * FSIDE][32];      // each lane's odd primes of D (p | e << 24), m1's from slot 0, m2's
@@ -576,7 +578,7 @@ struct WarpArea {
     uint32_t n_ext;
     uint8_t order[32];                   // lanes by row length, longest first
 };
-static_assert(sizeof(EJob) * 32 >= 4 * LCAP && 4 * 32 * 2 * FSIDE >= 4 * LCAP, "neighbours of dbuf");
+static_assert(sizeof(EJob) * 32 >= 4 * (LCAP + CPT) && 4 * 32 * 2 * FSIDE >= 4 * (LCAP + CPT), "neighbours of dbuf");
 static_assert(EWARPS * sizeof(WarpArea) + 1024 <= 228 * 1024 / 3, "three engine CTAs per SM");
 
 constexpr uint32_t NO_ITEM = 0xFFFFFFFFu;
@@ -1033,7 +1035,7 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
             }
             RowPlan plan;
             plan_rows(fits ? J.rows : 0, J.L, w->order, lane, plan);
-            // ---- phase B: 32 rows at a time, one per lane, two candidates of each per turn
+            // ---- phase B: 32 rows at a time, one per lane, CPT candidates of each per turn
             uint32_t qn = 0;
             for (uint32_t g0 = 0; g0 < plan.total; g0 += 32) {
                 uint32_t r;
@@ -1045,21 +1047,25 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
                 const int turns = (int)__reduce_max_sync(FULL, (unsigned)row.len);
                 const uint64_t tag = (uint64_t)jl << 58 | 32u;
 #pragma unroll 1
-                for (int l = 0; l < turns; l += 2) {
-                    uint64_t v0, v1;
-                    const uint32_t p0 = candidate(row.xf[0], row.xg[0], row.fy, row.gy, tag, jj.x, mm.x, mm.y, v0);
-                    const uint32_t p1 = candidate(row.xf[1], row.xg[-1], row.fy, row.gy, tag, jj.x, mm.x, mm.y, v1);
-                    row.xf += 2;
-                    row.xg -= 2;
-                    const bool b0 = l < row.len && (p0 & 1u), b1 = l + 1 < row.len && (p1 & 1u);
-                    const unsigned a0 = __ballot_sync(FULL, b0), a1 = __ballot_sync(FULL, b1);
+                for (int l = 0; l < turns; l += CPT) {
+                    uint64_t v[CPT];
+                    bool ok[CPT];
                     const unsigned below = (1u << lane) - 1u;
-                    const uint32_t n0 = __popc(a0);
-                    if (b0) w->q[qn + __popc(a0 & below)] = v0;
-                    if (b1) w->q[qn + n0 + __popc(a1 & below)] = v1;
-                    qn += n0 + __popc(a1);
+#pragma unroll
+                    for (int k = 0; k < CPT; k++) {
+                        const uint32_t p = candidate(row.xf[k], row.xg[-k], row.fy, row.gy, tag, jj.x, mm.x, mm.y, v[k]);
+                        ok[k] = l + k < row.len && (p & 1u);
+                    }
+                    row.xf += CPT;
+                    row.xg -= CPT;
+#pragma unroll
+                    for (int k = 0; k < CPT; k++) {
+                        const unsigned m = __ballot_sync(FULL, ok[k]);
+                        if (ok[k]) w->q[qn + __popc(m & below)] = v[k];
+                        qn += __popc(m);
+                    }
                     // the queue is emptied 64 at a time, and whole after the round's last turn
-                    const uint32_t least = l + 2 >= turns && g0 + 32 >= plan.total ? 1u : 64u;
+                    const uint32_t least = l + CPT >= turns && g0 + 32 >= plan.total ? 1u : 64u;
                     while (qn >= least) {
                         const uint32_t n = min(qn, 64u);
                         qn -= n;
