@@ -16,9 +16,9 @@
 //                 through a warp queue, where those that are the reference's ext_sqrt are
 //                 square-tested 64 at a time.                                  (s4.c:160-207)
 //
-// The engine is bound by instruction issue (67 % of issue slots busy, 28.8 of 32 threads active; DRAM 2.5 %).
-// Per [1,1e10) search its launches take 192 ms; with candidates spread over the lanes in 32 equal
-// runs, u64 lists, per-candidate member tests and IEEE double square roots they took 313 ms (25.5 -> 15.8 warp
+// The engine is bound by instruction issue (74 % of issue slots busy, 30.0 of 32 threads active; DRAM 2.4 %).
+// Per [1,1e10) search its launches take 163 ms; with candidates spread over the lanes in 32 equal
+// runs, u64 lists, per-candidate member tests and IEEE double square roots they took 313 ms (25.5 -> 14.8 warp
 // instructions per S).  Rows cost a partly empty turn (30.2 turns of 32 candidates per round against
 // 24.9 full ones) and save the per-candidate bookkeeping, half of the 85 instructions of the old loop.
 //
@@ -536,7 +536,7 @@ constexpr int DCAP = 640;                // divisor-list entries per warp (u32)
 constexpr int CPT = 4;                   // candidates of a row per turn: independent chains (4 / 3 / 2: 175.5 / 181.8 /
                                          //   179.2 ms per [1,1e10) search)
 constexpr int QCAP = 64 + 32 * CPT;      // square-test queue per warp
-constexpr int EXCAP = 8;                 // extensions per warp and round
+constexpr int EXCAP = 8;                 // extensions found in a warp's round
 constexpr int ICACHE = 8;                // items whose counters a warp holds back
 
 struct __align__(16) EJob {              // one lane's 4-set
@@ -569,17 +569,23 @@ struct WarpArea {
         uint64_t q[QCAP];                // candidates that pass the filters: f + g + 32 | job << 58
     };
     ItemCount ic[ICACHE];
-    ExtEntry ext[EXCAP];
+    uint64_t hit_u[EXCAP];               // what rare_work is left with: the round's extensions u, their
+    uint32_t hit_jid[EXCAP];             //   4-sets,
+    uint32_t big[64];                    //   and the 4-sets for the per-lane divisor walk (queue indices)
+    uint32_t n_hit, n_big, n_ext;
+    uint32_t pend, rel, took;            // the rounds' state while rare_work runs (lane masks)
     uint32_t jid[32];                    // queue index of each lane's 4-set
     // the loop's own state, out of the registers between its claims (the same for all lanes)
     uint32_t njobs, quota, stretch;      // queue length; lanes that hold a 4-set; 4-sets per stretch
     uint32_t st_cur, st_rem, last;       // the stretch at hand; whether it is the last
     uint32_t claimed;                    // 4-sets in the warps' first stretches
-    uint32_t n_ext;
     uint8_t order[32];                   // lanes by row length, longest first
 };
 static_assert(sizeof(EJob) * 32 >= 4 * (LCAP + CPT) && 4 * 32 * 2 * FSIDE >= 4 * (LCAP + CPT), "neighbours of dbuf");
 static_assert(EWARPS * sizeof(WarpArea) + 1024 <= 228 * 1024 / 3, "three engine CTAs per SM");
+
+constexpr int EXTCAP = 4 * DCAP / (int)sizeof(ExtEntry);     // a report's extensions, in dbuf
+static_assert(offsetof(WarpArea, dbuf) % 8 == 0 && EXTCAP >= EXCAP, "room for a report");
 
 constexpr uint32_t NO_ITEM = 0xFFFFFFFFu;
 
@@ -641,10 +647,10 @@ struct WarpCounters {
 };
 static_assert(ICACHE == 8, "the cache index is a 3-bit hash");
 
-// Report the extensions of one warp round: group them per 4-set, emit hit / ext / six
+// Report a warp's extensions: group them per 4-set, emit hit / ext / six
 // records and the counters sets5 / multi / sets6 / hist5 / max_extensions (s4.c:243-277).
 template <bool COH>
-static __device__ __noinline__ void report_warp_exts(const SearchArgs &a, ExtEntry *el, uint32_t n) {
+static __device__ void report_warp_exts(const SearchArgs &a, ExtEntry *el, uint32_t n) {
     for (uint32_t x = 1; x < n; x++) {
         ExtEntry k = el[x];
         uint32_t y = x;
@@ -735,6 +741,12 @@ struct LaneJob {                                 // a lane's 4-set in its round
     bool big;                                    // for the per-lane divisor walk
 };
 
+// p[i] by a 32-bit byte offset (tables are below 2^32 bytes): one register for an address in flight, not two
+template <class T>
+__device__ __forceinline__ T ldg_at(const T *p, uint32_t i) {
+    return __ldg((const T *)((const char *)p + (uint32_t)(i * (uint32_t)sizeof(T))));
+}
+
 // Phase A: one 4-set per lane.  Picks the difference to extend by (the fewest estimated divisors, in
 // the candidate order and with the tie-break of s4.c:163-171), factors it and writes the lane's
 // EJob.  False: an empty record, or more divisors than the cap.
@@ -748,7 +760,7 @@ __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJ
     uint32_t best = 0xFFFFFFFFu, rik = 0, rjk = 0;
     auto pair = [&](int t, uint32_t x, uint32_t y) {
         const uint32_t hi = max(x, y), lo = min(x, y);
-        const uint32_t est = (uint32_t)__ldg(&a.ndiv[hi - lo]) * (uint32_t)__ldg(&a.ndiv[hi + lo]);
+        const uint32_t est = (uint32_t)ldg_at(a.ndiv, hi - lo) * (uint32_t)ldg_at(a.ndiv, hi + lo);
         const uint32_t key = est * 8u + t;                                       // est < 2^26
         if (key < best) { best = key; rik = x; rjk = y; }
     };
@@ -767,7 +779,7 @@ __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJ
         m1 >>= z1;
         m2 >>= z2;
     }
-    const uint4 fa = __ldg(&a.fac[m1 >> 1]), fb = __ldg(&a.fac[m2 >> 1]);
+    const uint4 fa = ldg_at(a.fac, m1 >> 1), fb = ldg_at(a.fac, m2 >> 1);
     EJob &E = w->job[lane];
     {
         uint64_t v[4];
@@ -820,29 +832,30 @@ __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJ
 }
 
 // A 4-set whose factored divisor lists exceed the warp buffer or 32 bits: the per-lane divisor walk.
-// Returns its ext_sqrt.
+// Returns its ext_sqrt and its item.
 template <bool COH>
-static __device__ __noinline__ uint32_t extend_big(const SearchArgs &a, uint32_t qid, ExtEntry *el,
-                                                   uint32_t *el_n) {
+__device__ __forceinline__ uint32_t extend_big(const SearchArgs &a, uint32_t qid, ExtEntry *el, uint32_t *el_n,
+                                               uint32_t &item) {
     ull cand = 0, sq = 0;
-    uint32_t r[6], item, best, md = 0;
+    uint32_t r[6], best, md = 0;
     uint64_t v[4], S;
     int bi, bj, bk;
     get_job<COH>(a.jobs, qid, r, item);
     quad_values(r, v, S);
     choose_pair(v, r, a.ndiv, bi, bj, bk, best);
-    extend_quad(a, r, v, S, bi, bj, bk, qid, cand, sq, md, el, el_n, EXCAP);
+    extend_quad(a, r, v, S, bi, bj, bk, qid, cand, sq, md, el, el_n, EXTCAP);
     return (uint32_t)sq;
 }
 
-// The extension e = u^2 - A of lane jl's 4-set (rare).  Its order key is the reference's mixed-radix
+// The extension e = u^2 - A of the 4-set at queue index qid.  Its order key is the reference's mixed-radix
 // index of the smaller divisor f = u - w, w^2 = e + B, over the primes in first-seen order: 2, m1's, then
 // m2's others (s4.c:141-156).
-static __device__ __noinline__ void record_ext(const SearchArgs &a, WarpArea *w, uint32_t jl, uint64_t u) {
+__device__ __forceinline__ void record_ext(const SearchArgs &a, ExtEntry *el, uint32_t *el_n, uint32_t qid,
+                                           uint64_t u) {
     uint32_t rt[6], item, best;
     uint64_t v[4], S;
     int bi, bj, bk;
-    get_job<true>(a.jobs, w->jid[jl], rt, item);
+    get_job<true>(a.jobs, qid, rt, item);
     quad_values(rt, v, S);
     choose_pair(v, rt, a.ndiv, bi, bj, bk, best);
     const uint32_t ra = pick6(rt, pair_slot(bi, bk)), rb = pick6(rt, pair_slot(bj, bk));
@@ -869,23 +882,57 @@ static __device__ __noinline__ void record_ext(const SearchArgs &a, WarpArea *w,
             mult *= ex + 1;
         }
     }
-    const uint32_t slot = atomicAdd(&w->n_ext, 1u);
-    if (slot < EXCAP) {
-        ExtEntry &x = w->ext[slot];
-        x.qid = w->jid[jl];
+    const uint32_t slot = atomicAdd(el_n, 1u);
+    if (slot < EXTCAP) {
+        ExtEntry &x = el[slot];
+        x.qid = qid;
         x.key = key;
         x.lo = (uint64_t)e;
         x.hi = (uint64_t)(e >> 64);
     } else {
-        raise_capacity(a.status, E_EXTLIST, 4, slot + 1, EXCAP, 0);
+        raise_capacity(a.status, E_EXTLIST, 4, slot + 1, EXTCAP, 0);
     }
+}
+
+// What a round seldom has, between two runs of rounds: the 4-sets for the divisor walk, one per lane, and
+// the round's extensions, which are recorded and reported.  Called where nothing of a round is live:
+// with these calls inside the rounds the compiler kept the rounds' values in local memory (58 M of
+// 4.5 G instructions and half of the waiting on loads per 3e8 S at 5e9; [1,1e10) engine 175.5 ->
+// 163.4 ms), and one lane walked alone while the others waited (2e8 S at 1e12: 11.4 -> 10.5 ms).
+template <bool COH>
+static __device__ __noinline__ void rare_work(const SearchArgs &a, WarpArea *w) {
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31, nb = w->n_big, nh = w->n_hit;
+    ExtEntry *el = (ExtEntry *)w->dbuf;          // free between rounds
+    if (lane == 0) w->n_ext = 0;
+    __syncwarp();
+    for (uint32_t b = 0; b < nb; b += 32) {
+        const bool have = b + lane < nb;
+        uint32_t item = 0, sq = 0;
+        if (have) sq = extend_big<COH>(a, w->big[b + lane], el, &w->n_ext, item);
+        const uint32_t it0 = __shfl_sync(FULL, item, 0);
+        if (__all_sync(FULL, !have || item == it0)) {
+            sq = __reduce_add_sync(FULL, sq);
+            if (lane == 0) count_global(a, it0, 0, sq, 0);
+        } else if (have) {
+            count_global(a, item, 0, sq, 0);
+        }
+    }
+    if (lane < min(nh, (uint32_t)EXCAP)) record_ext(a, el, &w->n_ext, w->hit_jid[lane], w->hit_u[lane]);
+    __syncwarp();
+    if (lane == 0) {
+        if (nh > (uint32_t)EXCAP) raise_capacity(a.status, E_EXTLIST, 4, nh, EXCAP, 0);
+        if (w->n_ext) report_warp_exts<COH>(a, el, min(w->n_ext, (uint32_t)EXTCAP));
+        w->n_hit = w->n_big = 0;
+    }
+    __syncwarp();
 }
 
 // Queue entries [first, first+count), two per lane (their chains of double arithmetic overlap): those
 // with 0 < e = u^2 - A not in the 4-set are the reference's ext_sqrt (s4.c:195-198) and are
 // square-tested (s4.c:199-203).
-__device__ __forceinline__ void process_queue(const SearchArgs &a, WarpArea *w, uint32_t first, uint32_t count,
-                                              int lane, WarpCounters &cnt) {
+__device__ __forceinline__ void process_queue(WarpArea *w, uint32_t first, uint32_t count, int lane,
+                                              WarpCounters &cnt) {
     uint32_t jl[2];
     uint64_t u[2], u2[2];
     bool hit[2];
@@ -913,7 +960,13 @@ __device__ __forceinline__ void process_queue(const SearchArgs &a, WarpArea *w, 
     for (int k = 0; k < 2; k++)
         if (hit[k]) {                                                            // rare
             const int64_t d2 = w->job[jl[k]].d2;
-            if (is_square_near(u[k], d2, u2[k] + (uint64_t)d2)) record_ext(a, w, jl[k], u[k]);
+            if (is_square_near(u[k], d2, u2[k] + (uint64_t)d2)) {
+                const uint32_t slot = atomicAdd(&w->n_hit, 1u);
+                if (slot < EXCAP) {
+                    w->hit_u[slot] = u[k];
+                    w->hit_jid[slot] = w->jid[jl[k]];
+                }
+            }
         }
 }
 
@@ -925,26 +978,21 @@ __device__ __forceinline__ void process_queue(const SearchArgs &a, WarpArea *w, 
 // short to fill every warp of the launch; the candidates of few 4-sets are still walked by all
 // lanes).  The first `claimed` stretches belong to the warps in order, this one is number `first`.  Returns
 // whether the warp took any 4-set.
+// Runs rounds until rare_work is due (true), or the queue is drained or an error is raised (false).
 template <bool RING>
-__device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint32_t njobs, uint32_t quota,
-                                            uint32_t stretch, uint32_t first, uint32_t claimed) {
+__device__ __forceinline__ bool engine_rounds(const SearchArgs &a, WarpArea *w, int lane) {
     const unsigned FULL = 0xffffffffu;
-    if (lane == 0) {
-        w->n_ext = 0;
-        w->njobs = njobs; w->quota = quota; w->stretch = stretch;
-        // the warp's first stretch is its own place in the grid (a short queue needs no atomics, whose turns
-        // on one address took 12 of a small call's 29 us), the later ones are claimed behind them
-        const uint32_t at = min(first * stretch, njobs);
-        w->st_cur = at;
-        w->st_rem = RING ? 0 : min(stretch, njobs - at);
-        w->last = (uint64_t)claimed * stretch >= njobs;
-        w->claimed = claimed * stretch;
-    }
-    if (lane < ICACHE) w->ic[lane].item = NO_ITEM;
-    __syncwarp();
     WarpCounters cnt;
-    bool pending = false, drained = false, rel = false, took = false;
-    uint64_t mypos = 0;
+    bool pending = w->pend >> lane & 1u, drained = false, took = false, more = false;
+    bool rel = RING && (w->rel >> lane & 1u);
+    uint64_t mypos = RING ? w->q[lane] : 0;
+    auto release = [&]() {                     // finished 4-sets hand their slots back, after their report
+        const unsigned rm = __ballot_sync(FULL, rel);
+        if (rel) ring_release(a, mypos);
+        rel = false;
+        if (lane == 0 && rm) atomicAdd(&a.status->q_freed, (ull)__popc(rm));
+    };
+    if (RING) release();
 
     // Rounds: every lane without a 4-set takes the next one from the queue; a lane whose divisor lists
     // did not fit keeps its 4-set, sets it up again and goes first in the next round's placement.
@@ -1007,17 +1055,14 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
         J.item = J.ncand = J.nd = 0;
         J.big = false;
         const bool mine = pending;
-        uint32_t bsq = 0;
-        if (pending) {
-            pending = job_setup<RING>(a, w->jid[lane], J, w, lane);
-            if (pending && J.big) {                                      // rare
-                bsq = extend_big<RING>(a, w->jid[lane], w->ext, &w->n_ext);
-                pending = false;
-            }
+        if (pending) pending = job_setup<RING>(a, w->jid[lane], J, w, lane);
+        const bool fresh = pending && !old;                              // counted once
+        if (pending && J.big) {                                          // rare
+            w->big[atomicAdd(&w->n_big, 1u)] = w->jid[lane];             // fewer than 32 are there
+            pending = false;
         }
-        if (RING && mine && !pending) rel = true;                        // done: freed after the report
-        const bool fresh = mine && !old && (pending || J.big);           // counted once
-        cnt.add(a, w, lane, fresh, J.item, J.ncand, bsq, J.nd);
+        if (RING && mine && !pending) rel = true;
+        cnt.add(a, w, lane, fresh, J.item, J.ncand, 0, J.nd);
         const bool round = __any_sync(FULL, pending);
         if (round) {
             // place the factored divisor lists of as many pending lanes as fit: lanes left over
@@ -1070,7 +1115,7 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
                         const uint32_t n = min(qn, 64u);
                         qn -= n;
                         __syncwarp();
-                        process_queue(a, w, qn, n, lane, cnt);
+                        process_queue(w, qn, n, lane, cnt);
                         __syncwarp();
                     }
                 }
@@ -1082,25 +1127,49 @@ __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, in
             if (RING && fits) rel = true;
         }
         __syncwarp();
-        if (lane == 0 && w->n_ext) {          // this round's extensions (and any from the per-lane path)
-            report_warp_exts<RING>(a, w->ext, min(w->n_ext, (uint32_t)EXCAP));
-            w->n_ext = 0;
-        }
-        __syncwarp();
-        if (RING) {                            // the round's finished 4-sets hand their slots back
-            const unsigned rm = __ballot_sync(FULL, rel);
-            if (rel) ring_release(a, mypos);
-            rel = false;
-            if (lane == 0 && rm) atomicAdd(&a.status->q_freed, (ull)__popc(rm));
-        }
-        if (!round && drained) break;          // warp-uniform
+        const bool end = !round && drained;                              // warp-uniform
+        more = w->n_hit || w->n_big >= (RING || end ? 1u : 32u);         // warp-uniform
+        __syncwarp();                                                    // read by all
+        if (more) break;
+        if (RING) release();
+        if (end) break;
     }
     cnt.flush(a, w, lane);
+    const unsigned pm = __ballot_sync(FULL, pending), rm = __ballot_sync(FULL, rel);
+    const bool tm = __any_sync(FULL, took);
+    if (RING) w->q[lane] = mypos;
+    if (lane == 0) {
+        w->pend = pm;
+        w->rel = rm;
+        w->took |= tm;
+    }
     __syncwarp();
+    return more;
+}
+
+template <bool RING>
+__device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint32_t njobs, uint32_t quota,
+                                            uint32_t stretch, uint32_t first, uint32_t claimed) {
+    if (lane == 0) {
+        w->n_hit = w->n_big = 0;
+        w->pend = w->rel = w->took = 0;
+        w->njobs = njobs; w->quota = quota; w->stretch = stretch;
+        // the warp's first stretch is its own place in the grid (a short queue needs no atomics, whose turns
+        // on one address took 12 of a small call's 29 us), the later ones are claimed behind them
+        const uint32_t at = min(first * stretch, njobs);
+        w->st_cur = at;
+        w->st_rem = RING ? 0 : min(stretch, njobs - at);
+        w->last = (uint64_t)claimed * stretch >= njobs;
+        w->claimed = claimed * stretch;
+    }
+    if (lane < ICACHE) w->ic[lane].item = NO_ITEM;
+    __syncwarp();
+    while (engine_rounds<RING>(a, w, lane)) rare_work<RING>(a, w);
     if (lane < ICACHE && w->ic[lane].item != NO_ITEM)
         count_global(a, w->ic[lane].item, w->ic[lane].cand, w->ic[lane].sqrt_, w->ic[lane].mdiv);
+    const bool took = w->took != 0;
     __syncwarp();
-    return RING ? __any_sync(FULL, took) : false;
+    return took;
 }
 
 __global__ void __launch_bounds__(EBS, 3) extend_jobs(const __grid_constant__ SearchArgs a) {
