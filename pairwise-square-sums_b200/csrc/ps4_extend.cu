@@ -970,14 +970,6 @@ __device__ __forceinline__ void process_queue(WarpArea *w, uint32_t first, uint3
         }
 }
 
-// The engine loop of one warp.  Linear (RING false): the batch's queue [0, njobs), filled before
-// the launch, taken in stretches of `stretch` 4-sets; the loop ends when it is drained.  RING: the
-// persistent kernel's ring; positions are claimed below q_tail and waited for until published, each
-// finished 4-set's slot is handed back after the round's report, and the loop ends when a claim finds
-// the ring empty and no lane holds a 4-set.  quota: lanes that hold a 4-set (32 unless the queue is too
-// short to fill every warp of the launch; the candidates of few 4-sets are still walked by all
-// lanes).  The first `claimed` stretches belong to the warps in order, this one is number `first`.  Returns
-// whether the warp took any 4-set.
 // Runs rounds until rare_work is due (true), or the queue is drained or an error is raised (false).
 template <bool RING>
 __device__ __forceinline__ bool engine_rounds(const SearchArgs &a, WarpArea *w, int lane) {
@@ -1147,6 +1139,14 @@ __device__ __forceinline__ bool engine_rounds(const SearchArgs &a, WarpArea *w, 
     return more;
 }
 
+// The engine loop of one warp.  Linear (RING false): the batch's queue [0, njobs), filled before
+// the launch, taken in stretches of `stretch` 4-sets; the loop ends when it is drained.  RING: the
+// persistent kernel's ring; positions are claimed below q_tail and waited for until published, each
+// finished 4-set's slot is handed back after the round's report, and the loop ends when a claim finds
+// the ring empty and no lane holds a 4-set.  quota: lanes that hold a 4-set (32 unless the queue is too
+// short to fill every warp of the launch; the candidates of few 4-sets are still walked by all
+// lanes).  The first `claimed` stretches belong to the warps in order, this one is number `first`.  Returns
+// whether the warp took any 4-set.
 template <bool RING>
 __device__ __forceinline__ bool engine_loop(const SearchArgs &a, WarpArea *w, int lane, uint32_t njobs, uint32_t quota,
                                             uint32_t stretch, uint32_t first, uint32_t claimed) {
