@@ -77,6 +77,20 @@ def test_differences_with_a_large_square_vs_oracle(wide, S0):
     assert_stats_equal(r.stats, ost)
 
 
+@pytest.mark.parametrize("kernel,n", [("batched", 33), ("batched", 120000), ("persist", 4000)])
+def test_many_divisor_walks_vs_single_calls(wide, kernel, n):
+    """The same 4-sets for the per-lane walk, one item each: more than 32 per engine warp at 120000 (the walks
+    of several rounds are gathered), of different items, each counted with its own."""
+    S = [S0 * 49999 ** 2 for S0 in (4205, 5785, 6205)]
+    alone = [wide.range(s, s + 1).stats for s in S]
+    lo = [S[i * i % 7 % 3] for i in range(n)]
+    with Search(1 << 44, kernel=kernel) as s:
+        stats, r = s.batch(lo, [x + 1 for x in lo])
+    assert not r.lines
+    for x, st in zip(lo, stats):
+        assert all(st[k] == alone[S.index(x)][k] for k in COUNTERS), x
+
+
 @pytest.mark.parametrize("n", [1, 2, 31, 33, 4736, 4737, 9473])
 @pytest.mark.parametrize("scale", [1, 65537 ** 2])
 def test_triple_counts_and_scales_vs_oracle(wide, n, scale):
