@@ -687,20 +687,31 @@ __device__ __forceinline__ void sort_lists(unsigned char *smem, uint32_t n_is) {
     }
 }
 
-// f(entry) for every entry of a tile's list; four loads in flight per thread (they come from L2)
-template <int NT, class F>
+// f(entry) for the entries o, o + step, .. of one part; four loads in flight per thread (they come from L2)
+template <class F>
+__device__ __forceinline__ void part_entries(const uint64_t *list, uint32_t n, uint32_t o, uint32_t step, F f) {
+    for (; o < n; o += 4 * step) {
+        uint64_t e[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) e[u] = o + u * step < n ? __ldcg(list + o + u * step) : 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (o + u * step < n) f(e[u]);
+    }
+}
+
+// f(entry) for every entry of a tile's list.  SIDE: its parts are read side by side, each by its share of
+// the threads, since the latencies of many short parts add up one by one (eight parts, tile kernel: 2e4 S at
+// 4e11 42 -> 38 us, 2e8 at 1e12 2.73 -> 2.55 ms, 300 narrow subranges 0.91 -> 0.84).  Two parts are long
+// enough one by one, with steps known to the compiler ([1,1e10) 79.5 ms, side by side 80.2).
+template <int NT, bool SIDE, class F>
 __device__ __forceinline__ void for_entries(const uint64_t *list, const uint32_t *list_n, uint32_t parts, uint32_t cap,
                                             F f) {
-    for (uint32_t w = 0; w < parts; w++, list += cap) {
-        const uint32_t n = list_n[w];
-        for (uint32_t o = threadIdx.x; o < n; o += 4 * NT) {
-            uint64_t e[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) e[u] = o + u * NT < n ? __ldcg(list + o + u * NT) : 0;
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (o + u * NT < n) f(e[u]);
-        }
+    if (SIDE) {
+        const uint32_t step = NT >> (__ffs((int)parts) - 1), w = threadIdx.x / step;     // parts: a power of two
+        part_entries(list + w * cap, list_n[w], threadIdx.x - w * step, step, f);
+    } else {
+        for (uint32_t w = 0; w < parts; w++, list += cap) part_entries(list, list_n[w], threadIdx.x, NT, f);
     }
 }
 
@@ -708,7 +719,7 @@ __device__ __forceinline__ void for_entries(const uint64_t *list, const uint32_t
 // tile's representations from scan_group, list_n[w] entries in part w of `parts`, `cap` apart; other
 // CTAs of the cluster may have written them: read through L2) P1 and P3 read the list; without,
 // they scan.  INDEX: P4 also leaves each list's parity index (sort_lists).
-template <int TL, int NT = BS, bool INDEX = false>
+template <int TL, int NT = BS, bool INDEX = false, bool SIDE = false>
 __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0, uint32_t n,
                           const uint64_t *list = nullptr, const uint32_t *list_n = nullptr, uint32_t parts = 0,
                           uint32_t cap = 0) {
@@ -727,7 +738,7 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
     // P1: count, from the list or by scanning
     uint32_t found = 0;
     if (list) {
-        for_entries<NT>(list, list_n, parts, cap, [&](uint64_t e) {
+        for_entries<NT, SIDE>(list, list_n, parts, cap, [&](uint64_t e) {
             const uint32_t i = (uint32_t)e & 0x3FFFu;
             atomicAdd(&cnt32[i >> 1], 1u << ((i & 1) * 16));
             found++;
@@ -803,7 +814,7 @@ __device__ bool tile_reps(const SearchArgs &a, TileShared &ts, unsigned char *sm
     __syncthreads();
     // P3: fill, from the list or by scanning again
     if (list) {
-        for_entries<NT>(list, list_n, parts, cap, [&](uint64_t e) {
+        for_entries<NT, SIDE>(list, list_n, parts, cap, [&](uint64_t e) {
             const uint32_t i = (uint32_t)e & 0x3FFFu, wd = i >> 1, sh = (i & 1) * 16;
             if (!(((volatile uint32_t *)cnt32)[wd] >> sh & SELECTED)) return;
             const uint32_t pos = (atomicAdd(&cnt32[wd], 1u << sh) >> sh) & (SELECTED - 1);

@@ -1,6 +1,6 @@
 // ps4_extend.cu -- the batched search as two persistent kernels per batch of S:
 //
-//   gen_jobs<TL,NT>  tiles of 2^TL S in shared memory (P1-P4 of ps4_device.cuh), then every
+//   gen_jobs<TL,NT,SIDE>  tiles of 2^TL S in shared memory (P1-P4 of ps4_device.cuh), then every
 //                 4-set of the tile (P5: two searches per representation pair give the z intervals)
 //                 is written to a global job queue, each warp into stretches it reserves.
 //                                                                             (s4.c:280-341)
@@ -306,7 +306,7 @@ __device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
 // The tile kernel (RING false) queues what a step finds in the warp's open stretch.  The persistent
 // kernel counts first and reserves the tile's 4-sets at once (the ring's room is waited for), and
 // each 4-set is published after a fence.
-template <int TL, int NT, bool RING>
+template <int TL, int NT, bool RING, bool SIDE>
 __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0,
                                              uint32_t n, uint32_t item, const uint64_t *list,
                                              const uint32_t *list_n, uint32_t parts, uint32_t cap, JobSpan &span,
@@ -318,7 +318,7 @@ __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts
     const bool need_write_pass = !noext || (a.flags & (PS4_F_DUMP4 | PS4_F_VERIFY));
     tile_reset(ts);
     __syncthreads();
-    if (!tile_reps<TL, NT, true>(a, ts, smem, S0, n, list, list_n, parts, cap)) { __syncthreads(); return; }
+    if (!tile_reps<TL, NT, true, SIDE>(a, ts, smem, S0, n, list, list_n, parts, cap)) { __syncthreads(); return; }
     TileView v;
     v.off = (const uint16_t *)(smem + L::OFF_IS_OFF);
     v.k = (const uint16_t *)(smem + L::OFF_IS_K);
@@ -440,7 +440,7 @@ __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned 
         __syncthreads();
         for (uint32_t j = 0; j < ng; j++) {
             const uint64_t S0 = SA + ((uint64_t)j << TL);
-            produce_tile<TL, NT, true>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
+            produce_tile<TL, NT, true, false>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
                                        raw_n[j] <= a.raw_cap ? lists + (size_t)j * a.raw_cap : nullptr, &raw_n[j], 1,
                                        a.raw_cap, span, s_base, s_store);
         }
@@ -454,7 +454,7 @@ __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned 
 // nc-th q and appends what it finds to its part of the tiles' lists -- and then take the tiles one
 // by one from a common counter.  A scan costs ~0.29 sqrt(S) steps however few S it covers, and a
 // narrow call has too few tiles for one CTA each on a scan of its own, so both ends gain from sharing it.
-template <int TL, int NT>
+template <int TL, int NT, bool SIDE>
 __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const __grid_constant__ SearchArgs a) {
     using L = TileLayout<TL>;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const 
             }
             __syncthreads();
             const uint64_t S0 = SA + ((uint64_t)j << TL);
-            produce_tile<TL, NT, false>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
+            produce_tile<TL, NT, false, SIDE>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
                                         s_fit ? lists + (size_t)j * nc * cap : nullptr, s_n, nc, cap, span, s_base,
                                         s_store);
         }
@@ -1296,7 +1296,8 @@ int ext_grid(int num_sms) { return num_sms * 3; }
 template <int TL, int NT>
 static int launch_gen_tl(const SearchArgs &a, int grid, uint32_t cluster, cudaStream_t s) {
     const size_t smem = TileLayout<TL>::OFF_ELIST;       // up to the extension-list area, which it does not use
-    const int e = (int)cudaFuncSetAttribute(gen_jobs<TL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = cluster > 2 ? gen_jobs<TL, NT, true> : gen_jobs<TL, NT, false>;
+    const int e = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -1309,7 +1310,7 @@ static int launch_gen_tl(const SearchArgs &a, int grid, uint32_t cluster, cudaSt
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, gen_jobs<TL, NT>, a);
+    return (int)cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
 // up to this many tiles each has an SM to itself, and CTAs of 1024 threads
@@ -1319,7 +1320,8 @@ constexpr uint64_t FEW_TILES = 128;
 // (34,000 q cost about what a tile of 2^13 S does).
 //  * Cluster: 8 CTAs where scans weigh, i.e. for high S and for calls with few tiles, else 2.  Measured,
 //    tile kernel with 8 / 2 / 1 CTAs: [1,1e10) 98.9 / 80.9 / 80.0 ms; 2e8 S at 1e12 2.79 / 3.05 / 3.82; 3e7 S at
-//    1.2e13 1.05 / 1.65 / 2.45; 64 subranges below 1e11 10.3 / 9.0 / 9.3; 2e4 S at 4e11 0.042 / 0.066 / 0.096.
+//    1.2e13 1.05 / 1.65 / 2.45; 64 subranges below 1e11 10.3 / 9.0 / 9.3; 2e4 S at 4e11 0.042 / 0.066 / 0.096
+//    (all with parts read one by one; side by side, as eight are now, 2.57, 0.99 and 0.040 at 1e12, 1.2e13 and 4e11).
 //  * Tiles per claim: n tiles in groups of G on K clusters take n + s n / G of work and about G K / 2 of
 //    idling at the end, least at G = sqrt(2 n s / K).
 // `grid`: the CTAs that the lists of a.raw are sized for; whole clusters of them are launched, no more
