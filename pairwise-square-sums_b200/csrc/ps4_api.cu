@@ -115,6 +115,8 @@ static int set_err(ps4_ctx *c, int code, const char *fmt, ...) {
             return set_err(ctx, PS4_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(_e));      \
     } while (0)
 
+// A device buffer of at least `need` elements.  One that cannot be had leaves nothing behind: no buffer, no
+// capacity, no error for the next launch's check to find.
 template <class T>
 static int grow(ps4_ctx *c, T *&ptr, uint64_t &cap, uint64_t need) {
     if (need <= cap && ptr) return 0;
@@ -122,7 +124,13 @@ static int grow(ps4_ctx *c, T *&ptr, uint64_t &cap, uint64_t need) {
     ptr = nullptr;
     cap = 0;
     if (need == 0) return 0;
-    CUDA_TRY(c, cudaMalloc((void **)&ptr, need * sizeof(T)));
+    const cudaError_t e = cudaMalloc((void **)&ptr, need * sizeof(T));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
+        return set_err(c, PS4_ERR_CUDA, "no device buffer of %llu x %zu bytes: %s", (unsigned long long)need, sizeof(T),
+                       cudaGetErrorString(e));
+    }
     cap = need;
     return 0;
 }
@@ -459,7 +467,10 @@ static int enqueue_items(ps4_ctx *c) {
     if (reserve_stage(c, (small ? blk : 0) + segs_bytes)) return PS4_ERR_CUDA;
     Item *const dev_items = small ? reinterpret_cast<Item *>(c->d_block + blk) : c->d_items;
     if (kernel == PS4_KERNEL_BATCHED && c->d_jobs_words < 6 * c->jobs_cap)
-        if (grow(c, c->d_jobs, c->d_jobs_words, 6 * c->jobs_cap)) return PS4_ERR_CUDA;
+        if (grow(c, c->d_jobs, c->d_jobs_words, 6 * c->jobs_cap)) {
+            c->jobs_cap = 1ull << 20;                  // later calls ask for what they need themselves
+            return PS4_ERR_CUDA;
+        }
     // gen_ctas counts 512 threads per SM: one or two 512-thread CTAs on 2^14-S tiles, twice as
     // many 256-thread ones on smaller tiles; a narrow call needs no more CTAs (nor lists for them)
     // than it has tiles
@@ -1018,9 +1029,16 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
     const uint64_t off_out = (off_state + n + 15) & ~15ull;
     const uint64_t head = off_out - off_cnt + FIRST * sizeof(ps4_tri_ext);
     const bool few = off_cnt + 32 <= PIN_HALF && head <= PIN_HALF;
-    c->tri_out_cap = std::max<uint64_t>(c->tri_out_cap, std::max<uint64_t>(out_cap, 1u << 16));
-    auto reserve = [&]() {
-        return grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, off_out + c->tri_out_cap * sizeof(ps4_tri_ext)));
+    uint64_t want = std::max<uint64_t>(c->tri_out_cap, std::max<uint64_t>(out_cap, 1u << 16));
+    // room for `want` records, kept only once the block is there: a call that asks for too much fails alone
+    auto reserve = [&]() -> int {
+        c->tri_out_cap = 0;
+        if (want >= 1ull << 48)                        // no sum below leaves 64 bits
+            return set_err(c, PS4_ERR_CUDA, "no device buffer of %llu triple records", (unsigned long long)want);
+        if (grow(c, c->d_tri, c->tri_cap, std::max<uint64_t>(c->tri_cap, off_out + want * sizeof(ps4_tri_ext))))
+            return PS4_ERR_CUDA;
+        c->tri_out_cap = want;
+        return PS4_OK;
     };
     unsigned char *const land = c->h_pin + PIN_HALF;
     std::vector<uint8_t> st_buf(few ? 0 : n);
@@ -1066,7 +1084,7 @@ extern "C" int ps4_extend_triples(ps4_ctx *c, const uint64_t *abc, uint32_t n, u
         if (cnt[0] <= c->tri_out_cap) break;
         // more records than the device buffer holds: grow it and run again (results do not
         // depend on the buffer)
-        c->tri_out_cap = cnt[0] * 3 / 2 + 1024;
+        want = cnt[0] * 3 / 2 + 1024;
     }
     const uint64_t n_rec = cnt[0], first = std::min<uint64_t>(n_rec, FIRST);
     std::vector<ps4_tri_ext> recs(n_rec);
