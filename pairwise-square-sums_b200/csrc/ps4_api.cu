@@ -259,6 +259,9 @@ extern "C" int ps4_create(const ps4_config *cfg, ps4_ctx **out) {
     CUDA_TRY(c, cudaMalloc((void **)&c->d_spfq, c->tab_n * sizeof(uint64_t)));
     CUDA_TRY(c, cudaMalloc((void **)&c->d_ndiv, c->tab_n * sizeof(uint16_t)));
     CUDA_TRY(c, cudaMallocHost((void **)&c->h_pin, 2 * PIN_HALF));
+    // the block of small calls, and with it the 2 MiB that the driver cuts small buffers from: mapping those took
+    // most of a context's first call (50 triples 0.54 -> 0.15 ms, 2e4 S at 4e11 1.85 -> 1.60 ms)
+    if (reserve_block(c, SMALL_ITEMS)) return PS4_ERR_CUDA;
     CUDA_TRY(c, (cudaError_t)launch_tables(c->d_spfq, c->d_ndiv, c->tab_n, c->stream));
     CUDA_TRY(c, cudaMalloc((void **)&c->d_fac, fac_n(c->tab_n) * sizeof(uint4)));
     CUDA_TRY(c, (cudaError_t)launch_fac(c->d_fac, fac_n(c->tab_n), c->stream));
