@@ -517,7 +517,7 @@ static int enqueue_items(ps4_ctx *c) {
     a.flags = c->cfg.flags & (p.dump ? ~0u : ~(uint32_t)PS4_F_DUMP4);
     a.jobs = c->d_jobs;
     a.jobs_cap = c->jobs_cap;
-    if (kernel == PS4_KERNEL_BATCHED) { a.raw = c->d_raw; a.raw_cap = raw_cap_for(TL); }
+    if (kernel == PS4_KERNEL_BATCHED) { a.raw = c->d_raw; a.raw_cap = raw_cap_for(TL); a.raw_lists = SUPER_K; }
     if (persist) {
         a.jobs_cap = c->ring_cap;
         a.seq = c->d_seq;

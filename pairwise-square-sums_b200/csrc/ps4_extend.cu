@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const 
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), nc = cluster.num_blocks();
     const uint32_t cap = a.raw_cap / nc;
-    uint64_t *lists = a.raw + (size_t)(blockIdx.x / nc) * nc * SUPER_K * a.raw_cap;
+    uint64_t *lists = a.raw + (size_t)(blockIdx.x / nc) * nc * a.raw_lists * a.raw_cap;
     for (uint32_t i = tid; i < GEN_CLUSTER * SUPER_K; i += NT) raw_n[0][i] = 0;
     if (tid == 0) s_take[0] = 0;
     uint64_t ti = 0, ti_end = 0;
@@ -1334,7 +1334,7 @@ int launch_gen(SearchArgs a, int grid, void *stream) {
     const uint64_t fit = std::max<uint64_t>((uint64_t)grid / cl, 1), want = ((uint64_t)n + cl - 1) / cl;
     const uint64_t K = std::min(fit, want), ctas = K * cl;
     const double G = std::min(std::sqrt(2 * n * scan / (double)K), std::ceil(n / (double)K));
-    a.group = (uint32_t)std::min<double>(std::max<double>(G, cl), cl * SUPER_K);
+    a.group = (uint32_t)std::min<double>(std::max<double>(G, cl), cl * a.raw_lists);
     // a warp's reservations: a sixteenth of its expected share of about 0.2 4-sets per S, so that the
     // empty records at the end stay below a few percent, 128 at most (one atomic per 128 4-sets)
     const bool few = a.log2_tile == 12 && a.n_tiles <= FEW_TILES;

@@ -82,8 +82,9 @@ struct SearchArgs {
     uint32_t flags;            // PS4_F_*
     uint32_t *jobs;            // 4-set job queue between gen_jobs and extend_jobs: jobs_cap 24-byte records
     uint64_t jobs_cap;
-    uint64_t *raw;             // tile and persistent kernel: per CTA, SUPER_K lists of one tile's
+    uint64_t *raw;             // tile and persistent kernel: per CTA, raw_lists lists of one tile's
     uint32_t raw_cap;          //   representations, raw_cap entries each (a cluster pools its CTAs' lists)
+    uint32_t raw_lists;        // SUPER_K at most (the persistent kernel always has SUPER_K)
     uint64_t s_top;            // the launch's largest S, for the tile kernel's launch shape
     uint32_t group;            // tile kernel: tiles a cluster claims at once, and job records a warp
     uint32_t chunk;            //   reserves at once (both set by launch_gen)
@@ -105,7 +106,7 @@ constexpr uint32_t RAW_PER_TILE = 10240;
 constexpr uint32_t raw_cap_for(unsigned TL) { return RAW_PER_TILE >> (14 - TL); }
 // tile lists per CTA of the tile and the persistent kernel (592 CTAs x 16 x 40 KB = 388 MB): a
 // cluster of the tile kernel scans up to GEN_CLUSTER * SUPER_K adjacent tiles as one range, a
-// CTA of the persistent kernel SUPER_K
+// CTA of the persistent kernel SUPER_K (a server's have fewer)
 constexpr uint32_t SUPER_K = 16;
 // CTAs of a tile-kernel cluster (the portable maximum)
 constexpr uint32_t GEN_CLUSTER = 8;

@@ -256,6 +256,15 @@ struct StepBuf {
     cudaEvent_t ev_start = nullptr, ev_kern = nullptr, ev_post = nullptr, ev_fork = nullptr, ev_join = nullptr;
 };
 
+// The tile lists of a server, in entries: 310 MB, what the budgets that servers are opened with leave room for.
+// On 2^13-S tiles a CTA of the full grid then has 12 of SUPER_K lists, on smaller ones all.  (Full steps take about 8
+// tiles per CTA near 1e12.  SUPER_K lists of 4/5 the entries overflow often enough to cost 4 % of a burst of 150.)
+uint64_t serve_raw_words(int num_sms) { return (uint64_t)gen_grid(num_sms, 14) * SUPER_K * 8192; }
+uint32_t serve_lists(int num_sms, unsigned TL) {
+    const uint64_t per_list = (uint64_t)gen_grid(num_sms, TL) * raw_cap_for(TL);
+    return (uint32_t)std::min<uint64_t>(SUPER_K, serve_raw_words(num_sms) / per_list);
+}
+
 const uint32_t RANGE_SIXES = 16;
 const uint32_t TRI_RECS = 64;
 
@@ -268,7 +277,7 @@ struct ps4_server {
     cudaStream_t s_main = nullptr, s_tri = nullptr, s_post = nullptr, s_copy = nullptr;
     uint32_t *d_jobs = nullptr;
     uint64_t jobs_cap = 0;
-    uint64_t *d_raw = nullptr;               // per tile-kernel CTA representation lists
+    uint64_t *d_raw = nullptr;               // the tile-kernel CTAs' representation lists
     uint32_t *d_scratch = nullptr;
     uint64_t scratch_words = 0;
     SlotDev *d_slots = nullptr;
@@ -599,7 +608,7 @@ int launch_step(ps4_server *s, StepBuf &b) {
         a.flags = s->v.flags & ~(uint32_t)PS4_F_DUMP4;
         a.jobs = s->d_jobs; a.jobs_cap = s->jobs_cap;
         if (!b.fused) {
-            a.raw = s->d_raw; a.raw_cap = raw_cap_for(TL);
+            a.raw = s->d_raw; a.raw_cap = raw_cap_for(TL); a.raw_lists = serve_lists(s->v.num_sms, TL);
             a.s_top = s_top;
             SRV_CUDA(s, (cudaError_t)launch_gen(a, gen_grid(s->v.num_sms, TL), st));
             if (!(s->v.flags & PS4_F_NOEXT)) SRV_CUDA(s, (cudaError_t)launch_ext(a, ext_grid(s->v.num_sms), st));
@@ -948,8 +957,8 @@ extern "C" int ps4_serve_create(ps4_ctx *ctx, const ps4_serve_config *cfg, ps4_s
     s->jobs_cap = 1ull << 20;
     while (s->jobs_cap < (1ull << 27) && (double)s->jobs_cap < need) s->jobs_cap <<= 1;
     if (dev_alloc(s, s->d_jobs, 6 * s->jobs_cap)) return PS4_ERR_CUDA;
-    // lists for the tile kernel's full residency at any tile size (the same bytes at every size)
-    if (dev_alloc(s, s->d_raw, (uint64_t)gen_grid(s->v.num_sms, 14) * SUPER_K * RAW_PER_TILE)) return PS4_ERR_CUDA;
+    // lists for the tile kernel's full residency at any tile size
+    if (dev_alloc(s, s->d_raw, serve_raw_words(s->v.num_sms))) return PS4_ERR_CUDA;
     if (dev_alloc(s, s->d_slots, c.max_slots)) return PS4_ERR_CUDA;
     for (int i = 0; i < 2; i++)
         if (init_buf(s, s->buf[i])) return PS4_ERR_CUDA;

@@ -9,8 +9,10 @@ import ctypes as C
 import numpy as np
 import pytest
 
+from conftest import assert_stats_equal
 from oracle import orc
 from ps4b200 import Search, _abi, workloads
+from ps4b200.serve import Server
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +39,23 @@ def test_too_much_room_for_triples_fails_alone(room):
                 got[r.item].append(r.d)
             assert got == want
         assert s.range(10 ** 9, 10 ** 9 + 10 ** 5).stats["S_done"] == 10 ** 5
+
+
+# A server's buffers besides its arena: 24 bytes for each of 2^20 queued 4-sets, 310 MB of tile lists, 6 MB of
+# step buffers and 16 MB of arena at least.
+@pytest.mark.parametrize("budget", [364 << 20, 512 << 20])
+def test_server_on_a_small_budget(budget):
+    ranges = [(10 ** 9, 10 ** 9 + 3 * 10 ** 5), (10 ** 12 - 70001, 10 ** 12), (1, 4097)]
+    with Search(2 * 10 ** 12) as s:
+        with Server(s, hbm_budget=budget, max_slots=4, max_step_items=64, step_S=1 << 20, max_step_triples=16) as srv:
+            assert srv.info()["device_bytes"] <= budget
+            for i, (lo, hi) in enumerate(ranges):
+                srv.submit_range(i, lo, hi)
+            done = []
+            while len(done) < len(ranges):
+                done += srv.progress(100000)
+            got = [srv.take_range(i) for i in range(len(ranges))]
+        for (lo, hi), r in zip(ranges, got):
+            want = s.range(lo, hi)
+            assert r.lines == want.lines
+            assert_stats_equal(r.stats, want.stats)
