@@ -230,6 +230,13 @@ int ps4_check_roots(int device, const uint64_t *lo, const uint64_t *hi, uint32_t
  * and frees its own small device buffers on `device`; synchronous. */
 int ps4_check_ring_wait(int device, uint64_t *waited_ns);
 
+/* Self-check of the tile kernel's walk over the representation pairs of a tile's lists, 32 at a time:
+ * first[i] (i < n, ascending from 0) is the number of pairs before list i, first[n] <= 2^24 that of
+ * all.  owner[g] = the list of pair g in the low half, that list's first pair in the high one.  No
+ * counterpart in the reference (it loops over one S's pairs at a time, s4.c:313-341).  Allocates and
+ * frees its own device buffers on `device`; synchronous. */
+int ps4_check_pair_owners(int device, const uint32_t *first, uint32_t n, uint64_t *owner);
+
 /* ---- triple extension ----
  *
  * For each triple {a, b, c} of distinct positive integers whose three pairwise sums are

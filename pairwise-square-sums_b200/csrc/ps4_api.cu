@@ -911,6 +911,28 @@ extern "C" int ps4_check_ring_wait(int device, uint64_t *waited_ns) {
     return rc;
 }
 
+// ---- self-check of the tile kernel's walk over the representation pairs ----
+
+extern "C" int ps4_check_pair_owners(int device, const uint32_t *first, uint32_t n, uint64_t *owner) {
+    if (!first || !owner || n == 0 || first[0] != 0) return PS4_ERR_ARG;
+    for (uint32_t i = 0; i < n; i++)
+        if (first[i + 1] <= first[i] || first[i + 1] > 1u << 24) return PS4_ERR_ARG;
+    const size_t total = first[n];
+    int prev = 0;
+    if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return PS4_ERR_CUDA;
+    uint32_t *d_first = nullptr;
+    unsigned long long *d_out = nullptr;
+    cudaError_t e = cudaMalloc((void **)&d_first, ((size_t)n + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&d_out, total * sizeof(uint64_t));
+    if (e == cudaSuccess) e = cudaMemcpy(d_first, first, ((size_t)n + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = (cudaError_t)launch_pair_owner_probe(d_first, n, d_out);
+    if (e == cudaSuccess) e = cudaMemcpy(owner, d_out, total * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+    cudaFree(d_first);
+    cudaFree(d_out);
+    if (prev != device) cudaSetDevice(prev);
+    return e == cudaSuccess ? PS4_OK : PS4_ERR_CUDA;
+}
+
 // ---- tuning ----
 
 extern "C" int ps4_set_tuning(ps4_ctx *c, const ps4_tuning *t) {

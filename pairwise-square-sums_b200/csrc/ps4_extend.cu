@@ -189,20 +189,28 @@ struct PairSets {
     uint32_t ab;                       // first z of class 0 | of class 1 << 16, as places in the parity index
 };
 
+// The selected S of the pairs g0 + lane, as its place `lo` in the list and its first pair `base` (lanes past the last
+// pair get the last S).  pbase[lo]: pairs before the S at lo, n_is of them and the total.  lo0, warp-uniform:
+// the S of pair g0; moved on to pair g0 + 32's.  Every selected S has a pair at least, so 32 consecutive
+// pairs lie in 32 consecutive S from the first one's.
+__device__ __forceinline__ void pair_owner(const uint32_t *pbase, uint32_t n_is, uint32_t g0, int lane, uint32_t &lo0,
+                                           uint32_t &lo, uint32_t &base) {
+    const uint32_t pb = lo0 + lane < n_is ? pbase[lo0 + lane] : 0xFFFFFFFFu;
+    const uint32_t rel = pb - g0;                          // starts behind the first pair, as a bit mask
+    const unsigned starts = __reduce_or_sync(0xffffffffu, rel - 1u < 31u ? 1u << rel : 0u);
+    const uint32_t o = __popc(starts & (0xFFFFFFFFu >> (31 - lane)));
+    base = __shfl_sync(0xffffffffu, pb, o);
+    lo = lo0 + o;
+    lo0 += __popc(starts);
+    if (pbase[lo0 + 1] <= g0 + 32) lo0++;                  // its pairs end with this step
+}
+
 // The pairs g of a warp, one per lane (32 consecutive ones; ge ends the warp's block): each lane's
-// number of 4-sets and where they are.  lo0: a selected S not after the first pair's, warp-uniform;
-// moved on to the last one's.
+// number of 4-sets and where they are.  lo0: as for pair_owner.
 __device__ __forceinline__ uint32_t pair_sets(const TileView &v, uint64_t S0, uint32_t g, uint32_t ge, int lane,
                                               uint32_t &lo0, PairSets &ps) {
-    // every selected S has a pair at least, so 32 consecutive pairs lie in 32 consecutive ones
-    const uint32_t pb = lo0 + lane < v.n_is ? v.pbase[lo0 + lane] : 0xFFFFFFFFu;
-    const uint32_t rel = pb - (g - lane);                  // starts behind the first pair, as a bit mask
-    const unsigned upto = __popc(__ballot_sync(0xffffffffu, pb <= g - lane));
-    const unsigned starts = __reduce_or_sync(0xffffffffu, rel - 1u < 31u ? 1u << rel : 0u);
-    const uint32_t o = upto + __popc(starts & (0xFFFFFFFFu >> (31 - lane))) - 1;
-    const uint32_t base = __shfl_sync(0xffffffffu, pb, o);
-    const uint32_t lo = lo0 + o;
-    lo0 += upto + __popc(starts) - 1;
+    uint32_t lo, base;
+    pair_owner(v.pbase, v.n_is, g - lane, lane, lo0, lo, base);
     if (g >= ge) return 0;
     const uint32_t st = v.start[lo], k = v.k[lo];
     const uint64_t S = S0 + v.off[lo];
@@ -1281,6 +1289,16 @@ __global__ void ring_wait_probe(const SearchArgs a, unsigned long long *out) {
     out[1] = gtimer() - t0;
 }
 
+// The owners of all pairs, as one warp of the tile kernel finds them (ps4_check_pair_owners).
+__global__ void pair_owner_probe(const uint32_t *pbase, uint32_t n_is, unsigned long long *out) {
+    const uint32_t total = pbase[n_is];
+    uint32_t lo0 = 0, lo, base;
+    for (uint32_t g = 0; g < total; g += 32) {
+        pair_owner(pbase, n_is, g, threadIdx.x, lo0, lo, base);
+        if (g + threadIdx.x < total) out[g + threadIdx.x] = (ull)base << 32 | lo;
+    }
+}
+
 // seq[i] = i: every slot free for its first lap
 __global__ void ring_init(uint32_t *seq, uint64_t n) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
@@ -1371,6 +1389,11 @@ int launch_persist(const SearchArgs &a, int grid, void *stream) {
 
 int launch_ring_wait_probe(const SearchArgs &a, unsigned long long *out, void *stream) {
     ring_wait_probe<<<1, 1, 0, (cudaStream_t)stream>>>(a, out);
+    return (int)cudaGetLastError();
+}
+
+int launch_pair_owner_probe(const uint32_t *pbase, uint32_t n_is, unsigned long long *out) {
+    pair_owner_probe<<<1, 32>>>(pbase, n_is, out);
     return (int)cudaGetLastError();
 }
 

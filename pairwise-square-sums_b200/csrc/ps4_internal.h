@@ -172,6 +172,7 @@ int launch_ext(const SearchArgs &a, int grid, void *stream);
 // the persistent kernel (ps4_extend.cu): tiles of 2^13 S, ring of a.jobs_cap slots
 int launch_persist(const SearchArgs &a, int grid, void *stream);
 int launch_ring_init(uint32_t *seq, uint64_t n, void *stream);
+int launch_pair_owner_probe(const uint32_t *pbase, uint32_t n_is, unsigned long long *out);
 int launch_ring_wait_probe(const SearchArgs &a, unsigned long long *out, void *stream);
 int persist_ctas_per_sm();
 int gen_grid(int num_sms, unsigned TL);      // the tile kernel's full residency for 2^TL-S tiles
