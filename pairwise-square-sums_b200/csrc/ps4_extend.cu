@@ -554,9 +554,9 @@ struct __align__(16) EJob {              // one lane's 4-set
     int64_t d1, d2;                      // C - A of the other two members (square tests of u^2 + (C - A))
     uint32_t rA0, rA1, rA2;              // the roots sqrt(A + v) of the three other members: e is one of
                                          //   them iff u is one of these
-    uint32_t item;                       // | ext_sqrt << 20 where the round's items differ (a 4-set has
-                                         //   fewer than 2^12 candidates: no number below 2^44 has 2^14 divisors)
-    uint32_t pad[4];                     // 80 bytes: vector accesses of eight jobs meet no bank twice (64
+    uint32_t item;
+    uint32_t nsq;                        // ext_sqrt, where the round's items differ
+    uint32_t pad[3];                     // 80 bytes: vector accesses of eight jobs meet no bank twice (64
                                          //   bytes: engine 189.3 -> 182.7 ms per [1,1e10) search)
 };
 static_assert(sizeof(EJob) == 80 && offsetof(EJob, d1) == 32 && offsetof(EJob, rA0) == 48, "vector loads of job fields");
@@ -811,6 +811,7 @@ __device__ __forceinline__ bool job_setup(const SearchArgs &a, uint64_t j, LaneJ
         E.rA1 = bi == 0 ? r[1] : bi == 3 ? r[4] : r[3];
         E.rA2 = bi == 0 ? r[2] : bi == 1 ? r[4] : r[5];
         E.item = J.item;
+        E.nsq = 0;
         uint32_t m64 = 0xFFFFFFFFu;
         uint64_t m63 = ~0ull, m65 = ~0ull;
         and_masks(d1, m64, m63, m65);
@@ -959,9 +960,9 @@ __device__ __forceinline__ void process_queue(WarpArea *w, uint32_t first, uint3
         // u below 2^32: e > 0 iff u2 > A; e = A iff u2 = 2A; e another member iff u one of A's roots
         const bool test = at < count && ((u[k] >> 32) != 0 || (u2[k] > A && u2[k] != 2 * A && ul != ro.x &&
                                                                ul != ro.y && ul != ro.z));
-        const bool here = (ro.w & 0xFFFFFu) == cnt.item;
+        const bool here = ro.w == cnt.item;
         cnt.sqrt_ += test && here;
-        if (test && !here) atomicAdd(&w->job[jl[k]].item, 1u << 20);
+        if (test && !here) atomicAdd(&w->job[jl[k]].nsq, 1u);
         hit[k] = is_square_near(u[k], d1, u2[k] + (uint64_t)d1) && test;
     }
 #pragma unroll
@@ -1121,8 +1122,8 @@ __device__ __forceinline__ bool engine_rounds(const SearchArgs &a, WarpArea *w, 
                 }
             }
             const uint32_t it = w->job[lane].item;
-            const bool other = fits && (it & 0xFFFFFu) != cnt.item;      // counted with its 4-set
-            if (__any_sync(FULL, other)) cnt.add(a, w, lane, other, it & 0xFFFFFu, 0, it >> 20, 0);
+            const bool other = fits && it != cnt.item;                   // counted with its 4-set
+            if (__any_sync(FULL, other)) cnt.add(a, w, lane, other, it, 0, w->job[lane].nsq, 0);
             if (fits) pending = false;
             if (RING && fits) rel = true;
         }
