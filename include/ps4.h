@@ -147,8 +147,8 @@ int ps4_search_range(ps4_ctx *ctx, uint64_t lo, uint64_t hi, ps4_stats *stats, p
 
 /* Many independent subranges [lo[i], hi[i]) in ONE persistent launch (the block controller's
  * sequence of s4 invocations, run_exhaustive.py:200-238, done as one device batch).  stats
- * points at n_items ps4_stats (+=); every hit carries its item index.  Subranges may overlap;
- * each is searched in full. */
+ * points at n_items (2^30 at most, 1 KB of device memory each) ps4_stats (+=); every hit carries
+ * its item index.  Subranges may overlap; each is searched in full. */
 int ps4_search_batch(ps4_ctx *ctx, const uint64_t *lo, const uint64_t *hi, uint32_t n_items,
                      ps4_stats *stats, ps4_results *res);
 

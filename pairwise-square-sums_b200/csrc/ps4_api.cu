@@ -640,6 +640,8 @@ static int enqueue_items(ps4_ctx *c) {
 static int begin_items(ps4_ctx *c, const uint64_t *lo, const uint64_t *hi, uint32_t n_items, bool want_dump,
                        uint64_t dump_cap) {
     if (c->pend.active) return set_err(c, PS4_ERR_ARG, "a search is already enqueued on this context");
+    if (n_items > MAX_ITEMS)
+        return set_err(c, PS4_ERR_ARG, "%u subranges in one call, %u at most", n_items, MAX_ITEMS);
     PendingSearch &p = c->pend;
     p.items.assign(n_items, Item{});
     c->fused_fallback = false;

@@ -43,12 +43,12 @@ namespace ps4 {
 
 // A queued 4-set: its six pair roots (< 2^22), one 24-byte record per 4-set (three 8-byte
 // stores and loads; six u32 arrays took 2.2 % more tile-kernel and 1.2 % more engine time per
-// [1,1e10) step).  The query item id (< 2^20) rides in the spare top bits of r_ac (bits 0..9
-// of the id) and r_ad (bits 10..19).  The queue of cap records is 6 * cap u32.
+// [1,1e10) step).  The query item id (< 2^30, MAX_ITEMS) rides in the spare top bits of r_ac (bits 0..9
+// of the id), r_ad (bits 10..19) and r_bc (bits 20..29).  The queue of cap records is 6 * cap u32.
 __device__ __forceinline__ void put_job(uint32_t *jobs, uint64_t j, const uint32_t r[6], uint32_t item) {
     uint2 *p = (uint2 *)(jobs + 6 * j);               // 8-byte aligned: 24 * j
-    p[0] = make_uint2(r[0], r[1] | ((item & 1023u) << 22));
-    p[1] = make_uint2(r[2] | (((item >> 10) & 1023u) << 22), r[3]);
+    p[0] = make_uint2(r[0], r[1] | item << 22);
+    p[1] = make_uint2(r[2] | item >> 10 << 22, r[3] | item >> 20 << 22);
     p[2] = make_uint2(r[4], r[5]);
 }
 
@@ -59,14 +59,13 @@ __device__ __forceinline__ void get_job(const uint32_t *jobs, uint64_t j, uint32
     const uint2 *p = (const uint2 *)(jobs + 6 * j);
     const uint2 x = COH ? __ldcg(p) : __ldg(p), y = COH ? __ldcg(p + 1) : __ldg(p + 1),
                 z = COH ? __ldcg(p + 2) : __ldg(p + 2);
-    const uint32_t w1 = x.y, w2 = y.x;
     r[0] = x.x;
-    r[1] = w1 & 0x3FFFFFu;
-    r[2] = w2 & 0x3FFFFFu;
-    r[3] = y.y;
+    r[1] = x.y & 0x3FFFFFu;
+    r[2] = y.x & 0x3FFFFFu;
+    r[3] = y.y & 0x3FFFFFu;
     r[4] = z.x;
     r[5] = z.y;
-    item = (w1 >> 22) | ((w2 >> 22) << 10);
+    item = x.y >> 22 | y.x >> 22 << 10 | y.y >> 22 << 20;
 }
 
 // ================================================================== the persistent kernel's ring

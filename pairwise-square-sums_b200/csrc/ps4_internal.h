@@ -41,6 +41,9 @@ struct Item {
     uint32_t pad;
 };
 
+// items of one call at most: a queued 4-set carries its item's id in 30 bits
+constexpr uint32_t MAX_ITEMS = 1u << 30;
+
 // Status block copied back after every launch.
 struct Status {
     unsigned long long err;        // first error (code | S << 8)

@@ -59,3 +59,27 @@ def test_server_on_a_small_budget(budget):
             want = s.range(lo, hi)
             assert r.lines == want.lines
             assert_stats_equal(r.stats, want.stats)
+
+
+def test_more_than_a_million_items():
+    """Items on both sides of 2^20, the others empty: every counter and hit with its own item."""
+    n = (1 << 20) + 8
+    ranges = {3: (10 ** 9, 10 ** 9 + 400000), 7: (10 ** 6, 10 ** 6 + 5000), (1 << 20) - 1: (5, 900),
+              1 << 20: (10 ** 5, 2 * 10 ** 5), (1 << 20) + 3: (15 * 10 ** 8, 15 * 10 ** 8 + 500000),
+              (1 << 20) + 7: (1, 70000)}
+    lo, hi = np.ones(n, dtype=np.uint64), np.ones(n, dtype=np.uint64)
+    for i, (a, b) in ranges.items():
+        lo[i], hi[i] = a, b
+    as_u64 = C.POINTER(C.c_uint64)
+    with Search(2 * 10 ** 9) as s:
+        alone = {i: s.range(a, b) for i, (a, b) in ranges.items()}
+        stats = (_abi.Stats * n)()
+        res = s._res
+        assert s.lib.ps4_search_batch(s.ctx, lo.ctypes.data_as(as_u64), hi.ctypes.data_as(as_u64), n, stats,
+                                      C.byref(res)) == _abi.PS4_OK
+        for i, r in alone.items():
+            assert_stats_equal(stats[i].as_dict(), r.stats, label=f"item {i}")
+        got = [res.hits[k].item for k in range(res.n_hits)]
+        assert sorted(set(got)) == [i for i in sorted(alone) if alone[i].lines]
+        other = np.frombuffer(stats, dtype=np.uint64).reshape(n, -1)
+        assert sorted(np.flatnonzero(other.any(axis=1))) == sorted(ranges)
