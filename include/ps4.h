@@ -237,6 +237,19 @@ int ps4_check_ring_wait(int device, uint64_t *waited_ns);
  * frees its own device buffers on `device`; synchronous. */
 int ps4_check_pair_owners(int device, const uint32_t *first, uint32_t n, uint64_t *owner);
 
+/* Self-check of the re-runs.  A search is repeated -- with other tiles, narrower batches or the fused
+ * kernel -- when one of its fixed lists or its queue of 4-sets was too small, which no known interval makes
+ * them.  This makes it happen: the context's next `attempts` attempts at a search (and steps of servers on
+ * it) run with tile lists of at most `list` entries and a queue of at most `queue` 4-sets (0: as ever), and
+ * one that then ends without an error is taken to have ended with `code` (0, or a PS4_RERUN_* code).
+ * Results do not depend on it.  No counterpart in the reference (its lists have one size, s4.c:46-52). */
+enum { PS4_RERUN_TILE = 100,       /* a tile outgrew its lists                                      */
+       PS4_RERUN_EXTLIST = 101,    /* more extensions at once than a list of them holds              */
+       PS4_RERUN_QUEUE = 102 };    /* a batch's 4-sets outgrew the queue                             */
+int ps4_check_reruns(ps4_ctx *ctx, uint32_t attempts, uint32_t list, uint64_t queue, uint32_t code);
+/* Attempts that the last search call took, and the S per tile (log2) of the last one. */
+void ps4_last_attempts(const ps4_ctx *ctx, uint32_t *attempts, uint32_t *log2_tile);
+
 /* ---- triple extension ----
  *
  * For each triple {a, b, c} of distinct positive integers whose three pairwise sums are

@@ -74,6 +74,8 @@ struct ps4_ctx {
     uint64_t seq_cap = 0;                //   4-sets use d_jobs with ring_cap entries
     uint64_t ring_cap = 1ull << 26;
     uint64_t h2d_bytes = 0, d2h_bytes = 0;
+    uint32_t attempts = 0;               // attempts at the search at hand
+    Drill drill = {}, drill_now = {};    // ps4_check_reruns: asked for, and of the attempt in flight
     // tuning (ps4_autotune / ps4_set_tuning)
     uint32_t gen_ctas = 2, ext_ctas = 3;     // per SM: tile-kernel threads in units of 512 / engine CTAs
     uint64_t jobs_cap_max = 1ull << 29;      // largest job queue (entries; 2^29 = 12.9 GB): fewer,
@@ -97,6 +99,12 @@ struct ps4_ctx {
     uint64_t tri_out_cap = 0;                                        // records the device block holds
     std::string err;
 };
+
+Drill ps4::ctx_drill(ps4_ctx *c) {
+    if (!c->drill.attempts) return Drill{};
+    c->drill.attempts--;
+    return c->drill;
+}
 
 static int set_err(ps4_ctx *c, int code, const char *fmt, ...) {
     char buf[512];
@@ -407,6 +415,8 @@ static void key_add(std::string &k, const T &v) {
 static int enqueue_items(ps4_ctx *c) {
     PendingSearch &p = c->pend;
     const uint32_t n_items = (uint32_t)p.items.size();
+    c->attempts++;
+    c->drill_now = ctx_drill(c);
     int kernel = c->fused_fallback ? (int)PS4_KERNEL_FUSED : (int)c->cfg.kernel;
     if (kernel == PS4_KERNEL_PERSIST && c->persist_fallback) kernel = PS4_KERNEL_BATCHED;
     const bool persist = kernel == PS4_KERNEL_PERSIST;
@@ -516,8 +526,12 @@ static int enqueue_items(ps4_ctx *c) {
     a.cap_reps = c->cfg.cap_reps; a.cap_divs = c->cfg.cap_divs; a.cap_ext = c->cfg.cap_ext;
     a.flags = c->cfg.flags & (p.dump ? ~0u : ~(uint32_t)PS4_F_DUMP4);
     a.jobs = c->d_jobs;
-    a.jobs_cap = c->jobs_cap;
-    if (kernel == PS4_KERNEL_BATCHED) { a.raw = c->d_raw; a.raw_cap = raw_cap_for(TL); a.raw_lists = SUPER_K; }
+    a.jobs_cap = c->drill_now.queue_cap(c->jobs_cap);
+    if (kernel == PS4_KERNEL_BATCHED) {
+        a.raw = c->d_raw;
+        a.raw_cap = c->drill_now.list_cap(raw_cap_for(TL));
+        a.raw_lists = SUPER_K;
+    }
     if (persist) {
         a.jobs_cap = c->ring_cap;
         a.seq = c->d_seq;
@@ -526,7 +540,7 @@ static int enqueue_items(ps4_ctx *c) {
         a.ring_high = 32ull * (uint64_t)g_persist * PBS;         // ~1 ms of engine work at full rate
         a.ring_low = 4ull * (uint64_t)g_persist * PBS;
         a.raw = c->d_raw;
-        a.raw_cap = raw_cap_persist;
+        a.raw_cap = c->drill_now.list_cap(raw_cap_persist);
     }
     const bool ext = !(c->cfg.flags & PS4_F_NOEXT);
     const int g_ext = c->num_sms * (int)c->ext_ctas;
@@ -647,6 +661,7 @@ static int begin_items(ps4_ctx *c, const uint64_t *lo, const uint64_t *hi, uint3
     c->fused_fallback = false;
     c->persist_fallback = false;
     c->wide_tiles = false;
+    c->attempts = 0;
     c->last_launches = 0;
     c->last_ms = 0.0;
     c->h2d_bytes = c->d2h_bytes = 0;
@@ -707,7 +722,7 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
             }
         }
         const Status &st = *reinterpret_cast<const Status *>(c->h_block);
-        const unsigned code = (unsigned)(st.err & 0xFF);
+        const unsigned code = st.err ? (unsigned)(st.err & 0xFF) : c->drill_now.code;
         const unsigned long long errS = st.err >> 8;
         if (code == E_QUEUE) {                   // a batch outgrew the job queue: narrower batches
             if (c->batch_div < (1u << 16)) { c->batch_div *= 2; continue; }
@@ -933,6 +948,21 @@ extern "C" int ps4_check_pair_owners(int device, const uint32_t *first, uint32_t
     cudaFree(d_out);
     if (prev != device) cudaSetDevice(prev);
     return e == cudaSuccess ? PS4_OK : PS4_ERR_CUDA;
+}
+
+// ---- self-check of the re-runs ----
+
+extern "C" int ps4_check_reruns(ps4_ctx *c, uint32_t attempts, uint32_t list, uint64_t queue, uint32_t code) {
+    if (!c) return PS4_ERR_ARG;
+    if (code && (code < PS4_RERUN_TILE || code > PS4_RERUN_QUEUE))
+        return set_err(c, PS4_ERR_ARG, "ps4_check_reruns: code %u is not a PS4_RERUN_* code", code);
+    c->drill = Drill{attempts, list, code, queue};
+    return PS4_OK;
+}
+
+extern "C" void ps4_last_attempts(const ps4_ctx *c, uint32_t *attempts, uint32_t *log2_tile) {
+    if (attempts) *attempts = c ? c->attempts : 0;
+    if (log2_tile) *log2_tile = c ? c->run_tile_log2 : 0;
 }
 
 // ---- tuning ----

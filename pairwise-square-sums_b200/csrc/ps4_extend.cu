@@ -1185,7 +1185,9 @@ __global__ void __launch_bounds__(EBS, 3) extend_jobs(const __grid_constant__ Se
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     WarpArea *w = (WarpArea *)(esmem + (size_t)wid * sizeof(WarpArea));
     const uint32_t njobs = (uint32_t)min(*(volatile ull *)&a.status->n_jobs, (ull)a.jobs_cap);
-    if (njobs == 0) return;
+    // After an error the search is repeated or given up, and the end of an overflown queue may be unwritten
+    // (warps take their first stretch without another look).
+    if (njobs == 0 || *(volatile ull *)&a.status->err != 0ull) return;
     const uint32_t warps = gridDim.x * EWARPS;
     const uint32_t quota = min((njobs + warps - 1) / warps, 32u);                // 1 at least
     // a stretch is a 32nd of a warp's share, 32 to 256 4-sets (one atomic each)

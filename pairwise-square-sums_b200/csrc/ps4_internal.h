@@ -26,9 +26,9 @@ enum {
     E_CAP_DIVS = PS4_ERR_CAP_DIVS,
     E_CAP_EXT = PS4_ERR_CAP_EXT,
     E_VERIFY = PS4_ERR_VERIFY,
-    E_TILE = 100,      // a tile outgrew its shared-memory lists: re-run with smaller tiles
-    E_EXTLIST = 101,   // more extensions than a tile's (fused kernel) or an engine round's list holds
-    E_QUEUE = 102,     // the 4-set job queue of a batch overflowed: re-run with narrower batches
+    E_TILE = PS4_RERUN_TILE,          // a tile outgrew its shared-memory lists: re-run with smaller tiles
+    E_EXTLIST = PS4_RERUN_EXTLIST,    // more extensions than a tile's (fused kernel) or an engine round's list holds
+    E_QUEUE = PS4_RERUN_QUEUE,        // the 4-set job queue of a batch overflowed: re-run with narrower batches
     E_TIMEOUT = PS4_ERR_TIMEOUT   // a bounded wait of the persistent kernel gave up (code | where << 8)
 };
 
@@ -161,6 +161,14 @@ struct CtxView {
     void *stream;
 };
 int ctx_view(ps4_ctx *c, CtxView *v);
+// What ps4_check_reruns asks of the context's next attempt (all zero as a rule); counts the attempt.
+struct Drill {
+    uint32_t attempts, list, code;
+    uint64_t queue;
+    uint32_t list_cap(uint32_t n) const { return list && list < n ? list : n; }
+    uint64_t queue_cap(uint64_t n) const { return queue && queue < n ? queue : n; }
+};
+Drill ctx_drill(ps4_ctx *c);
 int ctx_fail(ps4_ctx *c, int code, const char *msg);
 
 // entries of the odd numbers' factor table next to tables of m < tab_n

@@ -226,6 +226,7 @@ struct StepBuf {
     int state = BUF_FREE;
     bool fused = false;
     unsigned tile_log2 = 13;
+    uint32_t drill_code = 0;              // ps4_check_reruns: the error that the step is taken to end with
     std::vector<Chunk> chunks;
     std::vector<uint32_t> tris;           // triple queries of the step
     std::vector<uint32_t> queries;        // distinct queries of the step
@@ -536,6 +537,8 @@ int launch_step(ps4_server *s, StepBuf &b) {
         tiles = 0;
     }
     const unsigned TL = b.tile_log2;
+    const Drill drill = n_items ? ctx_drill(s->ctx) : Drill{};
+    b.drill_code = drill.code;
     for (uint32_t i = 0; i < n_items; i++) {
         const Chunk &c = b.chunks[i];
         s_top = std::max(s_top, c.hi);
@@ -606,9 +609,11 @@ int launch_step(ps4_server *s, StepBuf &b) {
         a.status = b.d_status;
         a.cap_reps = s->v.cap_reps; a.cap_divs = s->v.cap_divs; a.cap_ext = s->v.cap_ext;
         a.flags = s->v.flags & ~(uint32_t)PS4_F_DUMP4;
-        a.jobs = s->d_jobs; a.jobs_cap = s->jobs_cap;
+        a.jobs = s->d_jobs; a.jobs_cap = drill.queue_cap(s->jobs_cap);
         if (!b.fused) {
-            a.raw = s->d_raw; a.raw_cap = raw_cap_for(TL); a.raw_lists = serve_lists(s->v.num_sms, TL);
+            a.raw = s->d_raw;
+            a.raw_cap = drill.list_cap(raw_cap_for(TL));
+            a.raw_lists = serve_lists(s->v.num_sms, TL);
             a.s_top = s_top;
             SRV_CUDA(s, (cudaError_t)launch_gen(a, gen_grid(s->v.num_sms, TL), st));
             if (!(s->v.flags & PS4_F_NOEXT)) SRV_CUDA(s, (cudaError_t)launch_ext(a, ext_grid(s->v.num_sms), st));
@@ -650,7 +655,7 @@ int check_step(ps4_server *s, StepBuf &b) {
     const Status &st = *b.h_status;
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, b.ev_start, b.ev_kern) == cudaSuccess) s->gpu_ms += ms;
-    const unsigned code = (unsigned)(st.err & 0xFF);
+    const unsigned code = st.err ? (unsigned)(st.err & 0xFF) : b.drill_code;
     const unsigned long long errS = st.err >> 8;
     bool rerun = false;
     auto chunk_of = [&](uint64_t S) -> int {
