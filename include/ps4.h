@@ -211,9 +211,9 @@ int ps4_plan_shards(uint64_t lo, uint64_t hi, uint32_t n, uint64_t *bounds);
 
 /* ---- exact-root self-check ----
  *
- * Runs the device's exact integer square roots -- the routines every square test and tile
- * scan of the search uses, restating isqrt64 / isqrt128 / is_sq128 (exhaustive/s4.c:95-108) --
- * on n[i] = hi[i]*2^64 + lo[i], so that they can be checked against exact host arithmetic
+ * Runs the device's exact integer square roots, restating isqrt64 / isqrt128 / is_sq128
+ * (exhaustive/s4.c:95-108) -- the routines of reports, of tiles that scan for themselves and of the
+ * per-lane divisor walk; the hot paths' are below -- on n[i] = hi[i]*2^64 + lo[i], so that they can be checked against exact host arithmetic
  * at their edges.  roots[4i..4i+3] = floor(sqrt(n)) (128-bit), floor(sqrt(lo)), ceil(sqrt(lo)),
  * and floor(sqrt(lo)) by the tile scan's single-precision estimate (lo < 2^46, else 0);
  * flags[i] bit 0: n is a square (exact test), bit 1: n is a square by the search's fast test,
@@ -221,6 +221,16 @@ int ps4_plan_shards(uint64_t lo, uint64_t hi, uint32_t n, uint64_t *bounds);
  * buffers on `device`; synchronous. */
 int ps4_check_roots(int device, const uint64_t *lo, const uint64_t *hi, uint32_t n, uint64_t *roots,
                     uint32_t *flags);
+
+/* The hot paths' own roots, on pairs a[i], b[i] of values, the result in out[i]:
+ *   PS4_ROOT_SQUARE  the engine's and the triple kernel's square test: 1 where u^2 + d is a square, u = a < 2^44,
+ *                    d = b as a signed number, |d| < 2^44, u^2 + d > 0;
+ *   PS4_ROOT_FIRST   the tile scan's first representation of S >= S0 with larger root q: S0 = a < 2^44, q = b >=
+ *                    sqrt(S0/2); the smaller root p >= 1 in the low half, p^2 + q^2 - S0 mod 2^32 in the high one;
+ *   PS4_ROOT_PAIR    pair number a < 2^25 as (x < y) with a = y(y-1)/2 + x: x in the low half, y in the high one.
+ * Other values give results without a meaning.  As ps4_check_roots otherwise. */
+enum { PS4_ROOT_SQUARE = 0, PS4_ROOT_FIRST = 1, PS4_ROOT_PAIR = 2 };
+int ps4_check_fast_roots(int device, uint32_t which, const uint64_t *a, const uint64_t *b, uint32_t n, uint64_t *out);
 
 /* Self-check of the bounded waits of PS4_KERNEL_PERSIST: one device thread waits, as a consuming
  * warp does, for a ring position that nothing publishes.  The wait gives up after its time limit

@@ -427,6 +427,35 @@ __device__ __forceinline__ uint32_t scan_reps(uint64_t S0, uint32_t n, uint32_t 
 constexpr uint32_t SCAN_RUN = 24;       // a q with more p than this is walked by a whole warp
 constexpr int SCAN_ILP = 4;            // q per lane and turn: their roots are independent chains
 
+// First p >= 1 of a q >= sqrt(SS0/2) with p^2 + q^2 >= SS0: p = ceil(sqrt(m)), m = SS0 - q^2, for SS0 < 2^44.  With qt = floor(sqrt(SS0)) and k = qt - q, m = (SS0 - qt^2) +
+// k (2 qt - k): k, 2 qt - k and SS0 - qt^2 <= 2 qt are below 2^24, exact in single precision, so one fused
+// multiply-add gives m to half a unit (2^-24 relative) and sqrt.approx (2^-23) the root, below 2^22, to
+// 2/3: its floor is off by one at most, and the difference m - r^2, below 2^24, comes from 32-bit products.
+// (A 64-bit conversion and 64-bit products per q: 680 cycles a turn of one q on a narrow call.)
+// i = p^2 + q^2 - SS0, modulo 2^32.
+struct ScanStart {
+    uint32_t qt, lo0;                              // floor(sqrt(SS0)); SS0 modulo 2^32
+    float ft;                                      // SS0 - qt^2
+};
+__device__ __forceinline__ ScanStart scan_start(uint64_t SS0) {
+    const uint32_t qt = (uint32_t)isqrt64(SS0);
+    return ScanStart{qt, (uint32_t)SS0, (float)(uint32_t)(SS0 - (uint64_t)qt * qt)};
+}
+__device__ __forceinline__ void first_rep(const ScanStart &s, uint32_t q, uint32_t &p, uint32_t &i) {
+    float f;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"(fmaf((float)(s.qt - q), (float)(s.qt + q), s.ft)));
+    uint32_t r = (uint32_t)f;
+    int32_t d = (int32_t)(s.lo0 - q * q - r * r);          // m - r^2, where q <= qt
+    if (d < 0) { r--; d += 2 * (int32_t)r + 1; }           // floor(root) or one below it from here on
+    if (d > 2 * (int32_t)r) { d -= 2 * (int32_t)r + 1; r++; }
+    p = d > 0 ? r + 1 : r;
+    i = d > 0 ? 2 * r + 1 - (uint32_t)d : 0u;
+    if (q > s.qt || p == 0) {                              // q^2 >= SS0: p from 1
+        p = 1;
+        i = q * q + 1 - s.lo0;
+    }
+}
+
 // The scan of scan_reps over a group of adjacent tiles [SS0, SS1) of one segment, done once by
 // `parts` CTAs together (this one takes every parts-th q, from `part`): every representation goes
 // to its tile's list (offset in the tile | p << 14 | q << 36; p <= q < 2^22, offset < 2^14), each CTA
@@ -434,19 +463,14 @@ constexpr int SCAN_ILP = 4;            // q per lane and turn: their roots are i
 // per representation, or per tile that a warp's turn of a long run meets).  A count above cap means the
 // part overflowed; that tile then scans for itself.
 //
-// First p of a q: p = ceil(sqrt(m)), m = SS0 - q^2.  With qt = floor(sqrt(SS0)) and k = qt - q, m = (SS0 - qt^2) +
-// k (2 qt - k): k, 2 qt - k and SS0 - qt^2 <= 2 qt are below 2^24, exact in single precision, so one fused
-// multiply-add gives m to half a unit (2^-24 relative) and sqrt.approx (2^-23) the root, below 2^22, to
-// 2/3: its floor is off by one at most, and the difference m - r^2, below 2^24, comes from 32-bit products.
-// (A 64-bit conversion and 64-bit products per q: 680 cycles a turn of one q on a narrow call.)
 template <int NT>
 __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned TLv, uint64_t *lists, uint32_t cap,
                                            uint32_t *cnt, uint32_t part, uint32_t parts) {
     uint32_t qmin = (uint32_t)ceil_sqrt64((SS0 + 1) >> 1);
     if (qmin < 1) qmin = 1;
-    const uint32_t qmax = SS1 >= 2 ? (uint32_t)isqrt64(SS1 - 2) : 0, qt = (uint32_t)isqrt64(SS0);
-    const uint32_t width = (uint32_t)(SS1 - SS0), wmask = (1u << TLv) - 1u, lo0 = (uint32_t)SS0;
-    const float ft = (float)(uint32_t)(SS0 - (uint64_t)qt * qt);
+    const uint32_t qmax = SS1 >= 2 ? (uint32_t)isqrt64(SS1 - 2) : 0;
+    const uint32_t width = (uint32_t)(SS1 - SS0), wmask = (1u << TLv) - 1u;
+    const ScanStart start = scan_start(SS0);
     // long runs need 2 * SCAN_RUN * p < width, so p < pc and q^2 >= SS0 - pc^2: below qc there are none
     const uint64_t pc = width / (2 * SCAN_RUN);
     const uint32_t qc = pc * pc < SS0 ? (uint32_t)isqrt64(SS0 - pc * pc) : 0u;
@@ -464,20 +488,8 @@ __device__ __forceinline__ void scan_group(uint64_t SS0, uint64_t SS1, unsigned 
         uint32_t p[SCAN_ILP], i[SCAN_ILP];                 // i = p^2 + q^2 - SS0, below width where it counts
 #pragma unroll
         for (int u = 0; u < SCAN_ILP; u++) {
-            const uint32_t q = qw + by_lane * lane + parts * NT * u, k = qt - q;
-            float f;
-            asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"(fmaf((float)k, (float)(qt + q), ft)));
-            uint32_t r = (uint32_t)f;
-            int32_t d = (int32_t)(lo0 - q * q - r * r);    // m - r^2, where q <= qt
-            if (d < 0) { r--; d += 2 * (int32_t)r + 1; }   // floor(root) or one below it from here on
-            if (d > 2 * (int32_t)r) { d -= 2 * (int32_t)r + 1; r++; }
-            p[u] = d > 0 ? r + 1 : r;
-            i[u] = d > 0 ? 2 * r + 1 - (uint32_t)d : 0u;
-            const bool top = q > qt || p[u] == 0;          // q^2 >= SS0: p from 1
-            if (top) {
-                p[u] = 1;
-                i[u] = q * q + 1 - lo0;                    // below 2^32 where q <= qmax: q^2 + 1 < SS1
-            }
+            const uint32_t q = qw + by_lane * lane + parts * NT * u;
+            first_rep(start, q, p[u], i[u]);               // i < 2^32 where q <= qmax: q^2 + 1 < SS1
             if (q > qmax || p[u] > q) i[u] = 0xFFFFFFFFu;
         }
 #pragma unroll

@@ -35,6 +35,7 @@
 #include "ps4_internal.h"
 
 #include "ps4_device.cuh"
+#include "ps4_rows.cuh"
 
 namespace ps4 {
 
@@ -314,6 +315,17 @@ __global__ void check_roots(const uint64_t *lo, const uint64_t *hi, uint32_t n, 
     flags[i] = f;
 }
 
+// The hot paths' own roots, one thread per value (ps4_check_fast_roots).
+__global__ void check_fast_roots(uint32_t which, const uint64_t *a, const uint64_t *b, uint32_t n, uint64_t *out) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    uint32_t x = 0, y = 0;
+    if (which == PS4_ROOT_SQUARE) x = is_square_near(a[k], (int64_t)b[k], a[k] * a[k] + b[k]);
+    else if (which == PS4_ROOT_FIRST) first_rep(scan_start(a[k]), (uint32_t)b[k], x, y);
+    else decode_pair((uint32_t)a[k], x, y);
+    out[k] = (uint64_t)y << 32 | x;
+}
+
 // ================================================================== launchers
 
 int search_block_threads() { return BS; }
@@ -412,6 +424,28 @@ extern "C" int ps4_check_roots(int device, const uint64_t *lo, const uint64_t *h
     cudaFree(d_in);
     cudaFree(d_out);
     cudaFree(d_flags);
+    if (prev != device) cudaSetDevice(prev);
+    return e == cudaSuccess ? PS4_OK : PS4_ERR_CUDA;
+}
+
+extern "C" int ps4_check_fast_roots(int device, uint32_t which, const uint64_t *a, const uint64_t *b, uint32_t n,
+                                    uint64_t *out) {
+    if (which > PS4_ROOT_PAIR) return PS4_ERR_ARG;
+    if (n == 0) return PS4_OK;
+    if (!a || !b || !out) return PS4_ERR_ARG;
+    int prev = 0;
+    if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return PS4_ERR_CUDA;
+    const size_t bytes = (size_t)n * sizeof(uint64_t);
+    uint64_t *d = nullptr;
+    cudaError_t e = cudaMalloc((void **)&d, 3 * bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        ps4::check_fast_roots<<<(n + 255) / 256, 256>>>(which, d, d + n, n, d + 2 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
     if (prev != device) cudaSetDevice(prev);
     return e == cudaSuccess ? PS4_OK : PS4_ERR_CUDA;
 }

@@ -151,6 +151,8 @@ def load() -> C.CDLL:
         "ps4_search_enqueue": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint64]),
         "ps4_plan_shards": (C.c_int, [C.c_uint64, C.c_uint64, C.c_uint32, P(C.c_uint64)]),
         "ps4_check_ring_wait": (C.c_int, [C.c_int, P(C.c_uint64)]),
+        "ps4_check_fast_roots": (C.c_int, [C.c_int, C.c_uint32, P(C.c_uint64), P(C.c_uint64), C.c_uint32,
+                                           P(C.c_uint64)]),
         "ps4_check_reruns": (C.c_int, [C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint64, C.c_uint32]),
         "ps4_last_attempts": (None, [C.c_void_p, P(C.c_uint32), P(C.c_uint32)]),
         "ps4_check_pair_owners": (C.c_int, [C.c_int, P(C.c_uint32), C.c_uint32, P(C.c_uint64)]),
