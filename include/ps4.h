@@ -66,7 +66,8 @@ typedef struct {
     uint32_t cap_ext;      /* extension cap per 4-set         (S4_MAX_EXT,  default 64,    s4.c:49)  */
     uint32_t flags;        /* PS4_F_*                                                               */
     uint32_t kernel;       /* PS4_KERNEL_*                                                          */
-    uint32_t log2_tile;    /* S values per tile = 2^log2_tile (12..14); 0 = autotuned/default        */
+    uint32_t log2_tile;    /* S values per tile = 2^log2_tile (12..14); 0 = autotuned/default, and      */
+                           /* smaller ones for calls with fewer tiles than the device takes at once  */
     uint32_t ctas_per_sm;  /* resident CTAs per SM for the persistent kernel; 0 = default            */
     void *stream;          /* cudaStream_t to launch on; NULL = a stream owned by the context        */
     uint32_t use_graph;    /* PS4_GRAPH_*: run a call's launch sequence as one captured CUDA graph   */
@@ -362,7 +363,8 @@ void ps4_serve_get_info(const ps4_server *srv, ps4_serve_info *info);
  * of the search fills at most 90 % of it).  No counterpart in the reference (its engine has
  * fixed compile-time sizes, s4.c:46-52). */
 typedef struct {
-    uint32_t log2_tile;       /* 12 .. 14                                                            */
+    uint32_t log2_tile;       /* 12 .. 14, of calls that fill the device (fewer tiles: smaller ones,   */
+                              /* unless ps4_config.log2_tile asked for a size)                       */
     uint32_t gen_ctas;        /* 1 .. 2: tile-kernel threads per SM in units of 512 (512-thread CTAs  */
                               /* on 2^14-S tiles, 256-thread ones on smaller tiles)                 */
     uint32_t ext_ctas;        /* 1 .. 3                                                              */

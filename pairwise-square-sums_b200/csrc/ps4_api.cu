@@ -57,6 +57,7 @@ struct ps4_ctx {
     double last_ms = 0.0;
     uint64_t last_launches = 0;
     unsigned tile_log2 = 13;             // current tile size (may shrink on E_TILE)
+    bool pin_tile = false;               // narrow calls keep that size too: asked for, or being timed
     unsigned run_tile_log2 = 13;         // the tile size of the launches in flight (smaller for narrow calls)
     PendingSearch pend;
     uint64_t *d_raw = nullptr;           // per tile-kernel CTA: SUPER_K tile lists of RAW_PER_TILE
@@ -244,6 +245,7 @@ extern "C" int ps4_create(const ps4_config *cfg, ps4_ctx **out) {
     // for the one-kernel designs, whose CTAs keep 512 threads
     if (c->cfg.kernel != PS4_KERNEL_BATCHED) c->tile_log2 = 14;
     if (c->cfg.log2_tile) c->tile_log2 = std::min(14u, std::max(12u, c->cfg.log2_tile));
+    c->pin_tile = c->cfg.log2_tile != 0;
     *out = c;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
@@ -421,7 +423,7 @@ static int enqueue_items(ps4_ctx *c) {
     if (kernel == PS4_KERNEL_PERSIST && c->persist_fallback) kernel = PS4_KERNEL_BATCHED;
     const bool persist = kernel == PS4_KERNEL_PERSIST;
     unsigned TL = persist ? 13u : c->tile_log2;            // the persistent kernel's tiles are 2^13 S
-    if (kernel == PS4_KERNEL_BATCHED && !c->wide_tiles) {
+    if (kernel == PS4_KERNEL_BATCHED && !c->wide_tiles && !c->pin_tile) {
         uint64_t tiles = 0;
         for (const Item &it : p.items) tiles += (it.hi - it.lo + (1ull << TL) - 1) >> TL;
         TL = narrow_tile_log2(TL, tiles, c->num_sms);
@@ -1047,12 +1049,15 @@ extern "C" int ps4_autotune(ps4_ctx *c, const uint64_t *lo, const uint64_t *hi, 
                 t.log2_tile = tl; t.gen_ctas = gc; t.ext_ctas = ec; t.rate = 0;
                 int rc = ps4_set_tuning(c, &t);
                 double ms = 1e300;
+                const bool pin = c->pin_tile;
+                c->pin_tile = true;                        // the shape by its name, also for a narrow sample
                 for (int rep = 0; rep < 2 && rc == PS4_OK; rep++) {
                     rc = begin_items(c, slo.data(), shi.data(), (uint32_t)slo.size(), false, 0);
                     if (rc == PS4_OK) rc = finish_items(c, st.data(), nullptr);
                     c->pend.active = false;
                     if (rc == PS4_OK && rep == 1) ms = c->last_ms;
                 }
+                c->pin_tile = pin;
                 if (rc != PS4_OK) {
                     ps4_set_tuning(c, &start);
                     return rc;

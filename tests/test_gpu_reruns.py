@@ -9,7 +9,7 @@ import ctypes as C
 import pytest
 
 from conftest import assert_stats_equal
-from ps4b200 import Search, _abi, workloads
+from ps4b200 import Ps4Error, Search, _abi, workloads
 from ps4b200.serve import Server
 
 pytestmark = pytest.mark.gpu
@@ -98,6 +98,32 @@ def test_server_steps(step_S, list_, queue, code, reruns):
             assert srv.info()["step_reruns"] == reruns
     for a, b in zip(got, want):
         same(a, b)
+
+
+@pytest.mark.parametrize("width", [4097, NARROW, WIDE])
+@pytest.mark.parametrize("tile", [12, 13, 14])
+def test_a_tile_size_asked_for_is_kept(width, tile):
+    with Search(2 * LO) as s:
+        want = s.range(LO, LO + width)
+    with Search(2 * LO, log2_tile=tile) as s:
+        same(s.range(LO, LO + width), want)
+        assert attempts(s) == (1, tile)
+        s.lib.ps4_check_reruns(s.ctx, 1, 0, 0, TILE)
+        if tile > 12:
+            same(s.range(LO, LO + width), want)
+            assert attempts(s) == (2, tile - 1)
+        else:
+            with pytest.raises(Ps4Error) as e:
+                s.range(LO, LO + width)
+            assert "tile capacity exceeded" in e.value.message and attempts(s) == (1, 12)
+
+
+def test_the_tuner_times_the_tiles_it_names():
+    with Search(2 * LO) as s:
+        t = s.autotune([LO], [LO + NARROW], budget_s=1e-9)       # the first candidate only
+        assert (t["log2_tile"], attempts(s)) == (14, (1, 14))
+        s.range(LO, LO + NARROW)
+        assert attempts(s) == (1, 12)
 
 
 def test_arguments():
