@@ -359,17 +359,22 @@ struct TileLayout {
     static constexpr uint32_t FLUSH_AT = W / 2;                             // staged 4-sets that trigger P6
 };
 
+// The segment of tile ti: the last one whose first tile is not after it.
+__device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
+    uint32_t lo = 0, hi = a.n_items;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (a.items[mid].tile_base <= ti) lo = mid; else hi = mid;
+    }
+    return a.items[lo];
+}
+
 // locate a tile: tiles are handed out highest-S first (longest work first); `item` is the
 // query item of the segment holding the tile
 __device__ __forceinline__ void tile_bounds(const SearchArgs &a, uint64_t tile, unsigned TLv, uint32_t &item,
                                             uint64_t &S0, uint32_t &n) {
     const uint64_t ti = a.n_tiles - 1 - tile;
-    uint32_t lo = 0, hi = a.n_items;                   // last item with tile_base <= ti
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a.items[mid].tile_base <= ti) lo = mid; else hi = mid;
-    }
-    const Item it = a.items[lo];
+    const Item it = segment_of(a, ti);
     item = it.id;
     S0 = it.lo + ((ti - it.tile_base) << TLv);
     const uint64_t S1 = S0 + (1ull << TLv) < it.hi ? S0 + (1ull << TLv) : it.hi;

@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "ps4_device.cuh"
 #include "ps4_rows.cuh"
@@ -297,16 +298,11 @@ struct JobSpan {
     uint64_t cur = 0;
     uint32_t rem = 0;
 };
-
-// The segment of tile ti: the last one whose first tile is not after it.
-__device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
-    uint32_t lo = 0, hi = a.n_items;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a.items[mid].tile_base <= ti) lo = mid; else hi = mid;
-    }
-    return a.items[lo];
-}
+// A tile's positions in the persistent kernel's ring, in shared memory: the first one, and whether there is room.
+struct RingSpan {
+    ull base;
+    int store;
+};
 
 // One tile [S0, S0+n) of query item `item`: P1-P4 (from its list's parts, or by scanning when list
 // is null), then P5: each warp takes a contiguous block of the tile's pairs, 32 at a time.  NT threads.
@@ -316,8 +312,8 @@ __device__ __forceinline__ Item segment_of(const SearchArgs &a, uint64_t ti) {
 template <int TL, int NT, bool RING, bool SIDE>
 __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t S0,
                                              uint32_t n, uint32_t item, const uint64_t *list,
-                                             const uint32_t *list_n, uint32_t parts, uint32_t cap, JobSpan &span,
-                                             unsigned long long &s_base, int &s_store) {
+                                             const uint32_t *list_n, uint32_t parts, uint32_t cap,
+                                             std::conditional_t<RING, RingSpan, JobSpan> &span) {
     using L = TileLayout<TL>;
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -350,15 +346,15 @@ __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts
     }
     PairSets ps;
     uint32_t mine = 0, total;
-    if (RING) {
+    if constexpr (RING) {
         const uint32_t lo_first = lo0;
         for (uint32_t g = gw; g < ge; g += 32) mine += pair_sets(v, S0, g + lane, ge, lane, lo0, ps);
         lo0 = lo_first;
         uint32_t off, d1, d2, tot[3];
         block_scan3<NT>(mine, 0u, 0u, off, d1, d2, tot, ts.wsum);
         if (tid == 0) {
-            s_base = 0;
-            s_store = 0;
+            span.base = 0;
+            span.store = 0;
             if (!noext && tot[0]) {
                 // room: the ring holds the reserved-but-unfinished 4-sets plus this tile's
                 WaitClock wc;
@@ -368,23 +364,23 @@ __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts
                     __nanosleep(256);
                 }
                 if (ok) {
-                    s_base = atomicAdd(&a.status->q_tail, (ull)tot[0]);
-                    s_store = 1;
+                    span.base = atomicAdd(&a.status->q_tail, (ull)tot[0]);
+                    span.store = 1;
                 }
             }
         }
         __syncthreads();
         if (need_write_pass) {
-            uint64_t cur = s_base + __shfl_sync(0xffffffffu, off, 0);
+            uint64_t cur = span.base + __shfl_sync(0xffffffffu, off, 0);
             for (uint32_t g = gw; g < ge; g += 32) {
                 const uint32_t m = pair_sets(v, S0, g + lane, ge, lane, lo0, ps);
                 const uint32_t first = warp_prefix(m, lane, total);
-                write_sets<true>(a, v, m, ps, first, total, lane, S0, item, s_store != 0, cur, total, 0);
+                write_sets<true>(a, v, m, ps, first, total, lane, S0, item, span.store != 0, cur, total, 0);
                 cur += total;
             }
         }
         __syncthreads();
-        if (tid == 0 && s_store && tot[0]) atomicAdd(&a.status->q_pub, (ull)tot[0]);
+        if (tid == 0 && span.store && tot[0]) atomicAdd(&a.status->q_pub, (ull)tot[0]);
     } else {
         for (uint32_t g = gw; g < ge; g += 32) {
             const uint32_t m = pair_sets(v, S0, g + lane, ge, lane, lo0, ps);
@@ -428,9 +424,8 @@ __device__ __forceinline__ void produce_tile(const SearchArgs &a, TileShared &ts
 // tiles, then tile by tile.  Returns the number of tiles.
 template <int TL, int NT>
 __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned char *smem, uint64_t c0,
-                                  uint64_t *lists, uint32_t *raw_n, unsigned long long &s_base, int &s_store) {
+                                  uint64_t *lists, uint32_t *raw_n, RingSpan &span) {
     using L = TileLayout<TL>;
-    JobSpan span;
     const uint64_t cn = min((uint64_t)SUPER_K, a.n_tiles - c0);
     uint64_t ti = a.n_tiles - c0 - cn;
     const uint64_t ti_end = a.n_tiles - c0;
@@ -449,7 +444,7 @@ __device__ uint32_t produce_group(const SearchArgs &a, TileShared &ts, unsigned 
             const uint64_t S0 = SA + ((uint64_t)j << TL);
             produce_tile<TL, NT, true, false>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
                                        raw_n[j] <= a.raw_cap ? lists + (size_t)j * a.raw_cap : nullptr, &raw_n[j], 1,
-                                       a.raw_cap, span, s_base, s_store);
+                                       a.raw_cap, span);
         }
         ti = g_end;
     }
@@ -466,8 +461,7 @@ __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const 
     using L = TileLayout<TL>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileShared ts;
-    __shared__ unsigned long long s_base, s_claim;
-    __shared__ int s_store;
+    __shared__ unsigned long long s_claim;
     JobSpan span;
     __shared__ uint32_t s_tile, s_fit;
     // entries that this CTA's scan appended to each tile's list, and the next tile to take (CTA 0's
@@ -524,8 +518,7 @@ __global__ void __launch_bounds__(NT, NT > BS ? 1 : BS / NT * 2) gen_jobs(const 
             __syncthreads();
             const uint64_t S0 = SA + ((uint64_t)j << TL);
             produce_tile<TL, NT, false, SIDE>(a, ts, smem, S0, (uint32_t)min((uint64_t)L::W, SB - S0), it.id,
-                                        s_fit ? lists + (size_t)j * nc * cap : nullptr, s_n, nc, cap, span, s_base,
-                                        s_store);
+                                        s_fit ? lists + (size_t)j * nc * cap : nullptr, s_n, nc, cap, span);
         }
         __syncthreads();                                                 // s_tile read by all
         ti = g_end;
@@ -1222,9 +1215,10 @@ __global__ void __launch_bounds__(PBS, 3) search_persist(const __grid_constant__
     using L = TileLayout<PTL>;
     extern __shared__ __align__(16) unsigned char smem[];
     TileShared &ts = *reinterpret_cast<TileShared *>(smem + P_TS_OFF);
-    __shared__ unsigned long long s_base, s_idle0;
+    __shared__ unsigned long long s_idle0;
+    __shared__ RingSpan s_span;
     __shared__ unsigned int s_claim;
-    __shared__ int s_store, s_role, s_busy;
+    __shared__ int s_role, s_busy;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     uint64_t *lists = a.raw + (size_t)blockIdx.x * SUPER_K * a.raw_cap;
     uint32_t *raw_n = (uint32_t *)(smem + L::OFF_ELIST);
@@ -1258,7 +1252,7 @@ __global__ void __launch_bounds__(PBS, 3) search_persist(const __grid_constant__
         const int role = s_role;
         if (role == 0) break;                                // block-uniform
         if (role == 1) {
-            const uint32_t cn = produce_group<PTL, PBS>(a, ts, smem, s_claim, lists, raw_n, s_base, s_store);
+            const uint32_t cn = produce_group<PTL, PBS>(a, ts, smem, s_claim, lists, raw_n, s_span);
             if (tid == 0) {
                 __threadfence();
                 atomicAdd(&a.status->q_produced, (ull)cn);
