@@ -16,7 +16,7 @@
 //                 through a warp queue, where those that are the reference's ext_sqrt are
 //                 square-tested 64 at a time.                                  (s4.c:160-207)
 //
-// The engine is bound by instruction issue (74 % of issue slots busy, 30.0 of 32 threads active; DRAM 2.4 %).
+// The engine is bound by instruction issue (74 % of issue slots busy, 30.0 of 32 threads active; DRAM 3.0 %).
 // Per [1,1e10) search its launches take 163 ms; with candidates spread over the lanes in 32 equal
 // runs, u64 lists, per-candidate member tests and IEEE double square roots they took 313 ms (25.5 -> 14.8 warp
 // instructions per S).  Rows cost a partly empty turn (30.2 turns of 32 candidates per round against
