@@ -41,10 +41,10 @@ struct ps4_ctx {
     // one block holds the status and the items' counters, so that both are cleared and copied back at
     // once; a call of few items has its segments behind them, and clears and uploads in one copy
     unsigned char *d_block = nullptr; uint64_t block_cap = 0;
-    unsigned char *h_block = nullptr;    // pinned: where the block lands
+    unsigned char *h_block = nullptr;    // pinned: where the block lands (of many items, the status)
     unsigned char *h_stage = nullptr;    // pinned: zeros and segments to upload
     unsigned char *h_pin = nullptr;      // one pinned allocation, in whose halves both lie while they fit
-    unsigned char *h_big_block = nullptr; uint64_t h_big_block_cap = 0;
+    unsigned char *h_big_block = nullptr; uint64_t h_big_block_cap = 0;     // or two pieces of counters
     unsigned char *h_big_stage = nullptr; uint64_t h_big_stage_cap = 0;
     Status *d_status = nullptr;
     unsigned long long *d_counters = nullptr;
@@ -54,6 +54,7 @@ struct ps4_ctx {
     ps4_quad *d_quads = nullptr; uint64_t quads_cap = 0;
     uint32_t *d_scratch = nullptr; size_t scratch_words = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_piece[2] = {nullptr, nullptr};
     double last_ms = 0.0;
     uint64_t last_launches = 0;
     unsigned tile_log2 = 13;             // current tile size (may shrink on E_TILE)
@@ -151,14 +152,14 @@ static int grow32(ps4_ctx *c, T *&ptr, uint32_t &cap, uint64_t need) {
     return rc;
 }
 
-// a pinned host buffer of at least `need` elements (grown by half again, kept between calls)
+// a pinned host buffer of at least `need` elements (grown by half again unless `exact`, kept between calls)
 template <class T>
-static int grow_pinned(ps4_ctx *c, T *&ptr, uint64_t &cap, uint64_t need) {
+static int grow_pinned(ps4_ctx *c, T *&ptr, uint64_t &cap, uint64_t need, bool exact = false) {
     if (need <= cap && ptr) return 0;
     if (ptr) cudaFreeHost(ptr);
     ptr = nullptr;
     cap = 0;
-    const uint64_t n = std::max<uint64_t>(need + need / 2, 1024);
+    const uint64_t n = std::max<uint64_t>(exact ? need : need + need / 2, 1024);
     CUDA_TRY(c, cudaMallocHost((void **)&ptr, n * sizeof(T)));
     cap = n;
     return 0;
@@ -169,6 +170,10 @@ static const size_t BLOCK_HEAD = (sizeof(Status) + 255) & ~(size_t)255;
 static size_t block_bytes(uint64_t n_items) { return BLOCK_HEAD + (size_t)n_items * K_SLOTS * sizeof(unsigned long long); }
 static const uint32_t SMALL_ITEMS = 16, SMALL_SEGS = 64;             // uploaded together with their zeros
 static const size_t PIN_HALF = 32768;
+// The counters of more than two pieces of items are fetched piece by piece, to alternate halves of a pinned
+// buffer: pinning room for them all took 0.4 ms per MB (first call of 4096 small subranges 5 to 11 ms, now 2.6).
+static const uint32_t PIECE = 256;
+static size_t landing_bytes(uint32_t n_items) { return n_items <= 2 * PIECE ? block_bytes(n_items) : BLOCK_HEAD; }
 static int reserve_block(ps4_ctx *c, uint32_t n_items) {
     if (grow(c, c->d_block, c->block_cap, std::max<uint64_t>(c->block_cap, block_bytes(n_items) + SMALL_SEGS * sizeof(Item))))
         return PS4_ERR_CUDA;
@@ -176,8 +181,9 @@ static int reserve_block(ps4_ctx *c, uint32_t n_items) {
     c->d_counters = reinterpret_cast<unsigned long long *>(c->d_block + BLOCK_HEAD);
     c->h_block = c->h_pin + PIN_HALF;
     if (block_bytes(n_items) <= PIN_HALF) return 0;
-    if (grow_pinned(c, c->h_big_block, c->h_big_block_cap, block_bytes(n_items))) return PS4_ERR_CUDA;
-    c->h_block = c->h_big_block;
+    const uint64_t need = n_items <= 2 * PIECE ? block_bytes(n_items) : 2 * PIECE * K_SLOTS * sizeof(unsigned long long);
+    if (grow_pinned(c, c->h_big_block, c->h_big_block_cap, need, true)) return PS4_ERR_CUDA;
+    if (n_items <= 2 * PIECE) c->h_block = c->h_big_block;
     return 0;
 }
 static int reserve_stage(ps4_ctx *c, size_t bytes) {
@@ -220,6 +226,8 @@ extern "C" void ps4_destroy(ps4_ctx *c) {
     for (cudaEvent_t e : c->kev) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
+    for (cudaEvent_t e : c->ev_piece)
+        if (e) cudaEventDestroy(e);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -569,7 +577,6 @@ static int enqueue_items(ps4_ctx *c) {
         key_add(key, a);
         key_add(key, kernel); key_add(key, n_items); key_add(key, grid); key_add(key, g_gen); key_add(key, g_ext);
         key_add(key, stage_cap); key_add(key, c->d_scratch); key_add(key, c->h_stage); key_add(key, dev_items);
-        key_add(key, c->h_block);
         key_add(key, c->stream);
     }
     if (small) memset(c->h_stage, 0, blk);
@@ -648,8 +655,8 @@ static int enqueue_items(ps4_ctx *c) {
         if (rc) return rc;
     }
     CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-    // the status and every item's counters, in one copy that the result's wait covers
-    CUDA_TRY(c, cudaMemcpyAsync(c->h_block, c->d_block, blk, cudaMemcpyDeviceToHost, c->stream));
+    // the status and (up to two pieces) every item's counters, in one copy that the result's wait covers
+    CUDA_TRY(c, cudaMemcpyAsync(c->h_block, c->d_block, landing_bytes(n_items), cudaMemcpyDeviceToHost, c->stream));
     return PS4_OK;
 }
 
@@ -695,6 +702,37 @@ static int begin_items(ps4_ctx *c, const uint64_t *lo, const uint64_t *hi, uint3
     return rc;
 }
 
+// Adds the items' counters to stats (one per item, +=): from where they landed, or piece by piece, the next
+// one on its way while one is added.
+static int add_counters(ps4_ctx *c, uint32_t n_items, ps4_stats *stats) {
+    if (n_items <= 2 * PIECE) {
+        const unsigned long long *k = reinterpret_cast<const unsigned long long *>(c->h_block + BLOCK_HEAD);
+        for (uint32_t i = 0; i < n_items; i++) stats_add(&stats[i], &k[(size_t)i * K_SLOTS]);
+        return PS4_OK;
+    }
+    for (cudaEvent_t &e : c->ev_piece)
+        if (!e) CUDA_TRY(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    unsigned long long *const land = reinterpret_cast<unsigned long long *>(c->h_big_block);
+    const uint32_t pieces = (n_items + PIECE - 1) / PIECE;
+    for (uint32_t k = 0; k <= pieces; k++) {
+        if (k < pieces) {                                  // its half was added two rounds ago
+            const uint64_t first = (uint64_t)k * PIECE * K_SLOTS;
+            const size_t bytes = (size_t)std::min(PIECE, n_items - k * PIECE) * K_SLOTS * sizeof(unsigned long long);
+            CUDA_TRY(c, cudaMemcpyAsync(land + (k & 1) * PIECE * K_SLOTS, c->d_counters + first, bytes,
+                                        cudaMemcpyDeviceToHost, c->stream));
+            CUDA_TRY(c, cudaEventRecord(c->ev_piece[k & 1], c->stream));
+            c->d2h_bytes += bytes;
+        }
+        if (k > 0) {
+            const uint32_t first = (k - 1) * PIECE;
+            CUDA_TRY(c, cudaEventSynchronize(c->ev_piece[(k - 1) & 1]));
+            for (uint32_t i = first; i < std::min(first + PIECE, n_items); i++)
+                stats_add(&stats[i], land + ((k - 1) & 1) * PIECE * K_SLOTS + (size_t)(i - first) * K_SLOTS);
+        }
+    }
+    return PS4_OK;
+}
+
 // Wait for the enqueued search, re-run it on internal capacity limits, then copy the results
 // into the caller's buffers and add the counters (stats: one per item, +=).
 static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
@@ -708,7 +746,7 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
             if (rc) return rc;
         }
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        c->d2h_bytes += block_bytes(n_items);
+        c->d2h_bytes += landing_bytes(n_items);
         if (p.tiles > 0) {
             float ms = 0.f;
             cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -786,7 +824,6 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
                                (unsigned long long)res->quads_cap, st.n_quads);
             }
         }
-        const unsigned long long *k = reinterpret_cast<const unsigned long long *>(c->h_block + BLOCK_HEAD);
         const bool fits = res && st.n_hits <= res->hits_cap && st.n_exts <= res->exts_cap &&
                           st.n_sixes <= res->sixes_cap;
         if (fits) {                              // the records land in pinned buffers, then go in order to res
@@ -826,9 +863,7 @@ static int finish_items(ps4_ctx *c, ps4_stats *stats, ps4_results *res) {
             canonical_order_into(c->h_hits, st.n_hits, c->h_exts, c->h_sixes, st.n_sixes, res->hits, res->exts);
             if (st.n_sixes) memcpy(res->sixes, c->h_sixes, st.n_sixes * sizeof(ps4_six));
         }
-        if (stats)
-            for (uint32_t i = 0; i < n_items; i++) stats_add(&stats[i], &k[(size_t)i * K_SLOTS]);
-        return PS4_OK;
+        return stats ? add_counters(c, n_items, stats) : PS4_OK;
     }
     return set_err(c, PS4_ERR_CUDA, "search did not converge after repeated re-runs");
 }

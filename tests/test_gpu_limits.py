@@ -83,3 +83,17 @@ def test_more_than_a_million_items():
         assert sorted(set(got)) == [i for i in sorted(alone) if alone[i].lines]
         other = np.frombuffer(stats, dtype=np.uint64).reshape(n, -1)
         assert sorted(np.flatnonzero(other.any(axis=1))) == sorted(ranges)
+
+
+# items uploaded with their zeros (16), counters landing in the context's own block (31), in one of their own
+# (512) and piece by piece (256 each)
+@pytest.mark.parametrize("n", [1, 16, 17, 31, 32, 512, 513, 768, 769, 5000])
+def test_counters_of_every_item(n):
+    los = [10 ** 6 + 997 * i % 10 ** 6 for i in range(n)]
+    widths = [i * i % 389 + (i % 7 > 0) for i in range(n)]
+    with Search(3 * 10 ** 6) as s:
+        for _ in range(2):                               # the second call adds to nothing left from the first
+            stats, _ = s.batch(los, [a + w for a, w in zip(los, widths)])
+            assert [st["S_done"] for st in stats] == widths
+        for i in {0, n // 2, n - 1, 255 % n, 256 % n, 511 % n, 512 % n}:
+            assert_stats_equal(stats[i], s.range(los[i], los[i] + widths[i]).stats, label=f"item {i}")
