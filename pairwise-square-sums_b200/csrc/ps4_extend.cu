@@ -1336,6 +1336,11 @@ constexpr uint64_t FEW_TILES = 128;
 //    tile kernel with 8 / 2 / 1 CTAs: [1,1e10) 98.9 / 80.9 / 80.0 ms; 2e8 S at 1e12 2.79 / 3.05 / 3.82; 3e7 S at
 //    1.2e13 1.05 / 1.65 / 2.45; 64 subranges below 1e11 10.3 / 9.0 / 9.3; 2e4 S at 4e11 0.042 / 0.066 / 0.096
 //    (all with parts read one by one; side by side, as eight are now, 2.57, 0.99 and 0.040 at 1e12, 1.2e13 and 4e11).
+//  * Segments of fewer tiles than a cluster has CTAs share no more than their own scan: a cluster of c takes s / c +
+//    ceil(t / c) for one of t tiles, and K clusters take segs / K rounds, half of the last one idle.  Where that promises a
+//    fifth at least, the c with the least of it.  Tile kernel, one scan per CTA and 16 tiles / the rule above / this
+//    one: 8000 subranges of 8000 S at 1e12 8.50 / 9.39 / 6.87 ms, 40000 of 30 S at 1e7 1.02 / 1.67 / 0.83, 1000 of 8000 S at 1e9
+//    1.14 / 0.44 / 0.10, 200 of 1000 S at 1e7 0.31 / 0.11 / 0.03.  (Without the fifth: 200 of 30000 S at 1e12 0.40 -> 0.54.)
 //  * Tiles per claim: n tiles in groups of G on K clusters take n + s n / G of work and about G K / 2 of
 //    idling at the end, least at G = sqrt(2 n s / K).
 // `grid`: the CTAs that the lists of a.raw are sized for; whole clusters of them are launched, no more
@@ -1344,7 +1349,17 @@ int launch_gen(SearchArgs a, int grid, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const double n = (double)std::max<uint64_t>(a.n_tiles, 1);
     const double scan = 0.29 * std::sqrt((double)a.s_top) / (34e3 * std::ldexp(1.0, (int)a.log2_tile - 13));
-    const uint32_t cl = n < 11e3 * scan || grid < 16 ? GEN_CLUSTER : 2;
+    uint32_t cl = n < 11e3 * scan || grid < 16 ? GEN_CLUSTER : 2;
+    const double segs = a.n_items, t = n / segs;
+    if (segs > 1 && t < GEN_CLUSTER) {
+        auto cost = [&](uint32_t c) {
+            const double rounds = segs / std::min(std::max(grid / (int)c, 1) * 1.0, std::ceil(n / c));
+            return (rounds > 1 ? rounds + 0.5 : 1.0) * (scan / c + std::ceil(t / c));
+        };
+        double least = 0.8 * cost(cl);
+        for (const uint32_t c : {1u, 2u, GEN_CLUSTER})
+            if (cost(c) < least) { least = cost(c); cl = c; }
+    }
     const uint64_t fit = std::max<uint64_t>((uint64_t)grid / cl, 1), want = ((uint64_t)n + cl - 1) / cl;
     const uint64_t K = std::min(fit, want), ctas = K * cl;
     const double G = std::min(std::sqrt(2 * n * scan / (double)K), std::ceil(n / (double)K));

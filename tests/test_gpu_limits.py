@@ -9,7 +9,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from conftest import assert_stats_equal
+from conftest import COUNTERS, assert_stats_equal
 from oracle import orc
 from ps4b200 import Search, _abi, workloads
 from ps4b200.serve import Server
@@ -83,6 +83,23 @@ def test_more_than_a_million_items():
         assert sorted(set(got)) == [i for i in sorted(alone) if alone[i].lines]
         other = np.frombuffer(stats, dtype=np.uint64).reshape(n, -1)
         assert sorted(np.flatnonzero(other.any(axis=1))) == sorted(ranges)
+
+
+# subranges of 1 to 8 tiles, side by side: clusters of one, two and eight CTAs, with fewer subranges than clusters
+# and with several rounds of them
+@pytest.mark.parametrize("lo,n,w", [(10 ** 6, 20, 30), (10 ** 9, 300, 12000), (10 ** 9, 700, 8192), (10 ** 9, 4000, 8193),
+                                    (10 ** 12, 20, 4096), (10 ** 12, 200, 30000), (10 ** 12, 1500, 20001),
+                                    (4 * 10 ** 11, 500, 7 * 8192 + 1), (4 * 10 ** 11, 300, 65536)])
+def test_batches_of_narrow_subranges_vs_one_range(lo, n, w):
+    cuts = [lo + i * w for i in range(n + 1)]
+    with Search(2 * 10 ** 12) as s:
+        stats, r = s.batch(cuts[:-1], cuts[1:])
+        one = s.range(lo, cuts[-1])
+    assert r.lines == one.lines
+    assert [st["S_done"] for st in stats] == [w] * n
+    for k in COUNTERS:
+        assert sum(st[k] for st in stats) == one.stats[k], k
+    assert max(st["max_reps"] for st in stats) == one.stats["max_reps"]
 
 
 # items uploaded with their zeros (16), counters landing in the context's own block (31), in one of their own
