@@ -1177,10 +1177,11 @@ __global__ void __launch_bounds__(EBS, 3) extend_jobs(const __grid_constant__ Se
     extern __shared__ __align__(16) unsigned char esmem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     WarpArea *w = (WarpArea *)(esmem + (size_t)wid * sizeof(WarpArea));
-    const uint32_t njobs = (uint32_t)min(*(volatile ull *)&a.status->n_jobs, (ull)a.jobs_cap);
-    // After an error the search is repeated or given up, and the end of an overflown queue may be unwritten
-    // (warps take their first stretch without another look).
-    if (njobs == 0 || *(volatile ull *)&a.status->err != 0ull) return;
+    // An overflown queue (more reserved than it holds) ends with unwritten records; its search is repeated.  (A look at
+    // the error word instead, which covers that too, is a second load: 2 of 34 us of the smallest calls.)
+    const ull queued = *(volatile ull *)&a.status->n_jobs;
+    if (queued == 0 || queued > a.jobs_cap) return;
+    const uint32_t njobs = (uint32_t)queued;
     const uint32_t warps = gridDim.x * EWARPS;
     const uint32_t quota = min((njobs + warps - 1) / warps, 32u);                // 1 at least
     // a stretch is a 32nd of a warp's share, 32 to 256 4-sets (one atomic each)
